@@ -51,6 +51,7 @@ thread_local std::string g_err;
 
 struct pfcg_handle {
 	int dev = 0;
+	int nsm = 148;
 	pfcg_prec prec = PFCG_FP64;
 	Model model{};
 	Geom geom{};
@@ -75,6 +76,11 @@ struct pfcg_handle {
 	void* twctx = nullptr;  // per-pass twiddle tables of the specialised kernels
 	void* twcty = nullptr;
 	int sbx = 1, sby = 1, sbx1 = 1, sby1 = 1;
+	bool widetab = false;   // the handle has kernels_wide.cuh's tables
+	void* wtwx = nullptr;
+	void* wtwy = nullptr;
+	int wsbx = 1, wsby = 1;
+	int ccr = 1;            // columns per CTA of the run-time y-pass modes (geom.CC: the STEP kernel's)
 	double* d_real = nullptr;   // U*Ny*Nx doubles
 	double* d_fields = nullptr; // f(r) work fields
 	double* d_part = nullptr;   // partial sums of the field means
@@ -136,46 +142,48 @@ bool factor_ok(int n) {
 	return n == 1;
 }
 
-// n = RM^nmain * rtail * 3^n3 * 5^n5 * 7^n7, rtail in {1,2,4,8} below RM
-bool make_plan(int n, int rmain, FftPlan* p) {
-	if (!factor_ok(n)) return false;
-	int m = n, k2 = 0;
-	p->n = n;
-	p->n3 = p->n5 = p->n7 = 0;
-	while (m % 2 == 0) { m /= 2; k2++; }
-	while (m % 3 == 0) { m /= 3; p->n3++; }
-	while (m % 5 == 0) { m /= 5; p->n5++; }
-	while (m % 7 == 0) { m /= 7; p->n7++; }
-	const int lg = (rmain == 16) ? 4 : 3;
-	p->nmain = k2 / lg;
-	p->rtail = 1 << (k2 % lg);
-	return true;
+// the plan of a transform of length n (fft_rt.cuh); false where one sequence
+// does not fit MAX_THREADS threads
+bool make_plan(int n, bool fp64, FftPlan* p) {
+	return factor_ok(n) && rt_make_plan(n, fp64, MAX_THREADS, RT_MAXE, p);
 }
 
-// threads one fft_batch over P sequences needs (0 if more than MAX_THREADS)
-int threads_for(const FftPlan& p, int P, int maxe) {
-	auto need = [&](int R) {
-		const long long bfly = (long long)P * p.n / R;
-		const int nb = maxe / R;
-		return (int)((bfly + nb - 1) / nb);
-	};
-	int nt = 32;
-	if (p.nmain > 0) nt = std::max(nt, need(maxe));
-	if (p.rtail > 1) nt = std::max(nt, need(p.rtail));
-	if (p.n3) nt = std::max(nt, need(3));
-	if (p.n5) nt = std::max(nt, need(5));
-	if (p.n7) nt = std::max(nt, need(7));
-	nt = (nt + 31) / 32 * 32;
-	return nt <= MAX_THREADS ? nt : 0;
+// sequences per transform call: the fewest calls that fit MAX_THREADS threads, of equal size
+int sub_batch(const FftPlan& p, int S) {
+	int calls = 1;
+	while (calls < S && rt_plan_threads(p, (S + calls - 1) / calls) > MAX_THREADS) calls++;
+	return (S + calls - 1) / calls;
 }
 
-// largest sub-batch (<= S) whose FFT fits in MAX_THREADS threads; 0 if none
-int sub_batch(const FftPlan& p, int S, int maxe, int* nt) {
+// FP32 systems of three and four fields run the kernels of kernels_wide.cuh
+bool is_wide(const pfcg_handle* h) { return h->prec == PFCG_FP32 && h->U >= 3 && h->widetab; }
+
+RadixPlan radix_plan(int n) {
+	RadixPlan p{n, 0, 1, 0, 0, 0};
+	int k2 = 0;
+	while (n % 2 == 0) { n /= 2; k2++; }
+	while (n % 3 == 0) { n /= 3; p.n3++; }
+	while (n % 5 == 0) { n /= 5; p.n5++; }
+	while (n % 7 == 0) { n /= 7; p.n7++; }
+	p.nmain = k2 / 4;
+	p.rtail = 1 << (k2 % 4);
+	return p;
+}
+
+// sequences per transform call of those kernels (the most that fit MAX_THREADS threads), and the threads
+int wide_sub_batch(const RadixPlan& p, int S, int* nt) {
 	for (int sb = S; sb >= 1; sb--) {
-		const int t = threads_for(p, sb, maxe);
-		if (t) { *nt = t; return sb; }
+		auto need = [&](int r) { return rt_threads(p.n, r, sb); };
+		*nt = 32;
+		if (p.nmain) *nt = std::max(*nt, need(16));
+		if (p.rtail > 1) *nt = std::max(*nt, need(p.rtail));
+		if (p.n3) *nt = std::max(*nt, need(3));
+		if (p.n5) *nt = std::max(*nt, need(5));
+		if (p.n7) *nt = std::max(*nt, need(7));
+		*nt = (*nt + 31) / 32 * 32;
+		if (*nt <= MAX_THREADS) return sb;
 	}
-	return 0;
+	return 0; // (make_plan has refused such a length)
 }
 
 template <typename T> int padded_host(int n) { return padded_len<T>(n); }
@@ -189,83 +197,114 @@ bool x_tile_ok(const pfcg_handle* h, int r) {
 	const int CH = h->U * r;
 	if (CH > MAX_CH) return false;
 	const int P = (CH + 1) / 2;
-	if ((size_t)P * padded(h->Nx, fp64) * h->celem > budget) return false;
-	int nt;
-	return sub_batch(h->px, P, max_elems_per_thread(fp64), &nt) > 0;
+	return (size_t)P * padded(h->Nx, fp64) * h->celem <= budget;
 }
 
 bool y_group_ok(const pfcg_handle* h, int c) {
 	const bool fp64 = h->prec == PFCG_FP64;
 	const size_t budget = fp64 ? 200 * 1024 : 150 * 1024;
 	const int S = h->U * c;
-	if ((size_t)S * padded(h->Ny, fp64) * h->celem > budget) return false;
-	int nt;
-	return sub_batch(h->py, S, max_elems_per_thread(fp64), &nt) > 0;
+	return (size_t)S * padded(h->Ny, fp64) * h->celem <= budget;
 }
 
-// launch shapes of the runtime-plan kernels for row tile R and column group CC
-void set_generic_configs(pfcg_handle* h, int R, int CC) {
-	const bool fp64 = h->prec == PFCG_FP64;
-	const int maxe = max_elems_per_thread(fp64);
-	const int U = h->U;
-	h->geom.R = R;
-	h->geom.CC = CC;
-	int nt;
-	const int P = (U * R + 1) / 2;
-	h->sbx = sub_batch(h->px, P, maxe, &nt);
-	h->cx = {h->Ny / R, nt, (int)(P * padded(h->Nx, fp64) * h->celem)};
-	const int P1 = (R + 1) / 2;
-	h->sbx1 = sub_batch(h->px, P1, maxe, &nt);
-	h->cx1 = {h->Ny / R, nt, (int)(P1 * padded(h->Nx, fp64) * h->celem)};
-	const int S = U * CC;
-	h->sby = sub_batch(h->py, S, maxe, &nt);
-	h->cy = {(h->H + CC - 1) / CC, nt, (int)(S * padded(h->Ny, fp64) * h->celem)};
-	h->sby1 = sub_batch(h->py, CC, maxe, &nt);
-	h->cy1 = {(h->H + CC - 1) / CC, nt, (int)(CC * padded(h->Ny, fp64) * h->celem)};
+// CTAs of nt threads and smem bytes that run at once on an SM, at the register
+// counts the kernels of run-time lengths are compiled for (RT_MINB)
+int rt_resident(const pfcg_handle* h, int nt, int smem) {
+	const int regs = h->prec == PFCG_FP64 ? 128 : 64;
+	return std::max(1, std::min({65536 / (regs * nt), 227 * 1024 / (smem + 1024), 2048 / nt, 32}));
+}
+
+// Launch shape of the kernels of run-time lengths: S sequences of plan p per
+// CTA. More threads than the passes need shorten the chain (a thread per
+// butterfly, more loads in flight between the transforms) until the grid takes
+// another wave: 1024^2 U=1 FP64 steps in 31 us with 128 threads (one wave) and
+// 46 us with 256 (two); 1440 x 900 U=2 FP32 in 45.6 us with 256 and 47.6 with 224.
+LaunchCfg rt_config(const pfcg_handle* h, const FftPlan& p, int S, int grid, int* sb) {
+	*sb = sub_batch(p, S);
+	const int smem = (int)(S * p.ld * h->celem);
+	int nt = rt_plan_threads(p, *sb);
+	auto waves = [&](int n) { return (grid + h->nsm * rt_resident(h, n, smem) - 1) / (h->nsm * rt_resident(h, n, smem)); };
+	for (int n : {256, 128, 64})
+		if (n > nt && n <= S * p.n / 4 && waves(n) <= waves(nt)) {
+			nt = n;
+			break;
+		}
+	return {grid, nt, smem, 0};
+}
+
+// the STEP kernels of run-time lengths; the y-pass's last CTA does the k = 0 update
+void use_rt_steps(pfcg_handle* h) {
 	h->cxs = h->cx;
 	h->cys = h->cy;
+	h->cys.grid++;
+}
+
+// launch shapes of the kernels of run-time lengths for row tile R and column group CC
+void set_generic_configs(pfcg_handle* h, int R, int CC) {
+	const int U = h->U;
+	h->geom.R = R;
+	h->geom.CC = h->ccr = CC;
+	if (is_wide(h)) h->ccr = 1;
+	h->cx = rt_config(h, h->px, (U * R + 1) / 2, h->Ny / R, &h->sbx);
+	h->cx1 = rt_config(h, h->px, (R + 1) / 2, h->Ny / R, &h->sbx1);
+	const int groups = (h->H + h->ccr - 1) / h->ccr;
+	h->cy = rt_config(h, h->py, U * h->ccr, groups, &h->sby);
+	h->cy1 = rt_config(h, h->py, h->ccr, groups, &h->sby1);
+	use_rt_steps(h);
+	if (is_wide(h)) {
+		int nt;
+		const int P = (U * R + 1) / 2, S = U * CC;
+		h->wsbx = wide_sub_batch(radix_plan(h->Nx), P, &nt);
+		h->cxs = {h->Ny / R, nt, (int)(P * padded(h->Nx, false) * h->celem), 0};
+		h->wsby = wide_sub_batch(radix_plan(h->Ny), S, &nt);
+		h->cys = {(h->H + CC - 1) / CC + 1, nt, (int)(S * padded(h->Ny, false) * h->celem), 0};
+	}
+}
+
+// Row tile R of the kernels of run-time lengths. FP64: as few rows as fill whole
+// sequences (two at U = 1 and 3, one at U = 2 and 4), since two sequences of a
+// long row leave one CTA per SM (4096^2 U=2: 827 us per step at R = 1, 887 at 2)
+// and short rows only lose latency by sharing a CTA. FP32: four rows, whose 32
+// bytes per column are a whole sector of the y-pass's gather (3000 x 2700 U=2:
+// 238 us at R = 4, 247 at 2, 259 at 1), two where four would leave SMs without a
+// tile (512^2 U=1: 15.4 us at both).
+int rt_rows(const pfcg_handle* h) {
+	const int least = h->U % 2 ? 2 : 1;
+	if (h->prec == PFCG_FP32)
+		for (int r : {4, 2})
+			if (r > least && x_tile_ok(h, r) && h->Ny / r >= h->nsm) return r;
+	return x_tile_ok(h, least) ? least : x_tile_ok(h, 1) ? 1 : 0;
 }
 
 // Chooses the row tile R (x-pass) and column group CC (y-pass): the shape of
-// the compile-time specialised kernels where the size has one, otherwise the
-// largest sizes that fit shared memory and still give two CTAs per SM
+// the compile-time specialised kernels where the size has one, otherwise
+// rt_rows and one column per CTA (more lost at every size measured: 512^2 U=2
+// FP32 18.3, 20.2 and 25.9 us per step at 1, 2 and 4; 2048^2 U=2 FP64 182 and 201)
 // (pfcg_autotune can replace this guess by measurement).
-int choose_layout(pfcg_handle* h, int nsm) {
-	const bool fp64 = h->prec == PFCG_FP64;
-	const int want = 2 * nsm;
+int choose_layout(pfcg_handle* h) {
 	const int U = h->U;
-	int R = 0;
 	// PFCG_GENERIC_KERNELS=1 in the environment disables the specialised kernels (A/B checks)
 	const char* gen = std::getenv("PFCG_GENERIC_KERNELS");
-	const bool allow_spec = !(gen && gen[0] == '1');
-	const int rs = allow_spec ? spec_rows(fp64, U, h->Nx) : 0;
-	if (rs && h->Ny % rs == 0) R = rs;
-	for (int r : {8, 4, 2, 1}) {
-		if (R) break;
-		if (!x_tile_ok(h, r)) continue;
-		R = r;
-		if (h->Ny / r >= want) break;
-	}
+	const bool allow_spec = h->prec == PFCG_FP32 && !(gen && gen[0] == '1');
+	int R = allow_spec ? spec_rows(U, h->Nx) : 0;
+	const bool xspec = R > 0 && h->Ny % R == 0;
+	int CC = 1;
+	if (is_wide(h)) {
+		R = x_tile_ok(h, 2) ? 2 : x_tile_ok(h, 1) ? 1 : 0;
+		CC = y_group_ok(h, 4) ? 4 : y_group_ok(h, 2) ? 2 : 1;
+	} else if (!xspec) R = rt_rows(h);
 	if (!R) return fail(h, PFCG_ESIZE, "no x-pass tile fits shared memory for this Nx");
-	int CC = 0;
-	const bool yspec = allow_spec && spec_cols(fp64, U, h->Ny) && spec_rows(fp64, U, h->Ny) == R;
-	if (yspec) CC = spec_cols(fp64, U, h->Ny);
-	for (int c : {4, 2, 1}) {
-		if (CC) break;
-		if (!y_group_ok(h, c)) continue;
-		CC = c;
-		if ((h->H + c - 1) / c >= want) break;
-	}
-	if (!CC) return fail(h, PFCG_ESIZE, "no y-pass column group fits shared memory for this Ny");
+	if (!y_group_ok(h, 1)) return fail(h, PFCG_ESIZE, "no y-pass column group fits shared memory for this Ny");
 	set_generic_configs(h, R, CC);
-	if (rs && R == rs) h->cxs = {h->Ny / R, spec_x_threads(fp64, U, h->Nx), spec_x_smem(fp64, U, h->Nx), 1};
-	if (yspec) {
+	if (xspec) h->cxs = {h->Ny / R, spec_x_threads(U, h->Nx), spec_x_smem(U, h->Nx), 1};
+	if (allow_spec && spec_cols(U, h->Ny) && spec_rows(U, h->Ny) == R) {
+		CC = h->geom.CC = spec_cols(U, h->Ny);
 		// The specialised y-pass keeps the update between the two transforms in
 		// shared memory by default (measured faster at 4096^2 U=2: 0.299 vs 0.328 ms);
 		// PFCG_YPASS_FUSED=1 selects the register-fused variant.
 		const char* fu = std::getenv("PFCG_YPASS_FUSED");
 		const bool fused = fu && fu[0] == '1';
-		h->cys = {(h->H + CC - 1) / CC, spec_y_threads(fp64, U, h->Ny, fused), spec_y_smem(fp64, U, h->Ny), fused ? 1 : 2};
+		h->cys = {(h->H + CC - 1) / CC + 1, spec_y_threads(U, h->Ny, fused), spec_y_smem(U, h->Ny), fused ? 1 : 2};
 		const char* ri = std::getenv("PFCG_YPASS_REGIO");
 		h->regio = (ri && ri[0] == '0') ? 0 : 1;
 	}
@@ -276,7 +315,7 @@ int choose_layout(pfcg_handle* h, int nsm) {
 // CtPlan): passes of radix rmain with the tail radix second; pass p > 0 contributes
 // entries [q * Ns + jm] = exp(-2 pi i r_q jm / (Ns R)) with r_q = q + 1, or for
 // radix 16 r_q in {1, 2, 3, 4, 8, 12} (ct_twiddle makes the other powers).
-template <typename T> int upload_ct_twiddles(pfcg_handle* h, int N, int rmain, void** dst) {
+int upload_ct_twiddles(pfcg_handle* h, int N, int rmain, void** dst) {
 	// N = rmain^A * tail; the tail radix is the second pass (fft_core.cuh, CtPlan)
 	std::vector<int> radix;
 	int rest = N;
@@ -285,7 +324,7 @@ template <typename T> int upload_ct_twiddles(pfcg_handle* h, int N, int rmain, v
 		rest /= rmain;
 	}
 	if (rest > 1) radix.insert(radix.begin() + (radix.empty() ? 0 : 1), rest);
-	std::vector<cplx<T>> tab;
+	std::vector<float2> tab;
 	int Ns = 1;
 	for (size_t p = 0; p < radix.size(); p++) {
 		const int R = radix[p];
@@ -296,28 +335,44 @@ template <typename T> int upload_ct_twiddles(pfcg_handle* h, int N, int rmain, v
 				for (int jm = 0; jm < Ns; jm++) {
 					const int r = R == 16 ? pow16[q] : q + 1;
 					const double a = -2.0 * PI * (double)r * (double)jm / ((double)Ns * R);
-					cplx<T> w;
-					w.x = (T)std::cos(a);
-					w.y = (T)std::sin(a);
+					float2 w;
+					w.x = (float)std::cos(a);
+					w.y = (float)std::sin(a);
 					tab.push_back(w);
 				}
 		Ns *= R;
 	}
-	if ((int)tab.size() != spec_twiddles(h->prec == PFCG_FP64, N)) return fail(h, PFCG_ESIZE, "twiddle table size mismatch");
-	CK(h, cudaMalloc(dst, sizeof(cplx<T>) * tab.size()));
-	CK(h, cudaMemcpy(*dst, tab.data(), sizeof(cplx<T>) * tab.size(), cudaMemcpyHostToDevice));
+	if ((int)tab.size() != spec_twiddles(N)) return fail(h, PFCG_ESIZE, "twiddle table size mismatch");
+	CK(h, cudaMalloc(dst, sizeof(float2) * tab.size()));
+	CK(h, cudaMemcpy(*dst, tab.data(), sizeof(float2) * tab.size(), cudaMemcpyHostToDevice));
 	return 0;
 }
 
-template <typename T> int upload_twiddles(pfcg_handle* h, int n, void** dst) {
-	std::vector<cplx<T>> tw(n);
-	for (int k = 0; k < n; k++) {
-		const double a = -2.0 * PI * (double)k / (double)n;
+// twiddles of a run-time plan (rt_twiddle_of)
+template <typename T> int upload_twiddles(pfcg_handle* h, const FftPlan& p, void** dst) {
+	std::vector<cplx<T>> tw(p.ntw + 1);
+	for (int k = 0; k < p.ntw; k++) {
+		int num, den;
+		rt_twiddle_of(p, sizeof(T) == 8, k, &num, &den);
+		const double a = -2.0 * PI * (double)num / (double)den;
 		tw[k].x = (T)std::cos(a);
 		tw[k].y = (T)std::sin(a);
 	}
-	CK(h, cudaMalloc(dst, sizeof(cplx<T>) * n));
-	CK(h, cudaMemcpy(*dst, tw.data(), sizeof(cplx<T>) * n, cudaMemcpyHostToDevice));
+	CK(h, cudaMalloc(dst, sizeof(cplx<T>) * tw.size()));
+	CK(h, cudaMemcpy(*dst, tw.data(), sizeof(cplx<T>) * tw.size(), cudaMemcpyHostToDevice));
+	return 0;
+}
+
+// exp(-2 pi i k / n), k < n, in FP32
+int upload_roots(pfcg_handle* h, int n, void** dst) {
+	std::vector<float2> tw(n);
+	for (int k = 0; k < n; k++) {
+		const double a = -2.0 * PI * (double)k / (double)n;
+		tw[k].x = (float)std::cos(a);
+		tw[k].y = (float)std::sin(a);
+	}
+	CK(h, cudaMalloc(dst, sizeof(float2) * n));
+	CK(h, cudaMemcpy(*dst, tw.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
 	return 0;
 }
 
@@ -331,7 +386,7 @@ int setup_tma(pfcg_handle* h) {
 	const char* env = std::getenv("PFCG_TMA");
 	if (env && env[0] == '0') return 0;
 	if (h->prec != PFCG_FP32 || !h->cys.spec || h->cys.spec == 1 || !h->regio || h->U > 2) return 0;
-	if (!spec_y_regio(false, h->U, h->Ny)) return 0;
+	if (!spec_y_regio(h->U, h->Ny)) return 0;
 	const int R = h->geom.R, CC = h->geom.CC, ntile = h->Ny / R;
 	const size_t el = sizeof(float2);
 	if ((R * el) % 16 != 0 || CC > 256 || R > 256) return 0;
@@ -433,10 +488,17 @@ template <typename T> XArgs<T> xargs(pfcg_handle* h) {
 	a.m = h->model;
 	a.g = h->geom;
 	a.part = h->nlpart;
+	a.k = host_nl_k<T>(h->model);
+	if (is_wide(h)) {
+		a.wtw = (const cplx<T>*)h->wtwx;
+		a.wplan = radix_plan(h->Nx);
+		a.wsb = h->wsbx;
+	}
 	return a;
 }
 
-template <typename T> YArgs<T> yargs(pfcg_handle* h) {
+// arguments of the y-pass modes other than STEP; step: those of the STEP kernel
+template <typename T> YArgs<T> yargs(pfcg_handle* h, bool step = false) {
 	YArgs<T> a{};
 	a.work = (cplx<T>*)h->work;
 	a.wstride = (long long)h->H * h->Ny;
@@ -450,6 +512,12 @@ template <typename T> YArgs<T> yargs(pfcg_handle* h) {
 	a.sb = h->sby;
 	a.m = h->model;
 	a.g = h->geom;
+	if (!step) a.g.CC = h->ccr;
+	if (is_wide(h)) {
+		a.wtw = (const cplx<T>*)h->wtwy;
+		a.wplan = radix_plan(h->Ny);
+		a.wsb = h->wsby;
+	}
 	a.regio = h->regio;
 	a.tmap = h->tmap;
 	a.tma_tiles = h->tma_tiles;
@@ -529,10 +597,15 @@ template <typename T> int spectral_from_real(pfcg_handle* h) {
 		CK(h, launch_field_means(h->d_real, h->U, (long long)npts, h->d_part, MEAN_BLOCKS, h->mean, h->stream));
 	}
 	XArgs<T> xa = xargs<T>(h);
-	rc = run_xpass<T>(h, XP_R2C, xa, h->cx);
+	rc = run_xpass<T>(h, XP_R2C, xa, is_wide(h) ? h->cxs : h->cx);
 	if (rc) return rc;
-	YArgs<T> ya = yargs<T>(h);
-	rc = run_ypass<T>(h, YP_INIT, ya, h->cy);
+	YArgs<T> ya = yargs<T>(h, is_wide(h));
+	LaunchCfg cy = h->cy;
+	if (is_wide(h)) {
+		cy = h->cys;
+		cy.grid--; // no k = 0 update
+	}
+	rc = run_ypass<T>(h, YP_INIT, ya, cy);
 	if (rc) return rc;
 	CK(h, cudaStreamSynchronize(h->stream));
 	return 0;
@@ -614,7 +687,7 @@ template <typename T> void capture_steps(pfcg_handle* h, const XArgs<T>& xa, con
 template <typename T> int do_steps(pfcg_handle* h, int nsteps) {
 	XArgs<T> xa = xargs<T>(h);
 	xa.acc = h->acc + ACC_NL;
-	YArgs<T> ya = yargs<T>(h);
+	YArgs<T> ya = yargs<T>(h, true);
 	// The reference resynchronises the spectral state every 100 steps and after
 	// evaluate (pfc-relax.c:1179-1185, 1125-1130); the y-pass does the same
 	// projection every step, so no separate pass is needed.
@@ -893,7 +966,7 @@ int pfcg_size_supported_for(int Nx, int Ny, int U, pfcg_prec prec) {
 	h.Ny = Ny;
 	h.H = Nx / 2 + 1;
 	h.celem = prec == PFCG_FP64 ? sizeof(double2) : sizeof(float2);
-	if (!make_plan(Nx, max_radix(prec == PFCG_FP64), &h.px) || !make_plan(Ny, max_radix(prec == PFCG_FP64), &h.py))
+	if (!make_plan(Nx, prec == PFCG_FP64, &h.px) || !make_plan(Ny, prec == PFCG_FP64, &h.py))
 		return 0;
 	return x_tile_ok(&h, 1) && y_group_ok(&h, 1);
 }
@@ -919,6 +992,7 @@ int pfcg_create(const pfcg_params* p, int Nx, int Ny, double dx, double dy, pfcg
 
 	pfcg_handle* h = new pfcg_handle();
 	h->dev = dev;
+	h->nsm = prop.multiProcessorCount;
 	h->prec = prec;
 	h->model = to_model(p);
 	h->U = p->U;
@@ -933,10 +1007,10 @@ int pfcg_create(const pfcg_params* p, int Nx, int Ny, double dx, double dy, pfcg
 	set_dk(h);
 	const bool fp64 = prec == PFCG_FP64;
 	h->celem = fp64 ? sizeof(double2) : sizeof(float2);
-	const int rmain = max_radix(fp64);
+	h->widetab = true;
 	int rc = 0;
-	if (!make_plan(Nx, rmain, &h->px) || !make_plan(Ny, rmain, &h->py)) rc = fail(h, PFCG_ESIZE, "bad factorisation");
-	if (!rc) rc = choose_layout(h, prop.multiProcessorCount);
+	if (!make_plan(Nx, fp64, &h->px) || !make_plan(Ny, fp64, &h->py)) rc = fail(h, PFCG_ESIZE, "bad factorisation");
+	if (!rc) rc = choose_layout(h);
 	auto bail = [&](int code) {
 		g_err = h->err;
 		pfcg_destroy(h);
@@ -967,14 +1041,12 @@ int pfcg_create(const pfcg_params* p, int Nx, int Ny, double dx, double dy, pfcg
 	CKC(cudaMemset(h->flag, 0, sizeof(int)));
 	CKC(cudaMemset(h->nlpart, 0, sizeof(double) * nlpart_elems(Ny)));
 #undef CKC
-	rc = fp64 ? upload_twiddles<double>(h, Nx, &h->twx) : upload_twiddles<float>(h, Nx, &h->twx);
-	if (!rc) rc = fp64 ? upload_twiddles<double>(h, Ny, &h->twy) : upload_twiddles<float>(h, Ny, &h->twy);
-	if (!rc && h->cxs.spec)
-		rc = fp64 ? upload_ct_twiddles<double>(h, Nx, ct_radix(true, Nx), &h->twctx)
-		          : upload_ct_twiddles<float>(h, Nx, ct_radix(false, Nx), &h->twctx);
-	if (!rc && h->cys.spec)
-		rc = fp64 ? upload_ct_twiddles<double>(h, Ny, ct_radix(true, Ny), &h->twcty)
-		          : upload_ct_twiddles<float>(h, Ny, ct_radix(false, Ny), &h->twcty);
+	rc = fp64 ? upload_twiddles<double>(h, h->px, &h->twx) : upload_twiddles<float>(h, h->px, &h->twx);
+	if (!rc) rc = fp64 ? upload_twiddles<double>(h, h->py, &h->twy) : upload_twiddles<float>(h, h->py, &h->twy);
+	if (!rc && is_wide(h)) rc = upload_roots(h, Nx, &h->wtwx);
+	if (!rc && is_wide(h)) rc = upload_roots(h, Ny, &h->wtwy);
+	if (!rc && h->cxs.spec) rc = upload_ct_twiddles(h, Nx, ct_radix(Nx), &h->twctx);
+	if (!rc && h->cys.spec) rc = upload_ct_twiddles(h, Ny, ct_radix(Ny), &h->twcty);
 	if (!rc) rc = setup_tma(h);
 	if (rc) return bail(rc);
 	*out = h;
@@ -989,6 +1061,8 @@ void pfcg_destroy(pfcg_handle* h) {
 	cudaFree(h->work1);
 	cudaFree(h->twx);
 	cudaFree(h->twy);
+	cudaFree(h->wtwx);
+	cudaFree(h->wtwy);
 	cudaFree(h->twctx);
 	cudaFree(h->twcty);
 	cudaFree(h->tmap);
@@ -1282,7 +1356,7 @@ std::map<std::tuple<int, int, int, int>, std::pair<int, int>> g_tune;
 template <typename T> int time_steps(pfcg_handle* h, int nsteps, float* ms) {
 	XArgs<T> xa = xargs<T>(h);
 	xa.acc = h->acc + ACC_NL;
-	YArgs<T> ya = yargs<T>(h);
+	YArgs<T> ya = yargs<T>(h, true);
 	cudaEvent_t e0, e1;
 	CK(h, cudaEventCreate(&e0));
 	CK(h, cudaEventCreate(&e1));
@@ -1317,7 +1391,7 @@ extern "C" int pfcg_autotune(pfcg_handle* h, int nsteps) {
 	float best = 1e30f;
 	int bR = h->geom.R, bC = h->geom.CC;
 	for (int r : {8, 4, 2, 1}) {
-		if (!x_tile_ok(h, r)) continue;
+		if (!x_tile_ok(h, r) || h->U * r < 2) continue; // (a lone real row would leave half a sequence empty)
 		for (int c : {4, 2, 1}) {
 			if (!y_group_ok(h, c)) continue;
 			set_generic_configs(h, r, c);
@@ -1343,8 +1417,8 @@ extern "C" int pfcg_autotune(pfcg_handle* h, int nsteps) {
 
 // ------------------------------------------------------------------ batch ---
 // Problems of a batch that run the same kernels: one length N = Nx = Ny and
-// field count U with specialised kernels, or (ct = false) every other problem,
-// on the runtime-plan kernels. A class's blocks are a contiguous range of the
+// field count U (batch_own_class; ct: on specialised kernels), or every other
+// problem, on the kernels of run-time lengths. A class's blocks are a contiguous range of the
 // batch's block tables, and its steps form one chain of the step graph on its
 // own stream, independent of the other classes' chains.
 struct BatchClass {
@@ -1376,6 +1450,12 @@ struct pfcg_batch {
 
 // whether a batch problem runs the specialised kernels (decided at creation)
 static bool batch_ct(const pfcg_handle* h) { return h->cxs.spec && h->cys.spec && h->Nx == h->Ny && h->U <= 2; }
+// whether it is in a class of its size and field count: those, and the large FP64
+// squares, whose shared memory would otherwise bound the CTAs per SM of every
+// smaller problem in the launch
+static bool batch_own_class(const pfcg_handle* h) {
+	return batch_ct(h) || (h->prec == PFCG_FP64 && h->Nx == h->Ny && h->U <= 2 && (h->Nx == 2048 || h->Nx == 4096));
+}
 
 namespace {
 
@@ -1389,7 +1469,7 @@ template <typename T> void batch_args(pfcg_batch* b, std::vector<XArgs<T>>& xa, 
 		xa[i] = xargs<T>(h);
 		xa[i].acc = h->acc + ACC_NL;
 		xa[i].flag = b->d_flags + i;
-		ya[i] = yargs<T>(h);
+		ya[i] = yargs<T>(h, true);
 		ya[i].flag = b->d_flags + i; // NaN and wait time-out of problem i
 	}
 }
@@ -1433,13 +1513,13 @@ template <typename T> int batch_build(pfcg_batch* b) {
 	for (int i = 0; i < n; i++) {
 		pfcg_handle* h = b->h[i];
 		int c;
-		if (batch_ct(h)) {
+		if (batch_own_class(h)) {
 			auto it = key.find({h->U, h->Nx});
 			if (it == key.end()) {
 				c = (int)b->cls.size();
 				key[{h->U, h->Nx}] = c;
 				BatchClass k;
-				k.ct = true;
+				k.ct = batch_ct(h);
 				k.U = h->U;
 				k.N = h->Nx;
 				k.cx = h->cxs;
@@ -1453,13 +1533,14 @@ template <typename T> int batch_build(pfcg_batch* b) {
 			if (generic < 0) {
 				generic = (int)b->cls.size();
 				b->cls.push_back(BatchClass{});
-				b->cls.back().threads = 32;
 				members.emplace_back();
 			}
 			c = generic;
+		}
+		if (!b->cls[c].ct) {
 			BatchClass& k = b->cls[c];
-			k.threads = std::max(k.threads, std::max(h->cx.block, h->cy.block));
-			k.smem = std::max(k.smem, std::max(h->cx.smem, h->cy.smem));
+			k.threads = std::max(k.threads, std::max(h->cxs.block, h->cys.block));
+			k.smem = std::max(k.smem, std::max(h->cxs.smem, h->cys.smem));
 		}
 		members[c].push_back(i);
 	}
@@ -1474,7 +1555,7 @@ template <typename T> int batch_build(pfcg_batch* b) {
 		k.yoff = (int)yp.size();
 		for (int i : m) {
 			const pfcg_handle* h = b->h[i];
-			const int gx = k.ct ? h->cxs.grid : h->cx.grid, gy = k.ct ? h->cys.grid : h->cy.grid;
+			const int gx = h->cxs.grid, gy = h->cys.grid;
 			for (int t = 0; t < gx; t++) { xp.push_back(i); xl.push_back(t); }
 			for (int g = 0; g < gy; g++) { yp.push_back(i); yl.push_back(g); }
 		}
@@ -1484,7 +1565,7 @@ template <typename T> int batch_build(pfcg_batch* b) {
 		if (e == cudaSuccess) e = cudaEventCreateWithFlags(&k.done, cudaEventDisableTiming);
 		// the kernels' shared-memory limits are set here, outside any capture
 		for (int pass = 0; pass < 2 && e == cudaSuccess; pass++)
-			e = k.ct ? launch_ct_batch<T>(pass, k.U, k.N, nullptr, nullptr, nullptr, 0, pass ? k.cy : k.cx, k.stream)
+			e = k.ct ? launch_ct_batch(pass, k.U, k.N, nullptr, nullptr, nullptr, 0, pass ? k.cy : k.cx, k.stream)
 			         : launch_generic_batch<T>(pass, nullptr, nullptr, nullptr, 0, k.threads, k.smem, k.stream);
 		if (e != cudaSuccess) return bfail(e, "batch class");
 	}
@@ -1523,9 +1604,9 @@ template <typename T> int batch_launch_steps(pfcg_batch* b, int nsteps) {
 		if (e == cudaSuccess) e = cudaStreamWaitEvent(k.stream, b->fork, 0);
 		for (int s = 0; s < nsteps && e == cudaSuccess; s++) {
 			if (k.ct) {
-				e = launch_ct_batch<T>(0, k.U, k.N, b->d_xargs, xp + k.xoff, xl + k.xoff, k.xn, k.cx, k.stream);
+				e = launch_ct_batch(0, k.U, k.N, b->d_xargs, xp + k.xoff, xl + k.xoff, k.xn, k.cx, k.stream);
 				if (e == cudaSuccess)
-					e = launch_ct_batch<T>(1, k.U, k.N, b->d_yargs, yp + k.yoff, yl + k.yoff, k.yn, k.cy, k.stream);
+					e = launch_ct_batch(1, k.U, k.N, b->d_yargs, yp + k.yoff, yl + k.yoff, k.yn, k.cy, k.stream);
 			} else {
 				e = launch_generic_batch<T>(0, b->d_xargs, xp + k.xoff, xl + k.xoff, k.xn, k.threads, k.smem, k.stream);
 				if (e == cudaSuccess)
@@ -1566,8 +1647,10 @@ int pfcg_batch_create(int nprob, const pfcg_params* params, const int* Nx, const
 		// sizes with specialised kernels run them in their fixed shape; the
 		// others run the runtime-plan kernels, in the shape the autotuner picks
 		if (batch_ct(h)) continue;
-		h->cxs = h->cx;
-		h->cys = h->cy;
+		if (h->cxs.spec || h->cys.spec) {
+			h->geom.CC = h->ccr;
+			use_rt_steps(h);
+		}
 		if (autotune) {
 			const int r2 = pfcg_autotune(h, 5);
 			if (r2) {
@@ -1684,11 +1767,13 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[PFCG_NOALLOC_SC
 
 size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
-// exp(-2 pi i k / n) in FP32 from a double-precision sincospi
-__global__ void noalloc_twiddles_kernel(float2* tw, int n) {
-	for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+// the plan's twiddles in FP32 from a double-precision sincospi
+__global__ void noalloc_twiddles_kernel(float2* tw, const FftPlan p) {
+	for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < p.ntw; k += gridDim.x * blockDim.x) {
+		int num, den;
+		rt_twiddle_of(p, false, k, &num, &den);
 		double sn, cs;
-		sincospi(-2.0 * (double)k / (double)n, &sn, &cs);
+		sincospi(-2.0 * (double)num / (double)den, &sn, &cs);
 		tw[k] = make_float2((float)cs, (float)sn);
 	}
 }
@@ -1736,6 +1821,7 @@ extern "C" int pfcg_relax_noalloc(const pfcg_params* p, int Nx, int Ny, double d
 	// host-side description of the relaxation; no device memory is allocated
 	pfcg_handle h;
 	h.dev = dev;
+	h.nsm = prop.multiProcessorCount;
 	h.prec = PFCG_FP32;
 	h.model = to_model(p);
 	h.U = p->U;
@@ -1751,13 +1837,13 @@ extern "C" int pfcg_relax_noalloc(const pfcg_params* p, int Nx, int Ny, double d
 	h.celem = sizeof(float2);
 	h.stream = (cudaStream_t)stream;
 	int rc = 0;
-	if (!make_plan(Nx, max_radix(false), &h.px) || !make_plan(Ny, max_radix(false), &h.py))
+	if (!make_plan(Nx, false, &h.px) || !make_plan(Ny, false, &h.py))
 		rc = fail(&h, PFCG_ESIZE, "bad factorisation");
-	if (!rc) rc = choose_layout(&h, prop.multiProcessorCount);
+	if (!rc) rc = choose_layout(&h);
 	if (rc) return fail(nullptr, rc, h.err);
 	// the runtime-plan STEP kernels (the specialised ones need per-pass tables)
-	h.cxs = h.cx;
-	h.cys = h.cy;
+	h.geom.CC = h.ccr;
+	use_rt_steps(&h);
 
 	unsigned char* base = (unsigned char*)scratch;
 	const size_t nspec = (size_t)h.H * Ny;
@@ -1795,9 +1881,9 @@ extern "C" int pfcg_relax_noalloc(const pfcg_params* p, int Nx, int Ny, double d
 	// the workspace keeps the previous call's contents: clear what must start at zero
 	CKN(cudaMemsetAsync(h.acc, 0, sizeof(double) * ACC_N, h.stream));
 	CKN(cudaMemsetAsync(h.flag, 0, sizeof(int), h.stream));
-	noalloc_twiddles_kernel<<<(Nx + 255) / 256, 256, 0, h.stream>>>((float2*)h.twx, Nx);
+	noalloc_twiddles_kernel<<<(Nx + 255) / 256, 256, 0, h.stream>>>((float2*)h.twx, h.px);
 	CKN(cudaGetLastError());
-	noalloc_twiddles_kernel<<<(Ny + 255) / 256, 256, 0, h.stream>>>((float2*)h.twy, Ny);
+	noalloc_twiddles_kernel<<<(Ny + 255) / 256, 256, 0, h.stream>>>((float2*)h.twy, h.py);
 	CKN(cudaGetLastError());
 
 	// upload (means, r2c along x, FFT along y), steps, download

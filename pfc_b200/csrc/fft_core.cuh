@@ -42,6 +42,15 @@ template <typename V> __host__ __device__ __forceinline__ V cmul(V a, V b) {
 }
 template <typename V> __host__ __device__ __forceinline__ V cconj(V a) { a.y = -a.y; return a; }
 template <typename V, typename T> __host__ __device__ __forceinline__ V cscale(V a, T s) { a.x *= s; a.y *= s; return a; }
+// a s + c with one rounding, and a product that no addition may absorb: where a
+// sum has two products, these say which one is fused, so that kernels compiled
+// apart (one problem, a batch) round alike.
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+template <typename V, typename T> __device__ __forceinline__ V cfma_rn(V a, T s, V c) { c.x = fma_rn(a.x, s, c.x); c.y = fma_rn(a.y, s, c.y); return c; }
+template <typename V, typename T> __device__ __forceinline__ V cmul_rn(V a, T s) { a.x = mul_rn(a.x, s); a.y = mul_rn(a.y, s); return a; }
 // a * (sign * i)
 template <int SIGN, typename V> __host__ __device__ __forceinline__ V cmul_si(V a) {
 	V r;
@@ -216,6 +225,58 @@ template <int SIGN, typename T> __host__ __device__ __forceinline__ void dft7(cp
 	v[4] = csub(r3, i3);
 }
 
+// length 9 as 3 x 3: DFT3 on stride-3 subsequences, twiddles exp(SIGN 2 pi i q k / 9), DFT3
+template <int SIGN, typename T> __host__ __device__ __forceinline__ void dft9(cplx<T>* v) {
+	const T c1 = (T)0.76604444311897803520239265055542, s1 = (T)SIGN * (T)0.64278760968653932632264340990726;  // 2 pi / 9
+	const T c2 = (T)0.17364817766693034885171662676931, s2 = (T)SIGN * (T)0.98480775301220805936674302458953;  // 4 pi / 9
+	const T c4 = (T)-0.93969262078590838405410927732473, s4 = (T)SIGN * (T)0.34202014332566873304409961468226; // 8 pi / 9
+	cplx<T> a[3][3];
+#pragma unroll
+	for (int q = 0; q < 3; q++) {
+#pragma unroll
+		for (int r = 0; r < 3; r++) a[q][r] = v[3 * r + q];
+		dft3<SIGN, T>(a[q]);
+	}
+	a[1][1] = cmul(a[1][1], mk<T>(c1, s1));
+	a[1][2] = cmul(a[1][2], mk<T>(c2, s2));
+	a[2][1] = cmul(a[2][1], mk<T>(c2, s2));
+	a[2][2] = cmul(a[2][2], mk<T>(c4, s4));
+#pragma unroll
+	for (int k = 0; k < 3; k++) {
+		cplx<T> b[3] = {a[0][k], a[1][k], a[2][k]};
+		dft3<SIGN, T>(b);
+#pragma unroll
+		for (int s = 0; s < 3; s++) v[k + 3 * s] = b[s];
+	}
+}
+
+template <int R, int SIGN, typename T> __host__ __device__ __forceinline__ void dft(cplx<T>* v);
+
+// Coprime lengths N1 x N2 by the prime-factor (Good-Thomas) index maps, which
+// need no twiddles: input n = (N2 n1 + N1 n2) mod N, output k with
+// k = k1 mod N1 and k = k2 mod N2, so that exp(SIGN 2 pi i n k / N) =
+// exp(SIGN 2 pi i n1 k1 / N1) exp(SIGN 2 pi i n2 k2 / N2).
+__host__ __device__ constexpr int inv_mod(int a, int m, int x = 1) { return (a * x) % m == 1 % m ? x : inv_mod(a, m, x + 1); }
+template <int N1, int N2, int SIGN, typename T> __host__ __device__ __forceinline__ void dft_pfa(cplx<T>* v) {
+	constexpr int N = N1 * N2, C1 = N2 * inv_mod(N2 % N1, N1), C2 = N1 * inv_mod(N1 % N2, N2);
+	cplx<T> a[N2][N1];
+#pragma unroll
+	for (int n2 = 0; n2 < N2; n2++) {
+#pragma unroll
+		for (int n1 = 0; n1 < N1; n1++) a[n2][n1] = v[(N2 * n1 + N1 * n2) % N];
+		dft<N1, SIGN, T>(a[n2]);
+	}
+#pragma unroll
+	for (int k1 = 0; k1 < N1; k1++) {
+		cplx<T> b[N2];
+#pragma unroll
+		for (int n2 = 0; n2 < N2; n2++) b[n2] = a[n2][k1];
+		dft<N2, SIGN, T>(b);
+#pragma unroll
+		for (int k2 = 0; k2 < N2; k2++) v[(C1 * k1 + C2 * k2) % N] = b[k2];
+	}
+}
+
 template <int R, int SIGN, typename T> __host__ __device__ __forceinline__ void dft(cplx<T>* v) {
 	if constexpr (R == 2) dft2<SIGN, T>(v);
 	else if constexpr (R == 3) dft3<SIGN, T>(v);
@@ -224,107 +285,12 @@ template <int R, int SIGN, typename T> __host__ __device__ __forceinline__ void 
 	else if constexpr (R == 6) dft6<SIGN, T>(v);
 	else if constexpr (R == 7) dft7<SIGN, T>(v);
 	else if constexpr (R == 8) dft8<SIGN, T>(v);
+	else if constexpr (R == 9) dft9<SIGN, T>(v);
+	else if constexpr (R == 10) dft_pfa<2, 5, SIGN, T>(v);
+	else if constexpr (R == 12) dft_pfa<3, 4, SIGN, T>(v);
+	else if constexpr (R == 14) dft_pfa<2, 7, SIGN, T>(v);
+	else if constexpr (R == 15) dft_pfa<3, 5, SIGN, T>(v);
 	else if constexpr (R == 16) dft16<SIGN, T>(v);
-}
-
-// ---------------------------------------------------------------- plans --
-
-// A transform length n = RMAIN^nmain * rtail * 3^n3 * 5^n5 * 7^n7 with
-// rtail in {1, 2, 4, 8} (< RMAIN), done as runs of one radix each: nmain
-// passes of RMAIN, one of rtail, then the odd radices. A loop body holding a
-// single radix keeps register allocation tight; the host fills the counts.
-struct FftPlan {
-	int n;
-	int nmain;
-	int rtail;
-	int n3, n5, n7;
-};
-
-// ---------------------------------------------------------------- passes -
-
-// One Stockham pass over P sequences (sequence p starts at buf + p*ld, padded
-// indexing inside a sequence). nthreads threads take part, thread index t.
-// Only the butterfly inputs are live across the barrier; twiddles are read
-// after it, so a thread needs about MAXE complex registers plus one DFT's
-// temporaries.
-template <int R, int SIGN, int MAXE, typename T>
-__device__ __forceinline__ void stockham_pass(cplx<T>* buf, int ld, int P, int n, int Ns,
-                                              const cplx<T>* __restrict__ tw, int t, int nthreads) {
-	constexpr int NB = MAXE / R;
-	static_assert(NB >= 1, "MAXE too small for radix");
-	const int nR = n / R;
-	const int total = P * nR;
-	cplx<T> v[NB][R];
-#pragma unroll
-	for (int i = 0; i < NB; i++) {
-		const int b = t + i * nthreads;
-		if (b < total) {
-			const int p = b / nR;
-			const int j = b - p * nR;
-			const cplx<T>* in = buf + p * ld;
-#pragma unroll
-			for (int r = 0; r < R; r++) v[i][r] = in[pad<T>(j + r * nR)];
-		}
-	}
-	__syncthreads();
-	const int tstep = n / (Ns * R);
-#pragma unroll
-	for (int i = 0; i < NB; i++) {
-		const int b = t + i * nthreads;
-		if (b < total) {
-			const int p = b / nR;
-			const int j = b - p * nR;
-			const int jm = j % Ns;
-			if (jm > 0) {
-				const cplx<T>* twj = tw + jm * tstep;
-#pragma unroll
-				for (int r = 1; r < R; r++) {
-					cplx<T> w = __ldg(twj + (r - 1) * jm * tstep);
-					if (SIGN > 0) w.y = -w.y;
-					v[i][r] = cmul(v[i][r], w);
-				}
-			}
-			dft<R, SIGN, T>(v[i]);
-			cplx<T>* out = buf + p * ld;
-			const int d0 = (j - jm) * R + jm;
-#pragma unroll
-			for (int r = 0; r < R; r++) out[pad<T>(d0 + r * Ns)] = v[i][r];
-		}
-	}
-	__syncthreads();
-}
-
-// Full transform of P sequences of length plan.n in place in shared memory.
-// RMAIN = MAXE; requires ceil(P * n / (R * nthreads)) <= MAXE / R for each radix R.
-template <int SIGN, int MAXE, typename T>
-__device__ __forceinline__ void fft_batch(cplx<T>* buf, int ld, int P, const FftPlan& plan,
-                                          const cplx<T>* __restrict__ tw, int t, int nthreads) {
-	constexpr int RM = MAXE;
-	const int n = plan.n;
-	int Ns = 1;
-	for (int s = 0; s < plan.nmain; s++) {
-		stockham_pass<RM, SIGN, MAXE, T>(buf, ld, P, n, Ns, tw, t, nthreads);
-		Ns *= RM;
-	}
-	if constexpr (RM > 8) {
-		if (plan.rtail == 8) { stockham_pass<8, SIGN, MAXE, T>(buf, ld, P, n, Ns, tw, t, nthreads); Ns *= 8; }
-	}
-	if (plan.rtail == 4) { stockham_pass<4, SIGN, MAXE, T>(buf, ld, P, n, Ns, tw, t, nthreads); Ns *= 4; }
-	else if (plan.rtail == 2) { stockham_pass<2, SIGN, MAXE, T>(buf, ld, P, n, Ns, tw, t, nthreads); Ns *= 2; }
-	for (int s = 0; s < plan.n3; s++) { stockham_pass<3, SIGN, MAXE, T>(buf, ld, P, n, Ns, tw, t, nthreads); Ns *= 3; }
-	for (int s = 0; s < plan.n5; s++) { stockham_pass<5, SIGN, MAXE, T>(buf, ld, P, n, Ns, tw, t, nthreads); Ns *= 5; }
-	for (int s = 0; s < plan.n7; s++) { stockham_pass<7, SIGN, MAXE, T>(buf, ld, P, n, Ns, tw, t, nthreads); Ns *= 7; }
-}
-
-// Transforms S resident sequences in sub-batches of at most SB (so that the
-// thread count needed by one fft_batch call stays within the CTA).
-template <int SIGN, int MAXE, typename T>
-__device__ __forceinline__ void fft_batches(cplx<T>* buf, int ld, int S, int SB, const FftPlan& plan,
-                                            const cplx<T>* __restrict__ tw, int t, int nthreads) {
-	for (int b0 = 0; b0 < S; b0 += SB) {
-		const int nb = (S - b0) < SB ? (S - b0) : SB;
-		fft_batch<SIGN, MAXE, T>(buf + b0 * ld, ld, nb, plan, tw, t, nthreads);
-	}
 }
 
 // ------------------------------------------------- compile-time lengths --

@@ -26,7 +26,7 @@
 
 #include <cuda_runtime.h>
 
-#include "fft_core.cuh"
+#include "fft_rt.cuh"
 
 namespace pfcg {
 
@@ -85,6 +85,18 @@ template <typename T> struct StepK {
 };
 template <typename T> StepK<T> host_step_k(const Model& m, const Geom& g);
 
+// The x-pass's nonlinear constants in the transform precision, the same way
+template <typename T> struct NlK {
+	T lam[MAXU], del[MAXU], gam[MAXU][MAXU], alp[MAXU][MAXU];
+};
+template <typename T> NlK<T> host_nl_k(const Model& m);
+
+// Passes of the FP32 kernels for three and four fields (kernels_wide.cuh):
+// n = 16^nmain * rtail * 3^n3 * 5^n5 * 7^n7 with rtail in {1, 2, 4, 8}, in that order
+struct RadixPlan {
+	int n, nmain, rtail, n3, n5, n7;
+};
+
 template <typename T> struct XArgs {
 	cplx<T>* work;          // U arrays at stride wstride
 	long long wstride;
@@ -92,10 +104,14 @@ template <typename T> struct XArgs {
 	double* real;           // XP_C2R output / XP_R2C input: U fields of Ny*Nx doubles
 	double* acc;            // FP64 accumulators of the modes that add atomically (see part)
 	int* flag;              // NaN flag
-	const cplx<T>* tw;      // twiddles of length Nx
+	const cplx<T>* tw;      // twiddles of the run-time plan
 	const cplx<T>* twct;    // per-pass twiddle table of the specialised kernels
 	FftPlan plan;
 	int sb;                 // channel pairs per FFT call
+	NlK<T> k;               // STEP, run-time lengths: the nonlinear term's constants
+	const cplx<T>* wtw;     // FP32, U >= 3: n-entry twiddle table of kernels_wide.cuh (nullptr: kernels_rt.cuh)
+	RadixPlan wplan;
+	int wsb;
 	Model m;
 	Geom g;
 	// STEP: the block sums of the nonlinear term go to part[tile * U + u] (the
@@ -125,10 +141,13 @@ template <typename T> struct YArgs {
 	long long sstride;
 	double* mean;           // U, updated in place by YP_STEP at k = 0
 	double* acc;            // without part: FP64 sum of NL per field (read and cleared by YP_STEP)
-	const cplx<T>* tw;      // twiddles of length Ny
+	const cplx<T>* tw;      // twiddles of the run-time plan
 	const cplx<T>* twct;    // per-pass twiddle table of the specialised kernels
 	FftPlan plan;
 	int sb;                 // sequences per FFT call
+	const cplx<T>* wtw;     // as in XArgs
+	RadixPlan wplan;
+	int wsb;
 	Model m;
 	Geom g;
 	int wkind, wsrc;        // YP_WEIGHT: weight kind and source field
@@ -157,18 +176,18 @@ struct LaunchCfg {
 	int spec;  // 1: the compile-time specialised STEP kernel for this shape (2: never the fused y-pass)
 };
 
-// Shapes of the compile-time specialised STEP kernels (kernels_impl.cuh):
-// rows per x-pass tile and columns per y-pass CTA for length 2048 / 4096.
-int spec_rows(bool fp64, int U, int N);
-int spec_cols(bool fp64, int U, int N);
+// Shapes of the compile-time specialised STEP kernels (FP32, kernels_impl.cuh):
+// rows per x-pass tile and columns per y-pass CTA for length N.
+int spec_rows(int U, int N);
+int spec_cols(int U, int N);
 // threads and shared-memory bytes of those kernels
-int spec_x_threads(bool fp64, int U, int N);
-int spec_y_threads(bool fp64, int U, int N, bool fused);
-int spec_x_smem(bool fp64, int U, int N);
-int spec_y_smem(bool fp64, int U, int N);
-int spec_twiddles(bool fp64, int N);
+int spec_x_threads(int U, int N);
+int spec_y_threads(int U, int N, bool fused);
+int spec_x_smem(int U, int N);
+int spec_y_smem(int U, int N);
+int spec_twiddles(int N);
 // 1 if that y-pass reads its input columns straight from memory (TMA-capable)
-int spec_y_regio(bool fp64, int U, int N);
+int spec_y_regio(int U, int N);
 
 // Host-side launchers; return cudaGetLastError().
 template <typename T> cudaError_t launch_xpass(int mode, const XArgs<T>& a, const LaunchCfg& c, cudaStream_t s);
@@ -181,8 +200,6 @@ template <typename T> cudaError_t launch_ypass(int mode, const YArgs<T>& a, cons
 // those problems); launch_generic_batch: the runtime-plan kernels, any sizes.
 // nblk = 0 only prepares the kernels' shared-memory limits (call it before
 // capturing a graph).
-template <typename T> void prepare_batch_kernels();
-template <typename T>
 cudaError_t launch_ct_batch(int pass, int U, int N, const void* probs, const int* bp, const int* bl, int nblk,
                             const LaunchCfg& c, cudaStream_t s);
 template <typename T>
@@ -217,10 +234,14 @@ cudaError_t launch_fields_mul(double* a, double* b, const double* s, long long n
 cudaError_t launch_fields_gradpow(const double* g4, long long n, double power, double* out, cudaStream_t st);
 cudaError_t launch_scaled_acc(double* acc, const double* r, long long n, double* part, int nparts, cudaStream_t st);
 
-// elements per thread and main radix of the runtime-plan kernels; main radix
-// of the kernels specialised on the length N
-int max_elems_per_thread(bool fp64);
-int max_radix(bool fp64);
-int ct_radix(bool fp64, int N);
+// main radix of the kernels specialised on the length N
+int ct_radix(int N);
+
+// the kernels of run-time lengths with U fields (kernels_rt.cuh)
+template <typename T, int U> cudaError_t rt_launch_x(int mode, const XArgs<T>& a, const LaunchCfg& c, cudaStream_t s);
+template <typename T, int U> cudaError_t rt_launch_y(int mode, const YArgs<T>& a, const LaunchCfg& c, cudaStream_t s);
+// and those of kernels_wide.cuh: STEP, R2C and STEP, INIT
+template <int U> cudaError_t wide_launch_x(int mode, const XArgs<float>& a, const LaunchCfg& c, cudaStream_t s);
+template <int U> cudaError_t wide_launch_y(int mode, const YArgs<float>& a, const LaunchCfg& c, cudaStream_t s);
 
 } // namespace pfcg

@@ -1,94 +1,62 @@
 // Precision-independent kernels and helpers of the B200 relaxation path.
 #include "kernels_impl.cuh"
 
+#include <algorithm>
+
 namespace pfcg {
 
-int max_elems_per_thread(bool fp64) { (void)fp64; return RT_MAXE; }
-int max_radix(bool fp64) { (void)fp64; return RT_MAXE; }
-int ct_radix(bool fp64, int N) { return fp64 ? ct_maxe<double>(N) : ct_maxe<float>(N); }
+int ct_radix(int N) { return ct_maxe<float>(N); }
 
 // 0 where the size has no specialised kernel (Spec in kernels_impl.cuh)
-int spec_rows(bool fp64, int U, int N) { return fp64 ? Spec<double>::xr(U, N) : Spec<float>::xr(U, N); }
-int spec_cols(bool fp64, int U, int N) { return fp64 ? Spec<double>::ycc(U, N) : Spec<float>::ycc(U, N); }
+int spec_rows(int U, int N) { return Spec<float>::xr(U, N); }
+int spec_cols(int U, int N) { return Spec<float>::ycc(U, N); }
 
-template <typename T> static int ct_twn(int N) {
-	constexpr int M = FftCfg<T>::MAXE;
+// f(integral constant N) for the specialised length N, 0 for others
+template <typename F> static int for_ct_length(int N, F f) {
 	switch (N) {
-	case 4096: return CtPlan<4096, M>::TWN;
-	case 2048: return CtPlan<2048, M>::TWN;
-	}
-	if constexpr (M == 16) {
-		switch (N) {
-		case 384: return CtPlan<384, ct_maxe<T>(384)>::TWN;
-		case 1536: return CtPlan<1536, M>::TWN;
-		case 1024: return CtPlan<1024, M>::TWN;
-		case 768: return CtPlan<768, M>::TWN;
-		case 512: return CtPlan<512, M>::TWN;
-		case 256: return CtPlan<256, M>::TWN;
-		}
+	case 4096: return f(std::integral_constant<int, 4096>());
+	case 2048: return f(std::integral_constant<int, 2048>());
+	case 1536: return f(std::integral_constant<int, 1536>());
+	case 1024: return f(std::integral_constant<int, 1024>());
+	case 768: return f(std::integral_constant<int, 768>());
+	case 512: return f(std::integral_constant<int, 512>());
+	case 384: return f(std::integral_constant<int, 384>());
+	case 256: return f(std::integral_constant<int, 256>());
 	}
 	return 0;
 }
-int spec_twiddles(bool fp64, int N) { return fp64 ? ct_twn<double>(N) : ct_twn<float>(N); }
+int spec_twiddles(int N) {
+	return for_ct_length(N, [](auto n) { return CtPlan<n.value, ct_maxe<float>(n.value)>::TWN; });
+}
 
 // whether the specialised y-pass (not the register-fused variant) of this
 // shape takes its first transform's input straight from memory (register
 // ends, the path that can load by TMA)
-template <typename T, int U, int N> static bool y_regio() {
-	constexpr int CC = Spec<T>::ycc(U, N), R = Spec<T>::xr(U, N);
-	using C = YCfg<T, U, N, CC, R, false>;
-	constexpr int M = C::MAXE;
-	return C::NSUB == C::S && C::S * (N / M) == C::NT && CtPlan<N, M>::FUSABLE;
+template <int U, int N> static bool y_regio() {
+	using C = YCfg<float, U, N, Spec<float>::ycc(U, N), Spec<float>::xr(U, N), false>;
+	return C::NSUB == C::S && C::S * (N / C::MAXE) == C::NT && CtPlan<N, C::MAXE>::FUSABLE;
 }
-template <typename T, int U> static bool y_regio_n(int N) {
-	switch (N) {
-	case 4096: return y_regio<T, U, 4096>();
-	case 2048: return y_regio<T, U, 2048>();
-	}
-	if constexpr (sizeof(T) == 4) {
-		switch (N) {
-		case 1536: return y_regio<T, U, 1536>();
-		case 1024: return y_regio<T, U, 1024>();
-		case 768: return y_regio<T, U, 768>();
-		case 512: return y_regio<T, U, 512>();
-		case 384: return y_regio<T, U, 384>();
-		case 256: return y_regio<T, U, 256>();
-		}
-	}
-	return false;
-}
-int spec_y_regio(bool fp64, int U, int N) {
-	if (U == 1) return fp64 ? y_regio_n<double, 1>(N) : y_regio_n<float, 1>(N);
-	if (U == 2) return fp64 ? y_regio_n<double, 2>(N) : y_regio_n<float, 2>(N);
+int spec_y_regio(int U, int N) {
+	if (U == 1) return for_ct_length(N, [](auto n) -> int { return y_regio<1, n.value>(); });
+	if (U == 2) return for_ct_length(N, [](auto n) -> int { return y_regio<2, n.value>(); });
 	return 0;
 }
 
-int spec_x_threads(bool fp64, int U, int N) {
-	const int maxe = ct_radix(fp64, N);
-	const int P = (U * spec_rows(fp64, U, N) + 1) / 2;
-	return P * N / maxe <= MAXNT ? P * N / maxe : MAXNT;
+int spec_x_threads(int U, int N) {
+	const int P = (U * spec_rows(U, N) + 1) / 2;
+	return std::min(P * N / ct_radix(N), MAXNT);
 }
-int spec_y_threads(bool fp64, int U, int N, bool fused) {
+int spec_y_threads(int U, int N, bool fused) {
 	// fused y-pass: one thread per (field, column, butterfly); otherwise as many
 	// sequences per FFT call as fit MAXNT threads
-	const int maxe = ct_radix(fp64, N);
-	const int S = U * spec_cols(fp64, U, N);
-	if (fused && U <= 2 && S * N / maxe <= MAXNT) return S * N / maxe;
-	if (S * N / maxe <= MAXNT) return S * N / maxe;
-	return MAXNT;
+	(void)fused;
+	return std::min(U * spec_cols(U, N) * N / ct_radix(N), MAXNT);
 }
-int spec_x_smem(bool fp64, int U, int N) {
-	const int P = (U * spec_rows(fp64, U, N) + 1) / 2;
-	const int ce = fp64 ? 16 : 8;
-	const int ld = fp64 ? padded_len<double>(N) : padded_len<float>(N);
-	return (P * ld + spec_twiddles(fp64, N)) * ce;
+int spec_x_smem(int U, int N) {
+	const int P = (U * spec_rows(U, N) + 1) / 2;
+	return (P * padded_len<float>(N) + spec_twiddles(N)) * 8;
 }
-int spec_y_smem(bool fp64, int U, int N) {
-	const int S = U * spec_cols(fp64, U, N);
-	const int ce = fp64 ? 16 : 8;
-	const int ld = fp64 ? padded_len<double>(N) : padded_len<float>(N);
-	return (S * ld + spec_twiddles(fp64, N)) * ce;
-}
+int spec_y_smem(int U, int N) { return (U * spec_cols(U, N) * padded_len<float>(N) + spec_twiddles(N)) * 8; }
 
 // ------------------------------------------------------ energy density --
 template <int U>
@@ -290,6 +258,21 @@ template <typename T> StepK<T> host_step_k(const Model& m, const Geom& g) {
 	return k;
 }
 
+template <typename T> NlK<T> host_nl_k(const Model& m) {
+	NlK<T> k{};
+	for (int u = 0; u < MAXU; u++) {
+		k.lam[u] = (T)m.lambda[u];
+		k.del[u] = (T)m.delta[u];
+		for (int v = 0; v < MAXU; v++) {
+			k.gam[u][v] = (T)m.gamma[u][v];
+			k.alp[u][v] = (T)m.alpha[u][v];
+		}
+	}
+	return k;
+}
+
+template NlK<float> host_nl_k<float>(const Model&);
+template NlK<double> host_nl_k<double>(const Model&);
 template StepK<float> host_step_k<float>(const Model&, const Geom&);
 template StepK<double> host_step_k<double>(const Model&, const Geom&);
 

@@ -31,9 +31,6 @@ namespace pfcg {
 template <typename T> struct FftCfg;
 template <> struct FftCfg<float> { static constexpr int MAXE = 16; };
 template <> struct FftCfg<double> { static constexpr int MAXE = 8; };
-// and of the runtime-plan kernels, in both precisions: 16 elements per thread
-// let 512 threads hold one 8192-point sequence (and 7168 / 7680 with a factor 7 / 5)
-constexpr int RT_MAXE = 16;
 // Main radix (elements per thread) of the kernels specialised on the length N:
 // FftCfg's, except FP32 384 = 8 * 6 * 8, which has no radix-16 form with
 // radix-16 first and last passes.
@@ -110,7 +107,7 @@ __device__ __forceinline__ double k2_of(int kx, int ky, const Geom& g, double dx
 template <typename T> __device__ __forceinline__ T k2_step(int kx, int ky, int Ny, T dkx, T dky) {
 	const T kxv = (T)kx * dkx;
 	const T kyv = (T)(ky < Ny / 2 ? ky : ky - Ny) * dky;
-	return kxv * kxv + kyv * kyv;
+	return fma_rn(kyv, kyv, mul_rn(kxv, kxv));
 }
 
 // phi1(x) = (exp(x) - 1) / x given A = exp(x): Taylor series to x^6 / 7! for
@@ -171,10 +168,10 @@ __device__ __forceinline__ void entry_coef(const StepK<T>& K, T k2, T (&A)[U], T
 			for (int v = u + 1; v < U; v++) {
 				T d2 = K.mu2[u][v] - k2;
 				d2 *= d2;
-				cu[p++] = K.beta[u][v] * d2 + K.eps[u][v] * G2;
+				cu[p++] = fma_rn(K.beta[u][v], d2, mul_rn(K.eps[u][v], G2));
 			}
 	}
-	const T o = K.cc - (T)1 - K.cc * k2;
+	const T o = fma_rn(-K.cc, k2, K.cc - (T)1);
 #pragma unroll
 	for (int u = 0; u < U; u++) {
 		T P = (T)1;
@@ -182,9 +179,9 @@ __device__ __forceinline__ void entry_coef(const StepK<T>& K, T k2, T (&A)[U], T
 		for (int w = 0; w < MAXW; w++)
 			if (w < K.W[u]) {
 				const T q = K.nu2[u][w] - k2;
-				P *= K.omega[u][w] * q * q + K.phi[u][w];
+				P *= fma_rn(mul_rn(K.omega[u][w], q), q, K.phi[u][w]);
 			}
-		const T av = K.alpha[u] + K.betad[u] * P;
+		const T av = fma_rn(K.betad[u], P, K.alpha[u]);
 		const T x = o * av * K.dt;
 		if (K.semi) {
 			A[u] = (T)1 / ((T)1 - x);
@@ -195,13 +192,6 @@ __device__ __forceinline__ void entry_coef(const StepK<T>& K, T k2, T (&A)[U], T
 		if constexpr (sizeof(T) == 4) Bn[u] = o * K.dt * phi1f(x, A[u]);
 		else Bn[u] = (av == (T)0) ? o * K.dt : etd_b<T>(A[u], x, av);
 	}
-}
-
-// k^2 of entry (kx, ky) as the y-pass STEP computes it
-template <typename T>
-__device__ __forceinline__ T step_k2(int kx, int ky, int Ny, T dkxT, T dkyT, const Geom& g) {
-	if constexpr (sizeof(T) == 4) return k2_step<T>(kx, ky, Ny, dkxT, dkyT);
-	else return (T)k2_of(kx, ky, g, g.dx, g.dy);
 }
 
 // Hermitian projection of one resident column (kx = 0 or kx = Nx/2): entry ky
@@ -583,209 +573,26 @@ __device__ __forceinline__ void ypass_step_fused(const YArgs<T>& a, cplx<T>* sm,
 			dst[(long long)(y / RC) * tileH + y % RC] = rb.v[0][r];
 		}
 	}
-	if (kx0 == 0) ypass_mean_update<T, U>(a, tid, NT);
 }
 
 // ----------------------------------------------------------------- x-pass --
 
-// Body of the x-pass for row tile `tile`; called by xpass_kernel (one problem)
-// and by xpass_batch_kernel (many problems in one launch).
+// Body of the x-pass STEP for row tile `tile`; called by xpass_kernel (one
+// problem) and by xpass_ct_batch_kernel (many problems in one launch).
 // (in the fused instantiations the code after the early return is unreachable,
 // which is intended)
 #pragma nv_diag_suppress 128
-template <typename T, int U, int MODE, int NC, int RC>
+template <typename T, int U, int NC, int RC>
 __device__ __forceinline__ void xpass_body(const XArgs<T>& a, const int tile, const bool load_tw = true) {
 	using C = XCfg<T, U, NC, RC>;
 	constexpr int MAXE = C::MAXE;
 	extern __shared__ __align__(128) unsigned char smem_raw[];
 	cplx<T>* sm = reinterpret_cast<cplx<T>*>(smem_raw);
-	const int Nx = C::CT ? NC : a.g.Nx;
-	const int Ny = a.g.Ny;
-	const int H = Nx / 2 + 1;
-	const int R = C::CT ? RC : a.g.R;
-	const int CH = U * R;
-	const int P = (CH + 1) >> 1;
-	const int ld = C::CT ? C::LD : padded_len<T>(Nx);
-	const int y0 = tile * R;
 	const int tid = threadIdx.x;
-	const int nt = C::CT ? C::NT : (int)blockDim.x;
-	const long long tofs = (long long)tile * H * R;
-	cplx<T>* tws = sm + (C::CT ? C::P * C::LD : 0);
-	constexpr bool XFUSED = MODE == XP_STEP && C::CT && CtPlan<(C::CT ? NC : 256), MAXE>::FUSABLE && C::NSUB == C::P &&
-	                        U <= 2 && (U * RC) % 2 == 0;
-	if constexpr (C::CT && !XFUSED) {
-		if (load_tw) copy_twiddles<T, C::TWN, C::NT>(tws, a.twct, tid);
-	}
-	if constexpr (XFUSED) {
-		// the fused pass copies the twiddles after issuing its tile loads
-		xpass_step_fused<T, U, NC, RC, C::P, C::NT, MAXE>(a, sm, tws, tile, tid, load_tw);
-		return;
-	}
-
-	double off[U];
-#pragma unroll
-	for (int u = 0; u < U; u++) off[u] = a.off ? a.off[u] : 0.0;
-
-	if constexpr (MODE == XP_R2C) {
-		// real rows (minus their mean) -> pairs of channels in one complex sequence
-		for (int x = tid; x < Nx; x += nt) {
-#pragma unroll
-			for (int p = 0; p < MAX_CH / 2; p++) {
-				if (p < P) {
-					const int c0 = 2 * p, c1 = 2 * p + 1;
-					const int u0 = c0 % U, r0 = c0 / U, u1 = c1 % U, r1 = c1 / U;
-					const double v0 = a.real[((long long)u0 * Ny + y0 + r0) * Nx + x] - (a.off ? a.off[u0] : 0.0);
-					const double v1 = (c1 < CH) ? a.real[((long long)u1 * Ny + y0 + r1) * Nx + x] - (a.off ? a.off[u1] : 0.0) : 0.0;
-					sm[p * ld + pad<T>(x)] = mk<T>((T)v0, (T)v1);
-				}
-			}
-		}
-	} else {
-		// Hermitian-extended spectra of channel pairs: C = A + iB on 0..Nx/2,
-		// conj(A) + i conj(B) on Nx/2+1..Nx-1; imaginary parts of the kx = 0 and
-		// kx = Nx/2 entries are dropped like a c2r transform does.
-		for (int k = tid; k < H; k += nt) {
-			cplx<T> y[MAX_CH];
-#pragma unroll
-			for (int c = 0; c < MAX_CH; c++) {
-				y[c] = mk<T>((T)0, (T)0);
-				if (c < CH) {
-					const int u = c % U, r = c / U;
-					y[c] = a.work[u * a.wstride + tofs + (long long)k * R + r];
-				}
-			}
-			const bool selfc = (k == 0) || (2 * k == Nx);
-#pragma unroll
-			for (int p = 0; p < MAX_CH / 2; p++) {
-				if (p < P) {
-					cplx<T> A = y[2 * p], B = y[2 * p + 1];
-					if (selfc) { A.y = (T)0; B.y = (T)0; }
-					sm[p * ld + pad<T>(k)] = mk<T>(A.x - B.y, A.y + B.x);
-					if (k > 0 && 2 * k < Nx) sm[p * ld + pad<T>(Nx - k)] = mk<T>(A.x + B.y, B.x - A.y);
-				}
-			}
-		}
-		__syncthreads();
-		if constexpr (C::CT) fft_ct<NC, MAXE, C::P, C::NSUB, C::NT, +1, T>(sm, tws, tid);
-		else fft_batches<+1, MAXE, T>(sm, ld, P, a.sb, a.plan, a.tw, tid, nt);
-	}
-
-	if constexpr (MODE == XP_STEP || MODE == XP_EVAL || MODE == XP_C2R) {
-		constexpr int NACC = (MODE == XP_EVAL) ? 1 + U : U;
-		double acc[NACC];
-#pragma unroll
-		for (int i = 0; i < NACC; i++) acc[i] = 0.0;
-		bool nan = false;
-		T lam[U], del[U], gam[U][U], alp[U][U], offT[U];
-#pragma unroll
-		for (int u = 0; u < U; u++) {
-			offT[u] = (T)off[u];
-			lam[u] = (T)a.m.lambda[u];
-			del[u] = (T)a.m.delta[u];
-#pragma unroll
-			for (int v = 0; v < U; v++) { gam[u][v] = (T)a.m.gamma[u][v]; alp[u][v] = (T)a.m.alpha[u][v]; }
-		}
-		for (int x = tid; x < Nx; x += nt) {
-			T z[MAX_CH];
-#pragma unroll
-			for (int p = 0; p < MAX_CH / 2; p++) {
-				if (p < P) {
-					const cplx<T> v = sm[p * ld + pad<T>(x)];
-					z[2 * p] = v.x;
-					z[2 * p + 1] = v.y;
-				}
-			}
-#pragma unroll
-			for (int r = 0; r < MAX_CH / U; r++) {
-				if (r < R) {
-					if constexpr (MODE == XP_STEP) {
-						T mv[U], mc[U];
-#pragma unroll
-						for (int u = 0; u < U; u++) {
-							mv[u] = z[r * U + u] + offT[u];
-							nan |= (mv[u] != mv[u]);
-							mc[u] = (T)0;
-						}
-#pragma unroll
-						for (int u = 0; u < U - 1; u++)
-#pragma unroll
-							for (int v = u + 1; v < U; v++) {
-								mc[u] += alp[u][v] * mv[v] + (T)0.5 * gam[u][v] * ((T)2 * mv[u] * mv[v] + mv[v] * mv[v]);
-								mc[v] += alp[u][v] * mv[u] + (T)0.5 * gam[u][v] * ((T)2 * mv[v] * mv[u] + mv[u] * mv[u]);
-							}
-#pragma unroll
-						for (int u = 0; u < U; u++) {
-							const T m2 = mv[u] * mv[u];
-							const T nl = lam[u] + gam[u][u] * m2 + del[u] * mv[u] * m2 + mc[u];
-							z[r * U + u] = nl;
-							acc[u] += (double)nl;
-						}
-					} else if constexpr (MODE == XP_EVAL) {
-						double mv[U];
-#pragma unroll
-						for (int u = 0; u < U; u++) mv[u] = (double)z[r * U + u] + off[u];
-						double f = 0.0;
-#pragma unroll
-						for (int u = 0; u < U; u++) {
-							const double n1 = mv[u], n2 = n1 * n1;
-							f += a.m.lambda[u] * n1 + 0.5 * a.m.alpha[u][u] * n2 + (1.0 / 3.0) * a.m.gamma[u][u] * n1 * n2 +
-							     0.25 * a.m.delta[u] * n2 * n2;
-#pragma unroll
-							for (int v = u + 1; v < U; v++) {
-								const double nv = mv[v];
-								f += a.m.alpha[u][v] * n1 * nv + 0.5 * a.m.gamma[u][v] * (n2 * nv + n1 * nv * nv);
-							}
-							acc[1 + u] += n1;
-						}
-						acc[0] += f;
-					} else {
-#pragma unroll
-						for (int u = 0; u < U; u++)
-							a.real[((long long)u * Ny + y0 + r) * Nx + x] = (double)z[r * U + u] + off[u];
-					}
-				}
-			}
-			if constexpr (MODE == XP_STEP) {
-#pragma unroll
-				for (int p = 0; p < MAX_CH / 2; p++)
-					if (p < P) sm[p * ld + pad<T>(x)] = mk<T>(z[2 * p], (2 * p + 1 < CH) ? z[2 * p + 1] : (T)0);
-			}
-		}
-		if constexpr (MODE == XP_STEP) {
-			if (nan) atomicOr(a.flag, 1);
-			block_reduce_put<NACC>(acc, a.part ? a.part + (long long)tile * U : a.acc, a.part != nullptr);
-		} else if constexpr (MODE == XP_EVAL) {
-			block_reduce_put<NACC>(acc, a.part ? a.part + (long long)tile * NACC : a.acc, a.part != nullptr);
-		}
-	}
-
-	if constexpr (MODE == XP_STEP || MODE == XP_R2C) {
-		__syncthreads();
-		if constexpr (C::CT) fft_ct<NC, MAXE, C::P, C::NSUB, C::NT, -1, T>(sm, tws, tid);
-		else fft_batches<-1, MAXE, T>(sm, ld, P, a.sb, a.plan, a.tw, tid, nt);
-		// split each pair: Za = (C[k] + conj C[-k]) / 2, Zb = (C[k] - conj C[-k]) / (2i)
-		const T half = (T)0.5;
-		for (int k = tid; k < H; k += nt) {
-			const int km = (k == 0) ? 0 : Nx - k;
-			cplx<T> zz[MAX_CH];
-#pragma unroll
-			for (int p = 0; p < MAX_CH / 2; p++) {
-				if (p < P) {
-					const cplx<T> Ck = sm[p * ld + pad<T>(k)];
-					const cplx<T> Cm = sm[p * ld + pad<T>(km)];
-					zz[2 * p] = mk<T>(half * (Ck.x + Cm.x), half * (Ck.y - Cm.y));
-					zz[2 * p + 1] = mk<T>(half * (Ck.y + Cm.y), half * (Cm.x - Ck.x));
-				}
-			}
-#pragma unroll
-			for (int c = 0; c < MAX_CH; c++) {
-				if (c < CH) {
-					const int u = c % U, r = c / U;
-					a.work[u * a.wstride + tofs + (long long)k * R + r] = zz[c];
-				}
-			}
-		}
-	}
+	cplx<T>* tws = sm + C::P * C::LD;
+	static_assert(CtPlan<NC, MAXE>::FUSABLE && C::NSUB == C::P && U <= 2 && (U * RC) % 2 == 0, "shapes of the fused x-pass");
+	// the fused pass copies the twiddles after issuing its tile loads
+	xpass_step_fused<T, U, NC, RC, C::P, C::NT, MAXE>(a, sm, tws, tile, tid, load_tw);
 }
 #pragma nv_diag_default 128
 
@@ -796,7 +603,7 @@ __device__ __forceinline__ void xpass_body(const XArgs<T>& a, const int tile, co
 // Row tiles blockIdx.x, + gridDim.x, ... < ntiles: a grid of fewer CTAs than
 // tiles keeps each CTA resident over several tiles, loading the per-pass
 // twiddle table of the specialised kernels once.
-template <typename T, int U, int MODE, int NC, int RC>
+template <typename T, int U, int NC, int RC>
 __global__ void __launch_bounds__(XCfg<T, U, NC, RC>::NT, XCfg<T, U, NC, RC>::MINB)
     xpass_kernel(const XArgs<T> a, int ntiles) {
 	// programmatic dependent launch (pdl_launch): the previous kernel's results
@@ -805,7 +612,7 @@ __global__ void __launch_bounds__(XCfg<T, U, NC, RC>::NT, XCfg<T, U, NC, RC>::MI
 	asm volatile("griddepcontrol.launch_dependents;");
 	for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
 		if (t != (int)blockIdx.x) __syncthreads(); // the previous tile's readers of shared memory are done
-		xpass_body<T, U, MODE, NC, RC>(a, t, t == (int)blockIdx.x);
+		xpass_body<T, U, NC, RC>(a, t, t == (int)blockIdx.x);
 	}
 }
 
@@ -855,38 +662,30 @@ __device__ __forceinline__ bool tma_wait(unsigned bar, unsigned parity, unsigned
 	}
 }
 
-template <typename T, int U, int MODE, int NC, int CCC, int RC, bool FUSEDK = true>
+template <typename T, int U, int NC, int CCC, int RC, bool FUSEDK = true>
 __device__ __forceinline__ void ypass_body(const YArgs<T>& a, const int grp, const bool load_tw = true, const int iter = 0) {
 	using C = YCfg<T, U, NC, CCC, RC, FUSEDK>;
 	constexpr int MAXE = C::MAXE;
 	extern __shared__ __align__(128) unsigned char smem_raw[];
 	cplx<T>* sm = reinterpret_cast<cplx<T>*>(smem_raw);
 	const int Nx = a.g.Nx, H = a.g.H;
-	const int Ny = C::CT ? NC : a.g.Ny;
-	const int R = C::CT ? RC : a.g.R;
-	const int CC = C::CT ? CCC : a.g.CC;
-	const int S = U * CC;
-	const int ld = C::CT ? C::LD : padded_len<T>(Ny);
-	const int kx0 = grp * CC;
-	const int ncol = min(CC, H - kx0);
-	const int ntile = Ny / R;
-	const long long tileH = (long long)H * R;
-	const int chunk = CC * R;
+	const int kx0 = grp * CCC;
 	const int tid = threadIdx.x;
-	const int nt = C::CT ? C::NT : (int)blockDim.x;
-	cplx<T>* tws = sm + (C::CT ? C::S * C::LD : 0);
-	// (copying the twiddles after the register-end loads instead, as the
-	// x-pass does, measured 2 % slower here)
-	if constexpr (C::CT) {
-		if (load_tw)
-			for (int i = tid; i < C::TWN; i += C::NT) tws[i] = a.twct[i];
-	}
-
-	if constexpr (MODE == YP_STEP && C::FUSED && FUSEDK) {
-		ypass_step_fused<T, U, NC, CCC, RC, C::S, C::NT, MAXE>(a, sm, tws, kx0, ncol, tid);
+	if (kx0 >= H) { // the CTA of the k = 0 update
+		ypass_mean_update<T, U>(a, tid, C::NT);
 		return;
 	}
-	if constexpr (MODE == YP_STEP && C::CT) {
+	const int ncol = min(CCC, H - kx0);
+	const long long tileH = (long long)H * RC;
+	cplx<T>* tws = sm + C::S * C::LD;
+	// (copying the twiddles after the register-end loads instead, as the
+	// x-pass does, measured 2 % slower here)
+	if (load_tw)
+		for (int i = tid; i < C::TWN; i += C::NT) tws[i] = a.twct[i];
+
+	if constexpr (C::FUSED && FUSEDK) {
+		ypass_step_fused<T, U, NC, CCC, RC, C::S, C::NT, MAXE>(a, sm, tws, kx0, ncol, tid);
+	} else {
 		// this group's spectral-state columns into L2 now, so that the update's
 		// loads after the forward transform find them there: one 128-byte line
 		// per prefetch, all inside the live columns
@@ -896,75 +695,69 @@ __device__ __forceinline__ void ypass_body(const YArgs<T>& a, const int grp, con
 			const char* line = reinterpret_cast<const char*>(a.spec + u * a.sstride + (long long)kx0 * NC) + rest * 128;
 			asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
 		}
-	}
 
-	// Register ends (STEP, one butterfly per thread per pass): the forward
-	// transform's first pass takes its inputs straight from global memory and
-	// the inverse transform's last pass stores straight to it, which saves the
-	// shared-memory round trip and barrier of a separate load and store phase.
-	constexpr int NCX = C::CT ? NC : 256;
-	using PLX = CtPlan<NCX, MAXE>;
-	constexpr bool REGIO = C::CT && MODE == YP_STEP && !(C::FUSED && FUSEDK) && C::NSUB == C::S &&
-	                       C::S * (NCX / MAXE) == C::NT && PLX::FUSABLE;
-	using RBY = RegBlock<NCX, MAXE, C::S, C::NT, T>;
-	constexpr int CCX = C::CT ? CCC : 1;
-	// global address of element y of resident sequence p (field p / CCC, column p % CCC)
-	auto gaddr = [&](int p, int y) -> long long {
-		return (long long)(p / CCX) * a.wstride + (long long)(y / R) * tileH + (long long)(kx0 + p % CCX) * R +
-		       y % R;
-	};
-	bool regio = false;
-	if constexpr (REGIO) {
-		if (a.regio) {
-			regio = true;
-			RBY rb;
-			if (a.tmap) {
-				__shared__ __align__(8) unsigned long long tbar;
-				const unsigned bar = (unsigned)__cvta_generic_to_shared(&tbar);
-				if (iter == 0) {
-					if (tid == 0) tma_bar_init(bar);
-					__syncthreads();
-				}
-				constexpr int NTILE = NCX / RC;
-				if (tid == 0) {
-					const int tb = a.tma_tiles;
-					// earlier generic accesses to the buffer before the async-proxy writes
-					asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-					tma_expect(bar, (unsigned)(U * NCX * CCX * sizeof(cplx<T>)) + a.tma_extra);
-					for (int u = 0; u < U; u++)
-						for (int t0 = 0; t0 < NTILE; t0 += tb)
-							tma_load4((unsigned)__cvta_generic_to_shared(sm + (u * NTILE + t0) * CCX * RC), a.tmap, 0, kx0,
-							          t0, u, bar);
-				}
-				if (!tma_wait(bar, (unsigned)(iter & 1), a.tma_timeout_ns) && tid == 0) atomicOr(a.flag, FLAG_TIMEOUT);
+		// Register ends (one butterfly per thread per pass): the forward
+		// transform's first pass takes its inputs straight from global memory and
+		// the inverse transform's last pass stores straight to it, which saves the
+		// shared-memory round trip and barrier of a separate load and store phase.
+		using PLX = CtPlan<NC, MAXE>;
+		constexpr bool REGIO = C::NSUB == C::S && C::S * (NC / MAXE) == C::NT && PLX::FUSABLE;
+		using RBY = RegBlock<NC, MAXE, C::S, C::NT, T>;
+		// global address of element y of resident sequence p (field p / CCC, column p % CCC)
+		auto gaddr = [&](int p, int y) -> long long {
+			return (long long)(p / CCC) * a.wstride + (long long)(y / RC) * tileH + (long long)(kx0 + p % CCC) * RC + y % RC;
+		};
+		bool regio = false;
+		if constexpr (REGIO) {
+			if (a.regio) {
+				regio = true;
+				RBY rb;
+				if (a.tmap) {
+					__shared__ __align__(8) unsigned long long tbar;
+					const unsigned bar = (unsigned)__cvta_generic_to_shared(&tbar);
+					if (iter == 0) {
+						if (tid == 0) tma_bar_init(bar);
+						__syncthreads();
+					}
+					constexpr int NTILE = NC / RC;
+					if (tid == 0) {
+						const int tb = a.tma_tiles;
+						// earlier generic accesses to the buffer before the async-proxy writes
+						asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+						tma_expect(bar, (unsigned)(U * NC * CCC * sizeof(cplx<T>)) + a.tma_extra);
+						for (int u = 0; u < U; u++)
+							for (int t0 = 0; t0 < NTILE; t0 += tb)
+								tma_load4((unsigned)__cvta_generic_to_shared(sm + (u * NTILE + t0) * CCC * RC), a.tmap, 0, kx0,
+								          t0, u, bar);
+					}
+					if (!tma_wait(bar, (unsigned)(iter & 1), a.tma_timeout_ns) && tid == 0) atomicOr(a.flag, FLAG_TIMEOUT);
 #pragma unroll
-				for (int i = 0; i < RBY::NB; i++) {
-					const int p = RBY::seq(tid, i);
+					for (int i = 0; i < RBY::NB; i++) {
+						const int p = RBY::seq(tid, i);
 #pragma unroll
-					for (int r = 0; r < MAXE; r++) {
-						const int y = RBY::pos(tid, i, r);
-						rb.v[i][r] = sm[((p / CCX) * NTILE + y / RC) * CCX * RC + (p % CCX) * RC + y % RC];
+						for (int r = 0; r < MAXE; r++) {
+							const int y = RBY::pos(tid, i, r);
+							rb.v[i][r] = sm[((p / CCC) * NTILE + y / RC) * CCC * RC + (p % CCC) * RC + y % RC];
+						}
+					}
+				} else {
+#pragma unroll
+					for (int i = 0; i < RBY::NB; i++) {
+						const int p = RBY::seq(tid, i);
+						const bool live = p % CCC < ncol;
+#pragma unroll
+						for (int r = 0; r < MAXE; r++)
+							rb.v[i][r] = live ? a.work[gaddr(p, RBY::pos(tid, i, r))] : mk<T>((T)0, (T)0);
 					}
 				}
-			} else {
-#pragma unroll
-				for (int i = 0; i < RBY::NB; i++) {
-					const int p = RBY::seq(tid, i);
-					const bool live = p % CCX < ncol;
-#pragma unroll
-					for (int r = 0; r < MAXE; r++)
-						rb.v[i][r] = live ? a.work[gaddr(p, RBY::pos(tid, i, r))] : mk<T>((T)0, (T)0);
-				}
+				ct_first_from_regs<NC, MAXE, C::S, C::NT, -1, T>(sm, rb, tid);
+				ct_middle<NC, MAXE, C::S, C::NT, -1, T>(sm, tws, tid);
+				ct_pass<NC, PLX::radix(PLX::NPASS - 1), PLX::ns(PLX::NPASS - 1), PLX::twoff(PLX::NPASS - 1), C::S, C::NT, -1, T>(
+				    sm, tws, tid);
 			}
-			ct_first_from_regs<NCX, MAXE, C::S, C::NT, -1, T>(sm, rb, tid);
-			ct_middle<NCX, MAXE, C::S, C::NT, -1, T>(sm, tws, tid);
-			ct_pass<NCX, PLX::radix(PLX::NPASS - 1), PLX::ns(PLX::NPASS - 1), PLX::twoff(PLX::NPASS - 1), C::S, C::NT,
-			        -1, T>(sm, tws, tid);
 		}
-	}
-
-	if constexpr (MODE != YP_WEIGHT) if (!regio) {
-		if constexpr (C::CT && ((NC / RC) * CCC * RC) % C::NT == 0) {
+		static_assert(((NC / RC) * CCC * RC) % C::NT == 0 && (CCC * NC / 2) % C::NT == 0, "whole elements and pairs per thread");
+		if (!regio) {
 			// every load of the tile in flight before the first shared-memory store
 			constexpr int CH = CCC * RC;
 			constexpr int PER = (NC / RC) * CH / C::NT;
@@ -987,198 +780,72 @@ __device__ __forceinline__ void ypass_body(const YArgs<T>& a, const int grp, con
 					const int t = e / CH, rem = e % CH;
 					sm[(u * CCC + rem / RC) * C::LD + pad<T>(t * RC + rem % RC)] = v[u][i];
 				}
-		} else {
-#pragma unroll
-			for (int u = 0; u < U; u++) {
-				const cplx<T>* src = a.work + u * a.wstride + (long long)kx0 * R;
-				for (int e = tid; e < ntile * chunk; e += nt) {
-					const int t = e / chunk, rem = e - t * chunk;
-					const int c = rem / R, r = rem - c * R;
-					cplx<T> v = mk<T>((T)0, (T)0);
-					if (c < ncol) v = src[t * tileH + rem];
-					sm[(u * CC + c) * ld + pad<T>(t * R + r)] = v;
-				}
-			}
+			__syncthreads();
+			fft_ct<NC, MAXE, C::S, C::NSUB, C::NT, -1, T>(sm, tws, tid);
 		}
-		__syncthreads();
-		if constexpr (C::CT) fft_ct<NC, MAXE, C::S, C::NSUB, C::NT, -1, T>(sm, tws, tid);
-		else fft_batches<-1, MAXE, T>(sm, ld, S, a.sb, a.plan, a.tw, tid, nt);
-	}
 
-	const double dx = a.g.dx, dy = a.g.dy;
-	if constexpr (MODE == YP_STEP) {
-		// model constants in the transform precision, once per CTA
-		const StepK<T>& K = a.k;
-		const T dkxT = K.dkx, dkyT = K.dky;
 		// update of one (kx, ky) entry for all fields with its coefficients
 		// (A, B, couplings of k^2), pfc-relax.c:1215-1244
+		const StepK<T>& K = a.k;
 		auto apply = [&](int c, int kx, int ky, const cplx<T>(&Nv)[U], const T(&A)[U], const T(&Bn)[U],
 		                 const T(&cu)[npairs<T, U>()]) {
 			cplx<T> Mv[U];
 #pragma unroll
-			for (int u = 0; u < U; u++) Mv[u] = cscale(sm[(u * CC + c) * ld + pad<T>(ky)], K.invN);
+			for (int u = 0; u < U; u++) Mv[u] = cmul_rn(sm[(u * CCC + c) * C::LD + pad<T>(ky)], K.invN);
 			if constexpr (U > 1) {
 				int p = 0;
 #pragma unroll
 				for (int u = 0; u < U - 1; u++)
 #pragma unroll
 					for (int v = u + 1; v < U; v++, p++) {
-						Mv[u] = cadd(Mv[u], cscale(Nv[v], cu[p]));
-						Mv[v] = cadd(Mv[v], cscale(Nv[u], cu[p]));
+						Mv[u] = cfma_rn(Nv[v], cu[p], Mv[u]);
+						Mv[v] = cfma_rn(Nv[u], cu[p], Mv[v]);
 					}
 			}
 			const bool origin = (kx == 0 && ky == 0);
 #pragma unroll
 			for (int u = 0; u < U; u++) {
-				cplx<T> nn = cadd(cscale(Nv[u], A[u]), cscale(Mv[u], Bn[u]));
+				cplx<T> nn = cfma_rn(Mv[u], Bn[u], cmul_rn(Nv[u], A[u]));
 				if (origin) nn = mk<T>((T)0, (T)0);
 				// streaming (evict-first) accesses for the spectral state, read
 				// and written once per step, leave L2 to `work`, which the next
 				// pass reads back
-				__stcs(a.spec + u * a.sstride + (long long)kx * Ny + ky, nn);
-				sm[(u * CC + c) * ld + pad<T>(ky)] = nn;
+				__stcs(a.spec + u * a.sstride + (long long)kx * NC + ky, nn);
+				sm[(u * CCC + c) * C::LD + pad<T>(ky)] = nn;
 			}
 		};
-		auto update = [&](int c, int kx, int ky, const cplx<T>(&Nv)[U]) {
-			T A[U], Bn[U], cu[npairs<T, U>()];
-			entry_coef<T, U>(K, step_k2<T>(kx, ky, Ny, dkxT, dkyT, a.g), A, Bn, cu);
-			apply(c, kx, ky, Nv, A, Bn, cu);
-		};
-		if constexpr (C::CT && (CCC * NC / 2) % C::NT == 0) {
-			// entries ky and NC - ky have the same k^2 (signed wave numbers ky and
-			// -ky), so each thread takes such pairs and evaluates the coefficients
-			// once for both; ky = 0 is paired with the self-mirrored NC / 2 and
-			// evaluates them twice
-			constexpr int HALF = NC / 2;
-			constexpr int PH = CCC * HALF / C::NT;
-			cplx<T> Nv[PH][2][U];
+		// entries ky and NC - ky have the same k^2 (signed wave numbers ky and
+		// -ky), so each thread takes such pairs and evaluates the coefficients
+		// once for both; ky = 0 is paired with the self-mirrored NC / 2 and
+		// evaluates them twice
+		constexpr int HALF = NC / 2;
+		constexpr int PH = CCC * HALF / C::NT;
+		cplx<T> Nv[PH][2][U];
 #pragma unroll
-			for (int i = 0; i < PH; i++) {
-				const int h = tid + i * C::NT;
-				const int c = h / HALF, kb = h % HALF;
-				const int ky2 = kb ? NC - kb : HALF;
-				const long long col = (long long)(kx0 + c) * NC;
-#pragma unroll
-				for (int u = 0; u < U; u++) {
-					Nv[i][0][u] = (c < ncol) ? __ldcs(a.spec + u * a.sstride + col + kb) : mk<T>((T)0, (T)0);
-					Nv[i][1][u] = (c < ncol) ? __ldcs(a.spec + u * a.sstride + col + ky2) : mk<T>((T)0, (T)0);
-				}
-			}
-#pragma unroll
-			for (int i = 0; i < PH; i++) {
-				const int h = tid + i * C::NT;
-				const int c = h / HALF, kb = h % HALF;
-				const int kx = kx0 + c;
-				if (c < ncol) {
-					T A[U], Bn[U], cu[npairs<T, U>()];
-					entry_coef<T, U>(K, step_k2<T>(kx, kb, NC, dkxT, dkyT, a.g), A, Bn, cu);
-					apply(c, kx, kb, Nv[i][0], A, Bn, cu);
-					if (kb == 0) entry_coef<T, U>(K, step_k2<T>(kx, HALF, NC, dkxT, dkyT, a.g), A, Bn, cu);
-					apply(c, kx, kb ? NC - kb : HALF, Nv[i][1], A, Bn, cu);
-				}
-			}
-		} else if constexpr (C::CT && (CCC * NC) % C::NT == 0) {
-			// every thread owns PER entries: issue all spectral-state loads first
-			constexpr int PER = CCC * NC / C::NT;
-			cplx<T> Nv[PER][U];
-#pragma unroll
-			for (int i = 0; i < PER; i++) {
-				const int e = tid + i * C::NT;
-				const int c = e / NC, ky = e % NC;
-				const int kx = kx0 + c;
-#pragma unroll
-				for (int u = 0; u < U; u++)
-					Nv[i][u] = (c < ncol) ? a.spec[u * a.sstride + (long long)kx * NC + ky] : mk<T>((T)0, (T)0);
-			}
-#pragma unroll
-			for (int i = 0; i < PER; i++) {
-				const int e = tid + i * C::NT;
-				const int c = e / NC, ky = e % NC;
-				if (c < ncol) update(c, kx0 + c, ky, Nv[i]);
-			}
-		} else {
-			for (int e = tid; e < CC * Ny; e += nt) {
-				const int c = e / Ny, ky = e - c * Ny;
-				if (c >= ncol) continue;
-				const int kx = kx0 + c;
-				cplx<T> Nv[U];
-#pragma unroll
-				for (int u = 0; u < U; u++) Nv[u] = a.spec[u * a.sstride + (long long)kx * Ny + ky];
-				update(c, kx, ky, Nv);
-			}
-		}
-		if (kx0 == 0) ypass_mean_update<T, U>(a, tid, nt);
-	} else if constexpr (MODE == YP_INIT) {
-		const T invN = (T)(1.0 / ((double)Nx * (double)Ny));
-		for (int e = tid; e < CC * Ny; e += nt) {
-			const int c = e / Ny, ky = e - c * Ny;
-			if (c >= ncol) continue;
-			const int kx = kx0 + c;
-			const long long si = (long long)kx * Ny + ky;
+		for (int i = 0; i < PH; i++) {
+			const int h = tid + i * C::NT;
+			const int c = h / HALF, kb = h % HALF;
+			const int ky2 = kb ? NC - kb : HALF;
+			const long long col = (long long)(kx0 + c) * NC;
 #pragma unroll
 			for (int u = 0; u < U; u++) {
-				cplx<T> nn = cscale(sm[(u * CC + c) * ld + pad<T>(ky)], invN);
-				if (kx == 0 && ky == 0) nn = mk<T>((T)0, (T)0);
-				a.spec[u * a.sstride + si] = nn;
-				sm[(u * CC + c) * ld + pad<T>(ky)] = nn;
+				Nv[i][0][u] = (c < ncol) ? __ldcs(a.spec + u * a.sstride + col + kb) : mk<T>((T)0, (T)0);
+				Nv[i][1][u] = (c < ncol) ? __ldcs(a.spec + u * a.sstride + col + ky2) : mk<T>((T)0, (T)0);
 			}
 		}
-	} else {
-		// YP_WEIGHT (U == 1): w(k) * spec[src] -> sm, with the weight's
-		// parameters in a.wp (field index resolved on the host)
-		const double ag = -0.5 / a.m.sigma / a.m.sigma;
-		const cplx<T>* src = a.spec + a.wsrc * a.sstride;
-		for (int e = tid; e < CC * Ny; e += nt) {
-			const int c = e / Ny, ky = e - c * Ny;
-			const int kx = kx0 + c;
-			cplx<T> nn = mk<T>((T)0, (T)0);
-			if (c < ncol && !(kx == 0 && ky == 0)) {
-				const double k2 = k2_of(kx, ky, a.g, dx, dy);
-				double w = 1.0;
-				if (a.wkind == W_P) {
 #pragma unroll
-					for (int q = 0; q < MAXW; q++)
-						if (q < a.wp.W) {
-							const double d = a.wp.nu2[q] - k2;
-							w *= a.wp.omega[q] * d * d + a.wp.phi[q];
-						}
-				} else if (a.wkind == W_G) {
-					w = exp(ag * k2);
-				} else if (a.wkind == W_Q) {
-					const double d = a.wp.mu2 - k2;
-					w = d * d;
-				} else if (a.wkind == W_GS || a.wkind == W_DG) {
-					w = exp(-0.5 * k2 / (a.wp.gs * a.wp.gs));
-				}
-				const long long si = (long long)kx * Ny + ky;
-				if (a.wkind == W_OR) {
-					// orientation kernel K = exp(-(|k| - 1)^2 / (2 sk^2)) exp(i fold phi),
-					// fields.c:143-153; real and imaginary parts are even in k
-					// for even fold, so each part maps the field pair to a real field
-					const double kxv = kx * a.g.dkx;
-					const double kyv = (ky < Ny / 2 ? ky : ky - Ny) * a.g.dky;
-					const double q = sqrt(k2) - 1.0;
-					const double rad = exp(-0.5 * q * q / (a.wp.sk * a.wp.sk));
-					double sn, cs;
-					sincos(a.wp.fold * atan2(kyv, kxv), &sn, &cs);
-					const T kr = (T)(rad * cs), ki = (T)(rad * sn);
-					const cplx<T> s0 = a.spec[si], s1 = a.spec[a.sstride + si];
-					nn = a.wp.part == 0 ? csub(cscale(s0, kr), cscale(s1, ki)) : cadd(cscale(s0, ki), cscale(s1, kr));
-				} else if (a.wkind == W_DG) {
-					// i k_dir G(k) times the field (fields.c:260-271 on the smoothed spectrum)
-					const double kd = a.wp.dir == 0 ? kx * a.g.dkx : (ky < Ny / 2 ? ky : ky - Ny) * a.g.dky;
-					const cplx<T> v = src[si];
-					const T f = (T)(kd * w);
-					nn = mk<T>(-f * v.y, f * v.x);
-				} else {
-					nn = cscale(src[si], (T)w);
-				}
+		for (int i = 0; i < PH; i++) {
+			const int h = tid + i * C::NT;
+			const int c = h / HALF, kb = h % HALF;
+			const int kx = kx0 + c;
+			if (c < ncol) {
+				T A[U], Bn[U], cu[npairs<T, U>()];
+				entry_coef<T, U>(K, k2_step<T>(kx, kb, NC, K.dkx, K.dky), A, Bn, cu);
+				apply(c, kx, kb, Nv[i][0], A, Bn, cu);
+				if (kb == 0) entry_coef<T, U>(K, k2_step<T>(kx, HALF, NC, K.dkx, K.dky), A, Bn, cu);
+				apply(c, kx, kb ? NC - kb : HALF, Nv[i][1], A, Bn, cu);
 			}
-			sm[c * ld + pad<T>(ky)] = nn;
 		}
-	}
-
-	if constexpr (MODE == YP_STEP || MODE == YP_INIT) {
 		// kx = 0 and (even Nx) kx = Nx/2 columns: keep them exactly Hermitian
 		const bool has0 = (kx0 == 0);
 		const int kn = (Nx % 2 == 0) ? Nx / 2 : -1;
@@ -1187,41 +854,40 @@ __device__ __forceinline__ void ypass_body(const YArgs<T>& a, const int grp, con
 			__syncthreads();
 #pragma unroll
 			for (int u = 0; u < U; u++) {
-				if (has0) hermitian_column<T>(sm + (u * CC) * ld, a.spec + u * a.sstride, Ny, tid, nt);
+				if (has0) hermitian_column<T>(sm + (u * CCC) * C::LD, a.spec + u * a.sstride, NC, tid, C::NT);
 				if (hasn)
-					hermitian_column<T>(sm + (u * CC + (kn - kx0)) * ld, a.spec + u * a.sstride + (long long)kn * Ny, Ny,
-					                    tid, nt);
+					hermitian_column<T>(sm + (u * CCC + (kn - kx0)) * C::LD, a.spec + u * a.sstride + (long long)kn * NC, NC, tid,
+					                    C::NT);
 			}
 		}
-	}
-	__syncthreads();
-	if constexpr (REGIO) {
-		if (regio) {
-			ct_pass<NCX, PLX::radix(0), PLX::ns(0), PLX::twoff(0), C::S, C::NT, +1, T>(sm, tws, tid);
-			ct_middle<NCX, MAXE, C::S, C::NT, +1, T>(sm, tws, tid);
-			RBY rb;
-			ct_last_to_regs<NCX, MAXE, C::S, C::NT, +1, T>(sm, tws, rb, tid);
+		__syncthreads();
+		if constexpr (REGIO) {
+			if (regio) {
+				ct_pass<NC, PLX::radix(0), PLX::ns(0), PLX::twoff(0), C::S, C::NT, +1, T>(sm, tws, tid);
+				ct_middle<NC, MAXE, C::S, C::NT, +1, T>(sm, tws, tid);
+				RBY rb;
+				ct_last_to_regs<NC, MAXE, C::S, C::NT, +1, T>(sm, tws, rb, tid);
 #pragma unroll
-			for (int i = 0; i < RBY::NB; i++) {
-				const int p = RBY::seq(tid, i);
-				if (p % CCX < ncol) {
+				for (int i = 0; i < RBY::NB; i++) {
+					const int p = RBY::seq(tid, i);
+					if (p % CCC < ncol) {
 #pragma unroll
-					for (int r = 0; r < MAXE; r++) a.work[gaddr(p, RBY::pos(tid, i, r))] = rb.v[i][r];
+						for (int r = 0; r < MAXE; r++) a.work[gaddr(p, RBY::pos(tid, i, r))] = rb.v[i][r];
+					}
 				}
+				return;
 			}
-			return;
 		}
-	}
-	if constexpr (C::CT) fft_ct<NC, MAXE, C::S, C::NSUB, C::NT, +1, T>(sm, tws, tid);
-	else fft_batches<+1, MAXE, T>(sm, ld, S, a.sb, a.plan, a.tw, tid, nt);
-
+		fft_ct<NC, MAXE, C::S, C::NSUB, C::NT, +1, T>(sm, tws, tid);
+		constexpr int CH = CCC * RC;
 #pragma unroll
-	for (int u = 0; u < U; u++) {
-		cplx<T>* dst = a.work + u * a.wstride + (long long)kx0 * R;
-		for (int e = tid; e < ntile * chunk; e += nt) {
-			const int t = e / chunk, rem = e - t * chunk;
-			const int c = rem / R, r = rem - c * R;
-			if (c < ncol) dst[t * tileH + rem] = sm[(u * CC + c) * ld + pad<T>(t * R + r)];
+		for (int u = 0; u < U; u++) {
+			cplx<T>* dst = a.work + u * a.wstride + (long long)kx0 * RC;
+			for (int e = tid; e < NC * CCC; e += C::NT) {
+				const int t = e / CH, rem = e % CH;
+				const int c = rem / RC, r = rem % RC;
+				if (c < ncol) dst[t * tileH + rem] = sm[(u * CCC + c) * C::LD + pad<T>(t * RC + r)];
+			}
 		}
 	}
 }
@@ -1281,7 +947,7 @@ __global__ void __launch_bounds__(256) kspace_energy_kernel(const cplx<T>* __res
 
 // -------------------------------------------------------------- launchers --
 
-template <typename T, int U, int MODE, int NC, int CCC, int RC, bool FUSEDK = true>
+template <typename T, int U, int NC, int CCC, int RC, bool FUSEDK = true>
 __global__ void __launch_bounds__(YCfg<T, U, NC, CCC, RC, FUSEDK>::NT, YCfg<T, U, NC, CCC, RC, FUSEDK>::MINB)
     ypass_kernel(const YArgs<T> a, int ngroups) {
 	asm volatile("griddepcontrol.wait;" ::: "memory"); // as in xpass_kernel
@@ -1289,62 +955,29 @@ __global__ void __launch_bounds__(YCfg<T, U, NC, CCC, RC, FUSEDK>::NT, YCfg<T, U
 	// column groups blockIdx.x, + gridDim.x, ... (as the x-pass's tiles)
 	for (int g = blockIdx.x; g < ngroups; g += gridDim.x) {
 		if (g != (int)blockIdx.x) __syncthreads();
-		ypass_body<T, U, MODE, NC, CCC, RC, FUSEDK>(a, g, g == (int)blockIdx.x, (g - (int)blockIdx.x) / (int)gridDim.x);
+		ypass_body<T, U, NC, CCC, RC, FUSEDK>(a, g, g == (int)blockIdx.x, (g - (int)blockIdx.x) / (int)gridDim.x);
 	}
 }
 
 // ------------------------------------------------------------------ batch --
-// Many independent relaxations of runtime sizes in one launch: block b runs
-// tile (x-pass) or column group (y-pass) blk_local[b] of problem blk_prob[b],
-// whose arguments sit in global memory. Launched with the largest thread count
-// and shared memory any problem needs; the runtime-plan bodies use whatever
-// threads they get.
-template <typename T>
-__global__ void __launch_bounds__(MAXNT, 1)
-    xpass_batch_kernel(const XArgs<T>* __restrict__ probs, const int* __restrict__ blk_prob,
-                       const int* __restrict__ blk_local) {
-	const XArgs<T>& a = probs[blk_prob[blockIdx.x]];
-	const int local = blk_local[blockIdx.x];
-	switch (a.m.U) {
-	case 1: xpass_body<T, 1, XP_STEP, 0, 0>(a, local); break;
-	case 2: xpass_body<T, 2, XP_STEP, 0, 0>(a, local); break;
-	case 3: xpass_body<T, 3, XP_STEP, 0, 0>(a, local); break;
-	case 4: xpass_body<T, 4, XP_STEP, 0, 0>(a, local); break;
-	}
-}
-
-template <typename T>
-__global__ void __launch_bounds__(MAXNT, 1)
-    ypass_batch_kernel(const YArgs<T>* __restrict__ probs, const int* __restrict__ blk_prob,
-                       const int* __restrict__ blk_local) {
-	const YArgs<T>& a = probs[blk_prob[blockIdx.x]];
-	const int local = blk_local[blockIdx.x];
-	switch (a.m.U) {
-	case 1: ypass_body<T, 1, YP_STEP, 0, 0, 0>(a, local); break;
-	case 2: ypass_body<T, 2, YP_STEP, 0, 0, 0>(a, local); break;
-	case 3: ypass_body<T, 3, YP_STEP, 0, 0, 0>(a, local); break;
-	case 4: ypass_body<T, 4, YP_STEP, 0, 0, 0>(a, local); break;
-	}
-}
-
-// Raises the dynamic shared-memory limit of a kernel once per device.
 // Batched STEP passes of the kernels specialised on a length: every block of
 // the launch belongs to a problem of that length and field count (one launch
 // per such class of a batch), so the body is the single-problem one.
-template <typename T, int U, int MODE, int NC, int RC>
+template <typename T, int U, int NC, int RC>
 __global__ void __launch_bounds__(XCfg<T, U, NC, RC>::NT, XCfg<T, U, NC, RC>::MINB)
     xpass_ct_batch_kernel(const XArgs<T>* __restrict__ probs, const int* __restrict__ blk_prob,
                           const int* __restrict__ blk_local) {
-	xpass_body<T, U, MODE, NC, RC>(probs[blk_prob[blockIdx.x]], blk_local[blockIdx.x]);
+	xpass_body<T, U, NC, RC>(probs[blk_prob[blockIdx.x]], blk_local[blockIdx.x]);
 }
 
-template <typename T, int U, int MODE, int NC, int CCC, int RC, bool FUSEDK>
+template <typename T, int U, int NC, int CCC, int RC, bool FUSEDK>
 __global__ void __launch_bounds__(YCfg<T, U, NC, CCC, RC, FUSEDK>::NT, YCfg<T, U, NC, CCC, RC, FUSEDK>::MINB)
     ypass_ct_batch_kernel(const YArgs<T>* __restrict__ probs, const int* __restrict__ blk_prob,
                           const int* __restrict__ blk_local) {
-	ypass_body<T, U, MODE, NC, CCC, RC, FUSEDK>(probs[blk_prob[blockIdx.x]], blk_local[blockIdx.x]);
+	ypass_body<T, U, NC, CCC, RC, FUSEDK>(probs[blk_prob[blockIdx.x]], blk_local[blockIdx.x]);
 }
 
+// Raises the dynamic shared-memory limit of a kernel once per device.
 template <typename K> static void smem_attr(K k, unsigned long long& mask) {
 	int dev = 0;
 	cudaGetDevice(&dev);
@@ -1359,31 +992,11 @@ template <typename K> static void smem_attr(K k, unsigned long long& mask) {
 	}
 }
 
-// Grid of the compile-time specialised FP64 kernels: as many CTAs as fit on the
-// device at once (cached per kernel), each looping over several tiles or column
-// groups, so the 64 KB twiddle table loads once per CTA (1.8 % more steps/s at
-// 4096^2; the FP32 kernels measured 4.7 % slower this way and keep one CTA per
-// tile). PFCG_PERSISTENT=0 launches one CTA per tile in FP64 too.
-template <typename K> static int resident_grid(K k, const LaunchCfg& c, int& resident) {
-	if (resident == 0) {
-		const char* e = getenv("PFCG_PERSISTENT");
-		int dev = 0, sms = 0, per = 0;
-		cudaGetDevice(&dev);
-		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, c.block, c.smem);
-		resident = (e && e[0] == '0') || per < 1 || sms < 1 ? -1 : per * sms;
-	}
-	return resident > 0 && resident < c.grid ? resident : c.grid;
-}
-
 // Launch of the x- and y-pass kernels as programmatic dependent launches: the
 // next pass's CTAs may be scheduled while the last wave of the previous one
 // drains, and each kernel waits for the previous kernel's completion and
-// memory (griddepcontrol.wait, its first statement) before touching anything
-// that kernel writes. PFCG_PDL=0 launches them plainly. Persistent grids (one
-// CTA per resident slot, the FP64 specialised kernels) launch plainly too:
-// with every slot taken there is no drain to overlap, and dependent launches
-// measured 2 % slower there (1.041 against 1.019 ms per 4096^2 U=2 FP64 step).
+// memory (griddepcontrol.wait) before touching anything that kernel writes.
+// PFCG_PDL=0 launches them plainly.
 static bool pdl_on() {
 	static const int on = [] {
 		const char* e = std::getenv("PFCG_PDL");
@@ -1394,7 +1007,7 @@ static bool pdl_on() {
 
 template <typename K, typename A>
 static cudaError_t pdl_launch(K k, int grid, int block, int smem, cudaStream_t s, const A& a, int n) {
-	if (!pdl_on() || grid < n) {
+	if (!pdl_on()) {
 		k<<<grid, block, smem, s>>>(a, n);
 		return cudaGetLastError();
 	}
@@ -1411,27 +1024,23 @@ static cudaError_t pdl_launch(K k, int grid, int block, int smem, cudaStream_t s
 	return cudaLaunchKernelEx(&cfg, k, a, n);
 }
 
-template <typename T, int U, int MODE, int NC, int RC>
+template <typename T, int U, int NC, int RC>
 static cudaError_t xlaunch(const XArgs<T>& a, const LaunchCfg& c, cudaStream_t s) {
-	auto k = xpass_kernel<T, U, MODE, NC, RC>;
+	auto k = xpass_kernel<T, U, NC, RC>;
 	static unsigned long long mask = 0;
-	static int resident = 0;
 	smem_attr(k, mask);
-	const int grid = NC > 0 && std::is_same<T, double>::value ? resident_grid(k, c, resident) : c.grid;
-	return pdl_launch(k, grid, c.block, c.smem, s, a, c.grid);
+	return pdl_launch(k, c.grid, c.block, c.smem, s, a, c.grid);
 }
 
 // Compile-time specialisations of the STEP kernels: (length, rows per tile,
 // columns per y-pass CTA) for the sizes the workloads use; other sizes and
-// modes run the runtime-plan kernels.
-template <typename T, int U, int MODE, int NC, int CCC, int RC, bool FUSEDK = true>
+// modes run the kernels of run-time lengths (kernels_rt.cuh).
+template <typename T, int U, int NC, int CCC, int RC, bool FUSEDK = true>
 static cudaError_t ylaunch(const YArgs<T>& a, const LaunchCfg& c, cudaStream_t s) {
-	auto k = ypass_kernel<T, U, MODE, NC, CCC, RC, FUSEDK>;
+	auto k = ypass_kernel<T, U, NC, CCC, RC, FUSEDK>;
 	static unsigned long long mask = 0;
-	static int resident = 0;
 	smem_attr(k, mask);
-	const int grid = NC > 0 && std::is_same<T, double>::value ? resident_grid(k, c, resident) : c.grid;
-	return pdl_launch(k, grid, c.block, c.smem, s, a, c.grid);
+	return pdl_launch(k, c.grid, c.block, c.smem, s, a, c.grid);
 }
 
 template <typename T> struct Spec;
@@ -1452,15 +1061,6 @@ template <> struct Spec<float> {
 	static constexpr int xr(int U, int N) { return U == 1 ? x1(N) : U == 2 ? x1(N) / 2 : 0; }
 	static constexpr int ycc(int U, int N) { return U == 1 ? y1(N) : U == 2 ? y1(N) / 2 : 0; }
 };
-template <> struct Spec<double> {
-	static constexpr int xr(int U, int N) {
-		return N == 4096 ? (U == 1 ? 2 : U == 2 ? 1 : 0) : N == 2048 ? (U == 1 ? 4 : U == 2 ? 2 : 0) : 0;
-	}
-	static constexpr int ycc(int U, int N) {
-		return N == 4096 ? (U == 1 ? 1 : U == 2 ? 1 : 0) : N == 2048 ? (U == 1 ? 2 : U == 2 ? 1 : 0) : 0;
-	}
-};
-
 template <typename T, int U> static bool x_is_spec(const XArgs<T>& a) {
 	return Spec<T>::xr(U, a.g.Nx) > 0 && a.g.R == Spec<T>::xr(U, a.g.Nx);
 }
@@ -1472,19 +1072,19 @@ template <typename T, int U> static bool y_is_spec(const YArgs<T>& a) {
 // 2048 are instantiated in kernels_f32_<N>.cu, one file each, so that they
 // compile in parallel.
 template <typename T, int U, int N> cudaError_t ct_xstep(const XArgs<T>& a, const LaunchCfg& c, cudaStream_t s) {
-	return xlaunch<T, U, XP_STEP, N, Spec<T>::xr(U, N)>(a, c, s);
+	return xlaunch<T, U, N, Spec<T>::xr(U, N)>(a, c, s);
 }
 template <typename T, int U, int N> cudaError_t ct_ystep(const YArgs<T>& a, const LaunchCfg& c, cudaStream_t s) {
 	// c.spec: 1 = specialised (fused where possible), 2 = specialised, never fused
-	if (c.spec == 2) return ylaunch<T, U, YP_STEP, N, Spec<T>::ycc(U, N), Spec<T>::xr(U, N), false>(a, c, s);
-	return ylaunch<T, U, YP_STEP, N, Spec<T>::ycc(U, N), Spec<T>::xr(U, N)>(a, c, s);
+	if (c.spec == 2) return ylaunch<T, U, N, Spec<T>::ycc(U, N), Spec<T>::xr(U, N), false>(a, c, s);
+	return ylaunch<T, U, N, Spec<T>::ycc(U, N), Spec<T>::xr(U, N)>(a, c, s);
 }
 
 // Batched STEP passes over nblk blocks of problems of length N (nblk = 0 only
 // sets the kernel's shared-memory limit, which must not happen under capture).
 template <typename T, int U, int N>
 cudaError_t ct_xbatch(const XArgs<T>* probs, const int* bp, const int* bl, int nblk, const LaunchCfg& c, cudaStream_t s) {
-	auto k = xpass_ct_batch_kernel<T, U, XP_STEP, N, Spec<T>::xr(U, N)>;
+	auto k = xpass_ct_batch_kernel<T, U, N, Spec<T>::xr(U, N)>;
 	static unsigned long long mask = 0;
 	smem_attr(k, mask);
 	if (nblk > 0) k<<<nblk, c.block, c.smem, s>>>(probs, bp, bl);
@@ -1495,11 +1095,11 @@ cudaError_t ct_ybatch(const YArgs<T>* probs, const int* bp, const int* bl, int n
 	constexpr int CC = Spec<T>::ycc(U, N), R = Spec<T>::xr(U, N);
 	static unsigned long long m1 = 0, m2 = 0;
 	if (c.spec == 2) {
-		auto k = ypass_ct_batch_kernel<T, U, YP_STEP, N, CC, R, false>;
+		auto k = ypass_ct_batch_kernel<T, U, N, CC, R, false>;
 		smem_attr(k, m2);
 		if (nblk > 0) k<<<nblk, c.block, c.smem, s>>>(probs, bp, bl);
 	} else {
-		auto k = ypass_ct_batch_kernel<T, U, YP_STEP, N, CC, R, true>;
+		auto k = ypass_ct_batch_kernel<T, U, N, CC, R, true>;
 		smem_attr(k, m1);
 		if (nblk > 0) k<<<nblk, c.block, c.smem, s>>>(probs, bp, bl);
 	}
@@ -1553,16 +1153,12 @@ template <typename T, int U> static cudaError_t ct_xdispatch(const XArgs<T>& a, 
 	switch (a.g.Nx) {
 	case 4096: return ct_xstep<T, U, 4096>(a, c, s);
 	case 2048: return ct_xstep<T, U, 2048>(a, c, s);
-	}
-	if constexpr (std::is_same<T, float>::value) {
-		switch (a.g.Nx) {
-		case 1536: return ct_xstep<T, U, 1536>(a, c, s);
-		case 1024: return ct_xstep<T, U, 1024>(a, c, s);
-		case 768: return ct_xstep<T, U, 768>(a, c, s);
-		case 512: return ct_xstep<T, U, 512>(a, c, s);
-		case 384: return ct_xstep<T, U, 384>(a, c, s);
-		case 256: return ct_xstep<T, U, 256>(a, c, s);
-		}
+	case 1536: return ct_xstep<T, U, 1536>(a, c, s);
+	case 1024: return ct_xstep<T, U, 1024>(a, c, s);
+	case 768: return ct_xstep<T, U, 768>(a, c, s);
+	case 512: return ct_xstep<T, U, 512>(a, c, s);
+	case 384: return ct_xstep<T, U, 384>(a, c, s);
+	case 256: return ct_xstep<T, U, 256>(a, c, s);
 	}
 	return cudaErrorInvalidValue;
 }
@@ -1570,75 +1166,22 @@ template <typename T, int U> static cudaError_t ct_ydispatch(const YArgs<T>& a, 
 	switch (a.g.Ny) {
 	case 4096: return ct_ystep<T, U, 4096>(a, c, s);
 	case 2048: return ct_ystep<T, U, 2048>(a, c, s);
-	}
-	if constexpr (std::is_same<T, float>::value) {
-		switch (a.g.Ny) {
-		case 1536: return ct_ystep<T, U, 1536>(a, c, s);
-		case 1024: return ct_ystep<T, U, 1024>(a, c, s);
-		case 768: return ct_ystep<T, U, 768>(a, c, s);
-		case 512: return ct_ystep<T, U, 512>(a, c, s);
-		case 384: return ct_ystep<T, U, 384>(a, c, s);
-		case 256: return ct_ystep<T, U, 256>(a, c, s);
-		}
+	case 1536: return ct_ystep<T, U, 1536>(a, c, s);
+	case 1024: return ct_ystep<T, U, 1024>(a, c, s);
+	case 768: return ct_ystep<T, U, 768>(a, c, s);
+	case 512: return ct_ystep<T, U, 512>(a, c, s);
+	case 384: return ct_ystep<T, U, 384>(a, c, s);
+	case 256: return ct_ystep<T, U, 256>(a, c, s);
 	}
 	return cudaErrorInvalidValue;
-}
-
-// One launch of the batched STEP pass (pass 0 = x, 1 = y) of the class of
-// problems with U fields and length N; cudaErrorInvalidValue where the size
-// has no specialised kernel.
-template <typename T, int U>
-static cudaError_t ct_batch_u(int pass, int N, const void* probs, const int* bp, const int* bl, int nblk,
-                              const LaunchCfg& c, cudaStream_t s) {
-#define PFCG_CT_CASE(NN)                                                                                              \
-	case NN:                                                                                                           \
-		return pass == 0 ? ct_xbatch<T, U, NN>((const XArgs<T>*)probs, bp, bl, nblk, c, s)                            \
-		                 : ct_ybatch<T, U, NN>((const YArgs<T>*)probs, bp, bl, nblk, c, s);
-	switch (N) {
-		PFCG_CT_CASE(4096)
-		PFCG_CT_CASE(2048)
-	}
-	if constexpr (std::is_same<T, float>::value) {
-		switch (N) {
-			PFCG_CT_CASE(1536)
-			PFCG_CT_CASE(1024)
-			PFCG_CT_CASE(768)
-			PFCG_CT_CASE(512)
-			PFCG_CT_CASE(384)
-			PFCG_CT_CASE(256)
-		}
-	}
-#undef PFCG_CT_CASE
-	return cudaErrorInvalidValue;
-}
-template <typename T>
-cudaError_t launch_ct_batch(int pass, int U, int N, const void* probs, const int* bp, const int* bl, int nblk,
-                            const LaunchCfg& c, cudaStream_t s) {
-	if (U == 1) return ct_batch_u<T, 1>(pass, N, probs, bp, bl, nblk, c, s);
-	if (U == 2) return ct_batch_u<T, 2>(pass, N, probs, bp, bl, nblk, c, s);
-	return cudaErrorInvalidValue;
-}
-template <typename T>
-cudaError_t launch_generic_batch(int pass, const void* probs, const int* bp, const int* bl, int nblk, int threads,
-                                 int smem, cudaStream_t s) {
-	prepare_batch_kernels<T>();
-	if (nblk <= 0) return cudaGetLastError();
-	if (pass == 0) xpass_batch_kernel<T><<<nblk, threads, smem, s>>>((const XArgs<T>*)probs, bp, bl);
-	else ypass_batch_kernel<T><<<nblk, threads, smem, s>>>((const YArgs<T>*)probs, bp, bl);
-	return cudaGetLastError();
 }
 
 template <typename T, int U> static cudaError_t xlaunch_mode(int mode, const XArgs<T>& a, const LaunchCfg& c, cudaStream_t s) {
-	switch (mode) {
-	case XP_STEP:
-		if constexpr (U <= 2)
-			if (c.spec && x_is_spec<T, U>(a)) return ct_xdispatch<T, U>(a, c, s);
-		return xlaunch<T, U, XP_STEP, 0, 0>(a, c, s);
-	case XP_EVAL: return xlaunch<T, U, XP_EVAL, 0, 0>(a, c, s);
-	case XP_C2R: return xlaunch<T, U, XP_C2R, 0, 0>(a, c, s);
-	case XP_R2C: return xlaunch<T, U, XP_R2C, 0, 0>(a, c, s);
-	}
-	return cudaErrorInvalidValue;
+	if constexpr (U <= 2 && sizeof(T) == 4)
+		if (mode == XP_STEP && c.spec && x_is_spec<T, U>(a)) return ct_xdispatch<T, U>(a, c, s);
+	if constexpr (U >= 3 && sizeof(T) == 4)
+		if (a.wtw && (mode == XP_STEP || mode == XP_R2C)) return wide_launch_x<U>(mode, a, c, s);
+	return rt_launch_x<T, U>(mode, a, c, s);
 }
 
 template <typename T> cudaError_t launch_xpass(int mode, const XArgs<T>& a, const LaunchCfg& c, cudaStream_t s) {
@@ -1651,37 +1194,23 @@ template <typename T> cudaError_t launch_xpass(int mode, const XArgs<T>& a, cons
 	return cudaErrorInvalidValue;
 }
 
-
-template <typename T, int U> static cudaError_t ystep(const YArgs<T>& a, const LaunchCfg& c, cudaStream_t s) {
-	if (c.spec && y_is_spec<T, U>(a)) return ct_ydispatch<T, U>(a, c, s);
-	return ylaunch<T, U, YP_STEP, 0, 0, 0>(a, c, s);
+template <typename T, int U> static cudaError_t ylaunch_mode(int mode, const YArgs<T>& a, const LaunchCfg& c, cudaStream_t s) {
+	if constexpr (U <= 2 && sizeof(T) == 4)
+		if (mode == YP_STEP && c.spec && y_is_spec<T, U>(a)) return ct_ydispatch<T, U>(a, c, s);
+	if constexpr (U >= 3 && sizeof(T) == 4)
+		if (a.wtw && mode != YP_WEIGHT) return wide_launch_y<U>(mode, a, c, s);
+	return rt_launch_y<T, U>(mode, a, c, s);
 }
 
 template <typename T> cudaError_t launch_ypass(int mode, const YArgs<T>& a, const LaunchCfg& c, cudaStream_t s) {
-	if (mode == YP_WEIGHT) return ylaunch<T, 1, YP_WEIGHT, 0, 0, 0>(a, c, s);
-	if (mode == YP_STEP) {
-		switch (a.m.U) {
-		case 1: return ystep<T, 1>(a, c, s);
-		case 2: return ystep<T, 2>(a, c, s);
-		case 3: return ylaunch<T, 3, YP_STEP, 0, 0, 0>(a, c, s);
-		case 4: return ylaunch<T, 4, YP_STEP, 0, 0, 0>(a, c, s);
-		}
-	}
-	if (mode == YP_INIT) {
-		switch (a.m.U) {
-		case 1: return ylaunch<T, 1, YP_INIT, 0, 0, 0>(a, c, s);
-		case 2: return ylaunch<T, 2, YP_INIT, 0, 0, 0>(a, c, s);
-		case 3: return ylaunch<T, 3, YP_INIT, 0, 0, 0>(a, c, s);
-		case 4: return ylaunch<T, 4, YP_INIT, 0, 0, 0>(a, c, s);
-		}
+	// a weighted spectrum is one field, whatever the system's field count
+	switch (mode == YP_WEIGHT ? 1 : a.m.U) {
+	case 1: return ylaunch_mode<T, 1>(mode, a, c, s);
+	case 2: return ylaunch_mode<T, 2>(mode, a, c, s);
+	case 3: return ylaunch_mode<T, 3>(mode, a, c, s);
+	case 4: return ylaunch_mode<T, 4>(mode, a, c, s);
 	}
 	return cudaErrorInvalidValue;
-}
-
-template <typename T> void prepare_batch_kernels() {
-	static unsigned long long mx = 0, my = 0;
-	smem_attr(xpass_batch_kernel<T>, mx);
-	smem_attr(ypass_batch_kernel<T>, my);
 }
 
 template <typename T>

@@ -1,0 +1,8 @@
+// Batched STEP kernels of run-time lengths, F64 (kernels_rt_batch.cuh).
+#include "kernels_rt_batch.cuh"
+
+namespace pfcg {
+
+template cudaError_t launch_generic_batch<double>(int, const void*, const int*, const int*, int, int, int, cudaStream_t);
+
+} // namespace pfcg
