@@ -290,7 +290,7 @@ void pfcg_batch_destroy(pfcg_batch* b);
 #define PFCG_FNO_PARAMS 1052962
 typedef struct pfcg_fno pfcg_fno;
 size_t pfcg_fno_param_count(void);
-/* max_batch tiles per launch sequence; memory grows as max_batch * T^2 * 1.9 KB. */
+/* max_batch tiles per launch sequence; memory grows as max_batch * T^2 * 0.95 KB. */
 int pfcg_fno_create(int tile, int max_batch, pfcg_fno** out);
 int pfcg_fno_set_params(pfcg_fno* f, const float* host_params); /* also resets Adam */
 int pfcg_fno_get_params(pfcg_fno* f, float* host_params);

@@ -7,11 +7,13 @@
 // K_l v = irfft2 of R_l (complex C x C per retained mode) times rfft2(v) on the
 // retained modes kx in [0, MX), ky in {0..MY/2-1} u {T-MY/2..T-1}; all other
 // modes are dropped. The truncated transforms are direct sums against
-// twiddle matrices (dft_x, idft_x, dft_y_fwd, dft_y_inv); the adjoint of each
-// linear step is another of these kernels, which is how the backward pass is
-// built:
-//   idft_x^T = dft_x with the inverse's per-mode weights, dft_y_fwd^T =
-//   dft_y_inv, mix^T = mix with conj(R) transposed, dft_x^T = idft_x.
+// twiddle matrices; the adjoint of each linear step is the transform of the
+// other direction, which is how the backward pass is built. A layer is two kinds
+// of kernel: one pass over the activations (layer_fwd, or layer_grad and
+// layer_bwd on the way back), which does everything per row (channel product,
+// inverse x transform of the mixed modes, GELU, forward x transform of the result,
+// at the ends the lift and the projection), and the small kernels between two
+// passes, which work on the rows' eight retained modes (dft_y_fwd, mix, dft_y_inv).
 // Activations and sums are FP32; the kernels read a BF16 copy of the FP32
 // master weights, which Adam updates.
 #include <cuda_bf16.h>
@@ -54,9 +56,41 @@ constexpr int MAXT = 512; // largest tile (twiddle table in shared memory)
 
 __device__ __forceinline__ float wld(const __nv_bfloat16* w, size_t i) { return __bfloat162float(w[i]); }
 
-__device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
+// The normal distribution's lower tail at -u and the density's exponential, u = |z|
+// (clamped where both are zero in FP32): Phi(-u) = exp(-u^2 / 2) R(u), and R(u) =
+// t Q(t) with t = 1 / (1 + 0.21 u) and Q of degree 8, fitted here by iteratively
+// reweighted least squares to 1.4e-8 relative over u < 13.5. GELU from it is within
+// 2.4e-7 of FP64 on [-9, 9] (rms 4.7e-8), from erff 4.5e-7 (6.3e-8), in 16
+// instructions and two special-function ones instead of about 22; the derivative
+// shares both parts. GELU was half of a layer's instructions.
+struct Tail {
+	float u, phi, e;
+	__device__ __forceinline__ explicit Tail(float z) {
+		float t;
+		u = fminf(fabsf(z), 20.f);
+		asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.21f, u, 1.f)));
+		asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-0.72134752f * u * u));
+		float q = -0.07203336f;
+		q = fmaf(q, t, 0.28545034f);
+		q = fmaf(q, t, -0.33418325f);
+		q = fmaf(q, t, 0.35402617f);
+		q = fmaf(q, t, -0.097240396f);
+		q = fmaf(q, t, 0.1263528f);
+		q = fmaf(q, t, 0.068790667f);
+		q = fmaf(q, t, 0.085129313f);
+		q = fmaf(q, t, 0.083707705f);
+		phi = q * t * e;
+	}
+};
+__device__ __forceinline__ float gelu(float z) {
+	const Tail p(z);
+	float r; // max(z, 0), NaN kept
+	asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(z));
+	return fmaf(-p.u, p.phi, r);
+}
 __device__ __forceinline__ float gelu_d(float z) {
-	return 0.5f * (1.f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * __expf(-0.5f * z * z);
+	const Tail p(z);
+	return fmaf(z * 0.39894228040143268f, p.e, z < 0.f ? p.phi : 1.f - p.phi);
 }
 
 // wave number of retained row k along y
@@ -78,35 +112,17 @@ __global__ void twiddle_kernel(float2* tw, int T) {
 	}
 }
 
-// v0[b][c][p] = P[c][0] x[b][0][p] + P[c][1] x[b][1][p] + p[c]
-__global__ void lift_fwd(const float* __restrict__ x, const __nv_bfloat16* __restrict__ w, float* __restrict__ v, int B,
-                         int npix) {
-	__shared__ float Ps[3 * C];
-	for (int i = threadIdx.x; i < 3 * C; i += blockDim.x) Ps[i] = wld(w, OFF_P + i);
-	__syncthreads();
-	const long long n = (long long)B * npix;
-	for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-		const long long b = t / npix;
-		const int p = (int)(t - b * npix);
-		const float x0 = x[(b * 2) * npix + p], x1 = x[(b * 2 + 1) * npix + p];
-		float* vb = v + b * C * npix + p;
-#pragma unroll 8
-		for (int c = 0; c < C; c++) vb[(long long)c * npix] = Ps[2 * c] * x0 + Ps[2 * c + 1] * x1 + Ps[2 * C + c];
-	}
-}
-
-// ------------------------------------------- tensor-core channel products --
-// The per-pixel channel contractions (z = W v, dv = W^T dz, dW = dz v^T) are
-// GEMMs with a 32 x 32 weight or result and the pixels as the long dimension;
-// they run on the tensor cores as mma.sync m16n8k16 with BF16 operands and
-// FP32 accumulation. An FP32 operand is split into a BF16 high part and a
-// BF16 remainder (x = hi + lo to about 2^-16 relative) and the products that
-// matter are summed: with the BF16 weights, which are exact, W hi + W lo; with
-// two FP32 operands, hi hi + hi lo + lo hi. Fragment layouts are those of the
-// PTX ISA for m16n8k16: g = lane / 4, t = lane % 4; A (16 x 16, row major)
-// holds rows g, g + 8 and columns 2t, 2t + 1, 2t + 8, 2t + 9; B (16 x 8) holds
-// rows 2t, 2t + 1, 2t + 8, 2t + 9 of column g; the accumulator holds rows g,
-// g + 8 and columns 2t, 2t + 1.
+// --------------------------------------------------- tensor-core products --
+// The per-pixel channel contractions (z = W v, dv = W^T dz, dW = dz v^T) and the
+// x transforms (whose other operand is a fixed matrix of twiddles) are GEMMs on
+// the tensor cores, mma.sync m16n8k16 with BF16 operands and FP32 accumulation.
+// An FP32 operand is split into a BF16 high part and a BF16 remainder (x = hi +
+// lo to about 2^-16 relative) and the products that matter are summed: with the
+// BF16 weights, which are exact, W hi + W lo; with two FP32 operands, hi hi +
+// hi lo + lo hi. Fragment layouts are those of the PTX ISA for m16n8k16: g =
+// lane / 4, t = lane % 4; A (16 x 16, row major) holds rows g, g + 8 and columns
+// 2t, 2t + 1, 2t + 8, 2t + 9; B (16 x 8) holds rows 2t, 2t + 1, 2t + 8, 2t + 9
+// of column g; the accumulator holds rows g, g + 8 and columns 2t, 2t + 1.
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
 	asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
@@ -131,32 +147,35 @@ __device__ __forceinline__ uint32_t pack_bf16(const __nv_bfloat16* w, size_t i0,
 	return (uint32_t)a | ((uint32_t)b << 16);
 }
 
-// The truncated transforms along x are GEMMs too, with the rows as the long
-// dimension and a fixed matrix of twiddles as the other operand, whose
-// BF16-split mma fragments are tabulated once per tile size (dft_frag_kernel):
-//   dft_x:  D[row][2m + q] = sum_x in[row][x] E[x][2m + q], E = cos / -sin(2 pi m x / T)
-//   idft_x: D[row][x] = sum_{m, q} in'[row][2m + q] F[2m + q][x], F = cos / -sin(2 pi m x / T),
-//           in' = scale[m] (Re, Im) of the row's modes
-// Fragment entry (k-step or n-tile, lane) holds the B registers of the high
-// parts and of the remainders.
+// A warp works on 32 pixels of a row at a time, as four n-tiles of eight columns
+// (or, where they are summed over, two k-steps of sixteen). Column c of n-tile j is
+// pixel 4 (c / 2) + 16 (c % 2) + j: lane g then loads its column of all four tiles
+// as one float4, the eight g of a channel 128 contiguous bytes, and of a result
+// lane t holds pixels 4t .. 4t + 3 and 16 + 4t .. 16 + 4t + 3, two float4. The same
+// order makes an accumulator the A operand of the next product (k-step ks holds
+// n-tiles 2 ks and 2 ks + 1), so a result's x transform needs no exchange.
+constexpr int PX = 32;
+__host__ __device__ __forceinline__ int px_of(int c, int j) { return 4 * (c >> 1) + 16 * (c & 1) + j; }
 
-// fdx: [T/16 k-steps][2 n-tiles][32 lanes], fix: [T/8 n-tiles][32 lanes]
-__global__ void dft_frag_kernel(const float2* __restrict__ tw, int T, uint4* __restrict__ fdx, uint4* __restrict__ fix) {
-	const int nx = T / 16 * 2 * 32, ni = T / 8 * 32;
-	for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nx + ni; e += gridDim.x * blockDim.x) {
+// The twiddle matrices of the x transforms as B fragments, high parts and remainders:
+//   forward: E[x][2m + q] = cos / -sin(2 pi m x / T), fe: [T/32][2 k-steps][2 n-tiles][32 lanes]
+//   inverse: F[2m + q][x] = cos / -sin(2 pi m x / T), ff: [T/32][4 n-tiles][32 lanes]
+__global__ void dft_frag_kernel(const float2* __restrict__ tw, int T, uint4* __restrict__ fe, uint4* __restrict__ ff) {
+	const int n = T / PX * 4 * 32;
+	for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 2 * n; e += gridDim.x * blockDim.x) {
+		const int f = e % n, lane = f & 31, g = lane >> 2, t = lane & 3, x0 = (f >> 7) * PX;
 		float v[4];
-		if (e < nx) {
-			const int lane = e & 31, nt = (e >> 5) & 1, ks = e >> 6;
-			const int col = 8 * nt + (lane >> 2), m = col >> 1, q = col & 1, t = lane & 3;
-			const int xs[4] = {16 * ks + 2 * t, 16 * ks + 2 * t + 1, 16 * ks + 2 * t + 8, 16 * ks + 2 * t + 9};
+		if (e < n) {
+			const int nt = (f >> 5) & 1, ks = (f >> 6) & 1;
+			const int col = 8 * nt + g, m = col >> 1, q = col & 1;
+			const int xs[4] = {px_of(2 * t, 2 * ks), px_of(2 * t + 1, 2 * ks), px_of(2 * t, 2 * ks + 1), px_of(2 * t + 1, 2 * ks + 1)};
 #pragma unroll
 			for (int k = 0; k < 4; k++) {
-				const float2 w = tw[(m * xs[k]) & (T - 1)];
+				const float2 w = tw[(m * (x0 + xs[k])) & (T - 1)];
 				v[k] = q ? -w.y : w.x;
 			}
 		} else {
-			const int f = e - nx, lane = f & 31, nt = f >> 5;
-			const int x = 8 * nt + (lane >> 2), t = lane & 3;
+			const int x = x0 + px_of(g, (f >> 5) & 3);
 			const float2 w0 = tw[(t * x) & (T - 1)], w4 = tw[((t + 4) * x) & (T - 1)];
 			v[0] = w0.x;
 			v[1] = -w0.y;
@@ -166,93 +185,658 @@ __global__ void dft_frag_kernel(const float2* __restrict__ tw, int T, uint4* __r
 		uint32_t h0, l0, h1, l1;
 		split2(v[0], v[1], h0, l0);
 		split2(v[2], v[3], h1, l1);
-		const uint4 r = make_uint4(h0, h1, l0, l1);
-		if (e < nx) fdx[e] = r;
-		else fix[e - nx] = r;
+		(e < n ? fe : ff)[f] = make_uint4(h0, h1, l0, l1);
 	}
 }
 
-// out[r][m] = scale[m] * sum_x in[r][x] exp(-2 pi i m x / T) for m < MX; one
-// warp per 16 rows
-__global__ void __launch_bounds__(256) dft_x(const float* __restrict__ in, float2* __restrict__ out,
-                                             const uint4* __restrict__ fdx, const float* __restrict__ scale,
-                                             long long nrows, int T) {
-	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-	const long long ntile = nrows / 16, nw = ((long long)gridDim.x * blockDim.x) >> 5;
-	for (long long tile = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; tile < ntile; tile += nw) {
-		const float* r0 = in + (tile * 16 + g) * T + 2 * t;
-		const float* r8 = r0 + 8LL * T;
-		float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-		for (int ks = 0; ks < T / 16; ks++) {
-			const float2 x0 = *reinterpret_cast<const float2*>(r0 + 16 * ks);
-			const float2 x1 = *reinterpret_cast<const float2*>(r8 + 16 * ks);
-			const float2 x2 = *reinterpret_cast<const float2*>(r0 + 16 * ks + 8);
-			const float2 x3 = *reinterpret_cast<const float2*>(r8 + 16 * ks + 8);
-			uint32_t ah[4], al[4];
-			split2(x0.x, x0.y, ah[0], al[0]);
-			split2(x1.x, x1.y, ah[1], al[1]);
-			split2(x2.x, x2.y, ah[2], al[2]);
-			split2(x3.x, x3.y, ah[3], al[3]);
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) {
+	*reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
+}
+// the caller's tensors need not be 16-byte aligned
+__device__ __forceinline__ float4 ld4u(const float* p, bool vec) {
+	return vec ? ld4(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+__device__ __forceinline__ float at(const float4& v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
+
+// an A fragment kept in shared memory (volatile: read at each use, not held)
+__device__ __forceinline__ void ld_frag(uint32_t (&a)[4], const uint4* p) {
+	asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+	             : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
+	             : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+
+// d += A B with A = (ah, al) and B = the fragment f split the same way
+__device__ __forceinline__ void mma_split(float (&d)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], const uint4& f) {
+	const uint32_t bh[2] = {f.x, f.y}, bl[2] = {f.z, f.w};
+	mma_bf16(d, ah, bh);
+	mma_bf16(d, ah, bl);
+	mma_bf16(d, al, bh);
+}
+
+// A fragments of the modes of rows (b, o, y), o = 16 mt + g and + 8: (Re, Im) of
+// modes t and t + 4, times their weights
+__device__ __forceinline__ void load_modes(const float2* __restrict__ z, long long b, int y, int T, int mt, int g, int t,
+                                           float s0, float s4, uint32_t (&ah)[4], uint32_t (&al)[4]) {
 #pragma unroll
-			for (int nt = 0; nt < 2; nt++) {
-				const uint4 f = __ldg(fdx + (ks * 2 + nt) * 32 + lane);
-				const uint32_t bh[2] = {f.x, f.y}, bl[2] = {f.z, f.w};
-				mma_bf16(acc[nt], ah, bh);
-				mma_bf16(acc[nt], ah, bl);
-				mma_bf16(acc[nt], al, bh);
-			}
-		}
-		// accumulator columns 2t, 2t + 1 of n-tile nt are (Re, Im) of mode 4 nt + t
-#pragma unroll
-		for (int nt = 0; nt < 2; nt++) {
-			const int m = 4 * nt + t;
-			const float sc = scale ? scale[m] : 1.f;
-			out[(tile * 16 + g) * MX + m] = make_float2(acc[nt][0] * sc, acc[nt][1] * sc);
-			out[(tile * 16 + g + 8) * MX + m] = make_float2(acc[nt][2] * sc, acc[nt][3] * sc);
-		}
+	for (int h = 0; h < 2; h++) {
+		const float2* p = z + ((b * C + 16 * mt + g + 8 * h) * T + y) * MX;
+		const float2 z0 = p[t], z4 = p[t + 4];
+		split2(s0 * z0.x, s0 * z0.y, ah[h], al[h]);
+		split2(s4 * z4.x, s4 * z4.y, ah[2 + h], al[2 + h]);
 	}
 }
 
-// out[r][x] (+)= sum_m scale[m] Re(in[r][m] exp(+2 pi i m x / T)); one warp per
-// 16 rows, eight points of each per n-tile
-__global__ void __launch_bounds__(256) idft_x(const float2* __restrict__ in, float* __restrict__ out,
-                                              const uint4* __restrict__ fix, const float* __restrict__ scale,
-                                              long long nrows, int T, int accumulate) {
-	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-	const float s0 = scale ? scale[t] : 1.f, s4 = scale ? scale[t + 4] : 1.f;
-	const long long ntile = nrows / 16, nw = ((long long)gridDim.x * blockDim.x) >> 5;
-	for (long long tile = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; tile < ntile; tile += nw) {
-		const long long ra = tile * 16 + g, rb = ra + 8;
-		const float2 z0 = in[ra * MX + t], z1 = in[rb * MX + t], z2 = in[ra * MX + t + 4], z3 = in[rb * MX + t + 4];
+// acc[nt] += the x transform of 32 pixels of 16 channels held as accumulators d[j]
+__device__ __forceinline__ void add_dft(float (&acc)[2][4], const float (&d)[4][4], const uint4* __restrict__ fe, int tile,
+                                        int lane) {
+#pragma unroll
+	for (int ks = 0; ks < 2; ks++) {
 		uint32_t ah[4], al[4];
-		split2(s0 * z0.x, s0 * z0.y, ah[0], al[0]);
-		split2(s0 * z1.x, s0 * z1.y, ah[1], al[1]);
-		split2(s4 * z2.x, s4 * z2.y, ah[2], al[2]);
-		split2(s4 * z3.x, s4 * z3.y, ah[3], al[3]);
-		float* oa = out + ra * T + 2 * t;
-		float* ob = out + rb * T + 2 * t;
-		for (int nt = 0; nt < T / 8; nt++) {
-			const uint4 f = __ldg(fix + nt * 32 + lane);
-			const uint32_t bh[2] = {f.x, f.y}, bl[2] = {f.z, f.w};
-			float d[4] = {0.f, 0.f, 0.f, 0.f};
-			mma_bf16(d, ah, bh);
-			mma_bf16(d, ah, bl);
-			mma_bf16(d, al, bh);
-			float2* pa = reinterpret_cast<float2*>(oa + 8 * nt);
-			float2* pb = reinterpret_cast<float2*>(ob + 8 * nt);
-			float2 va = make_float2(d[0], d[1]), vb = make_float2(d[2], d[3]);
-			if (accumulate) {
-				const float2 qa = *pa, qb = *pb;
-				va.x += qa.x;
-				va.y += qa.y;
-				vb.x += qb.x;
-				vb.y += qb.y;
-			}
-			*pa = va;
-			*pb = vb;
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			split2(d[2 * ks + h][0], d[2 * ks + h][1], ah[2 * h], al[2 * h]);
+			split2(d[2 * ks + h][2], d[2 * ks + h][3], ah[2 * h + 1], al[2 * h + 1]);
+		}
+#pragma unroll
+		for (int nt = 0; nt < 2; nt++) mma_split(acc[nt], ah, al, __ldg(fe + ((tile * 2 + ks) * 2 + nt) * 32 + lane));
+	}
+}
+
+// the rows' modes from those sums: columns 2t, 2t + 1 of n-tile nt are (Re, Im) of mode 4 nt + t
+__device__ __forceinline__ void store_modes(float2* __restrict__ out, const float (&acc)[2][4], long long b, int y, int T,
+                                            int mt, int g, int t, const float* __restrict__ scale) {
+#pragma unroll
+	for (int nt = 0; nt < 2; nt++) {
+		const int m = 4 * nt + t;
+		const float sc = scale ? scale[m] : 1.f;
+		float2* p = out + ((b * C + 16 * mt + g) * T + y) * MX + m;
+		p[0] = make_float2(acc[nt][0] * sc, acc[nt][1] * sc);
+		p[8LL * T * MX] = make_float2(acc[nt][2] * sc, acc[nt][3] * sc);
+	}
+}
+
+// x transform of the lifted input: v0 = P x + p is linear, so its modes are P times
+// those of x's two fields, plus p T at m = 0. One warp per eight rows, whose two
+// fields are the sixteen rows of an A operand.
+__global__ void __launch_bounds__(128) lift_dft(const float* __restrict__ x, int xvec, const __nv_bfloat16* __restrict__ w,
+                                                float2* __restrict__ out, const uint4* __restrict__ fe, long long nrows, int T) {
+	__shared__ float Ps[3 * C];
+	for (int i = threadIdx.x; i < 3 * C; i += blockDim.x) Ps[i] = wld(w, OFF_P + i);
+	__syncthreads();
+	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+	const long long npix = (long long)T * T, nw = ((long long)gridDim.x * blockDim.x) >> 5;
+	for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows / 8; r += nw) {
+		const long long b = r * 8 / T;
+		const int y = (int)(r * 8 - b * T) + g;
+		const float* p = x + b * 2 * npix + (long long)y * T + 4 * t;
+		float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll 2
+		for (int tile = 0; tile < T / PX; tile++) {
+			float d[4][4];
+#pragma unroll
+			for (int c = 0; c < 2; c++)
+#pragma unroll
+				for (int h = 0; h < 2; h++) {
+					const float4 q = ld4u(p + h * npix + tile * PX + 16 * c, xvec);
+					d[0][2 * h + c] = q.x;
+					d[1][2 * h + c] = q.y;
+					d[2][2 * h + c] = q.z;
+					d[3][2 * h + c] = q.w;
+				}
+			add_dft(acc, d, fe, tile, lane);
+		}
+		float2* o = out + (b * C * T + y) * MX + t;
+		for (int c = 0; c < C; c++) {
+			const float p0 = Ps[2 * c], p1 = Ps[2 * c + 1], pc = t == 0 ? Ps[2 * C + c] * (float)T : 0.f;
+			float2* q = o + (long long)c * T * MX;
+			q[0] = make_float2(p0 * acc[0][0] + p1 * acc[0][2] + pc, p0 * acc[0][1] + p1 * acc[0][3]);
+			q[4] = make_float2(p0 * acc[1][0] + p1 * acc[1][2], p0 * acc[1][1] + p1 * acc[1][3]);
 		}
 	}
 }
+
+
+// Two-field pixel values of a lane's column for all four n-tiles (channel values of
+// the lift's output), v0[c][px] = P[c][0] x0 + P[c][1] x1 + p[c]
+struct LiftRow {
+	float p0, p1, pc;
+	__device__ __forceinline__ void load(const __nv_bfloat16* w, int c) {
+		p0 = wld(w, OFF_P + 2 * c);
+		p1 = wld(w, OFF_P + 2 * c + 1);
+		pc = wld(w, OFF_PB + c);
+	}
+	__device__ __forceinline__ float4 of(const float4& a, const float4& b) const {
+		return make_float4(p0 * a.x + p1 * b.x + pc, p0 * a.y + p1 * b.y + pc, p0 * a.z + p1 * b.z + pc, p0 * a.w + p1 * b.w + pc);
+	}
+};
+
+// One layer forward, a warp per row (b, y): z = W v + b + K v with K v the inverse x
+// transform of the row's mixed modes Bq, v' = gelu(z). FIRST: v is the lift of x.
+// Every layer but the last leaves the x transform of v' in A; the last one projects:
+// out = x + Q z + q and, with a target, the loss, dy = 2 (out - target) / n and the
+// gradients of Q and q. v is read and v' (in training also z) written once, where
+// separate kernels for the transforms and the product moved them seven times: 16
+// tiles of 512^2 take 302 us a layer (1.07 GB, 0.16 ms at the memory's rate; 848 us
+// before). What is left is latency at 16 warps per SM, so registers are kept at 128
+// (168 and 12 warps: 406 us) with the weights' fragments in shared memory.
+template <bool FIRST, bool LAST, bool TRAIN>
+__global__ void __launch_bounds__(128, LAST ? 3 : 4)
+    layer_fwd(const float* __restrict__ x, int xvec, const float* v, const float2* __restrict__ Bq,
+              const __nv_bfloat16* __restrict__ w, int l, const uint4* __restrict__ fe, const uint4* __restrict__ ff,
+              const float* __restrict__ sx, float* z, float* vout, float2* __restrict__ A, float* __restrict__ out,
+              const float* __restrict__ target, float* __restrict__ dy, double* __restrict__ loss, float* __restrict__ gr,
+              long long nrows, int T, int B) {
+	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+	const long long npix = (long long)T * T;
+	__shared__ uint4 sw[4][32]; // the weights' A fragments (in registers they cost a block per SM)
+	uint32_t aw[2][2][4];
+	float bias[2][2], Qr[2][2][2];
+	LiftRow lift[2][4];
+#pragma unroll
+	for (int mt = 0; mt < 2; mt++) {
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			const int o = 16 * mt + g + 8 * h;
+			bias[mt][h] = wld(w, off_b(l) + o);
+#pragma unroll
+			for (int ks = 0; ks < 2; ks++) {
+				const size_t at_ = off_W(l) + (size_t)o * C + 16 * ks + 2 * t;
+				aw[mt][ks][h] = pack_bf16(w, at_, at_ + 1);
+				aw[mt][ks][2 + h] = pack_bf16(w, at_ + 8, at_ + 9);
+			}
+			if (LAST) {
+				Qr[0][mt][h] = wld(w, OFF_Q + o);
+				Qr[1][mt][h] = wld(w, OFF_Q + C + o);
+			}
+		}
+	}
+	if (FIRST) {
+#pragma unroll
+		for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+			for (int k = 0; k < 4; k++) lift[ks][k].load(w, 16 * ks + 2 * t + (k & 1) + 8 * (k >> 1));
+	}
+	if (threadIdx.x < 32)
+#pragma unroll
+		for (int k = 0; k < 4; k++) sw[k][lane] = make_uint4(aw[k >> 1][k & 1][0], aw[k >> 1][k & 1][1], aw[k >> 1][k & 1][2], aw[k >> 1][k & 1][3]);
+	__syncthreads();
+	const float s0 = sx[t], s4 = sx[t + 4];
+	const float qb[2] = {LAST ? wld(w, OFF_QB) : 0.f, LAST ? wld(w, OFF_QB + 1) : 0.f};
+	float gq[2][2][2], gqb = 0.f;
+	double lacc = 0.0;
+#pragma unroll
+	for (int j = 0; j < 2; j++)
+#pragma unroll
+		for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+			for (int h = 0; h < 2; h++) gq[j][mt][h] = 0.f;
+	const float inv = 2.f / (float)(2 * (long long)B * npix);
+
+	const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+	for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows; r += nw) {
+		const long long b = r / T;
+		const int y = (int)(r - b * T);
+		const long long base = b * C * npix + (long long)y * T, base2 = b * 2 * npix + (long long)y * T;
+		uint32_t mh[2][4], ml[2][4];
+		float acc[2][2][4];
+#pragma unroll
+		for (int mt = 0; mt < 2; mt++) {
+			load_modes(Bq, b, y, T, mt, g, t, s0, s4, mh[mt], ml[mt]);
+#pragma unroll
+			for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+				for (int k = 0; k < 4; k++) acc[mt][nt][k] = 0.f;
+		}
+		for (int tile = 0; tile < T / PX; tile++) {
+			const int pl = tile * PX + px_of(g, 0); // the lane's four columns' pixels
+			const int ps = tile * PX + 4 * t;       // the lane's result pixels (and + 16)
+			float4 vv[2][4];
+			if (FIRST) {
+				const float4 x0 = ld4u(x + base2 + pl, xvec), x1 = ld4u(x + base2 + npix + pl, xvec);
+#pragma unroll
+				for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+					for (int k = 0; k < 4; k++) vv[ks][k] = lift[ks][k].of(x0, x1);
+			} else {
+#pragma unroll
+				for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+					for (int k = 0; k < 4; k++) vv[ks][k] = ld4(v + base + (16 * ks + 2 * t + (k & 1) + 8 * (k >> 1)) * npix + pl);
+			}
+			float d[2][4][4];
+#pragma unroll
+			for (int j = 0; j < 4; j++) {
+				const uint4 f = __ldg(ff + (tile * 4 + j) * 32 + lane);
+#pragma unroll
+				for (int mt = 0; mt < 2; mt++) {
+					d[mt][j][0] = d[mt][j][1] = bias[mt][0];
+					d[mt][j][2] = d[mt][j][3] = bias[mt][1];
+					mma_split(d[mt][j], mh[mt], ml[mt], f);
+				}
+#pragma unroll
+				for (int ks = 0; ks < 2; ks++) {
+					uint32_t bh[2], bl[2];
+					split2(at(vv[ks][0], j), at(vv[ks][1], j), bh[0], bl[0]);
+					split2(at(vv[ks][2], j), at(vv[ks][3], j), bh[1], bl[1]);
+#pragma unroll
+					for (int mt = 0; mt < 2; mt++) {
+						uint32_t aq[4];
+						ld_frag(aq, &sw[2 * mt + ks][lane]);
+						mma_bf16(d[mt][j], aq, bh);
+						mma_bf16(d[mt][j], aq, bl);
+					}
+				}
+			}
+			if constexpr (!LAST) {
+#pragma unroll
+				for (int mt = 0; mt < 2; mt++) {
+#pragma unroll
+					for (int h = 0; h < 2; h++) {
+						const long long o = base + (16 * mt + g + 8 * h) * npix + ps;
+						if (TRAIN) {
+							st4(z + o, d[mt][0][2 * h], d[mt][1][2 * h], d[mt][2][2 * h], d[mt][3][2 * h]);
+							st4(z + o + 16, d[mt][0][2 * h + 1], d[mt][1][2 * h + 1], d[mt][2][2 * h + 1], d[mt][3][2 * h + 1]);
+						}
+#pragma unroll
+						for (int j = 0; j < 4; j++) {
+							d[mt][j][2 * h] = gelu(d[mt][j][2 * h]);
+							d[mt][j][2 * h + 1] = gelu(d[mt][j][2 * h + 1]);
+						}
+						st4(vout + o, d[mt][0][2 * h], d[mt][1][2 * h], d[mt][2][2 * h], d[mt][3][2 * h]);
+						st4(vout + o + 16, d[mt][0][2 * h + 1], d[mt][1][2 * h + 1], d[mt][2][2 * h + 1], d[mt][3][2 * h + 1]);
+					}
+					add_dft(acc[mt], d[mt], fe, tile, lane);
+				}
+			} else {
+				// Q z: the lane's rows, then over the eight g, halving what a lane keeps: it
+				// ends with field (lane >> 4), pixels ps + 16 (bit 3) + 2 (bit 2) + {0, 1}
+				float s[2][2][4];
+#pragma unroll
+				for (int f = 0; f < 2; f++)
+#pragma unroll
+					for (int c = 0; c < 2; c++)
+#pragma unroll
+						for (int j = 0; j < 4; j++)
+							s[f][c][j] = (Qr[f][0][0] * d[0][j][c] + Qr[f][0][1] * d[0][j][2 + c]) +
+							             (Qr[f][1][0] * d[1][j][c] + Qr[f][1][1] * d[1][j][2 + c]);
+				const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+				float u[2][4], q4[4], q2[2];
+#pragma unroll
+				for (int c = 0; c < 2; c++)
+#pragma unroll
+					for (int j = 0; j < 4; j++) {
+						const float keep = b4 ? s[1][c][j] : s[0][c][j], send = b4 ? s[0][c][j] : s[1][c][j];
+						u[c][j] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+					}
+#pragma unroll
+				for (int j = 0; j < 4; j++) {
+					const float keep = b3 ? u[1][j] : u[0][j], send = b3 ? u[0][j] : u[1][j];
+					q4[j] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+				}
+#pragma unroll
+				for (int j = 0; j < 2; j++) {
+					const float keep = b2 ? q4[2 + j] : q4[j], send = b2 ? q4[j] : q4[2 + j];
+					q2[j] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+				}
+				const long long i = base2 + (b4 ? npix : 0) + ps + (b3 ? 16 : 0) + (b2 ? 2 : 0);
+				float e[2];
+#pragma unroll
+				for (int j = 0; j < 2; j++) {
+					const float yv = x[i + j] + (q2[j] + (b4 ? qb[1] : qb[0]));
+					out[i + j] = yv;
+					if (TRAIN) {
+						const float er = yv - target[i + j];
+						lacc += (double)er * er;
+						e[j] = inv * er;
+						dy[i + j] = e[j];
+						gqb += e[j];
+					}
+				}
+				if constexpr (TRAIN) {
+					// every lane's sixteen dy values back, doubling what a lane has
+					float d4[4], d8[2][4], dd[2][2][4];
+#pragma unroll
+					for (int j = 0; j < 2; j++) {
+						const float o = __shfl_xor_sync(0xffffffffu, e[j], 4);
+						d4[j] = b2 ? o : e[j];
+						d4[2 + j] = b2 ? e[j] : o;
+					}
+#pragma unroll
+					for (int j = 0; j < 4; j++) {
+						const float o = __shfl_xor_sync(0xffffffffu, d4[j], 8);
+						d8[0][j] = b3 ? o : d4[j];
+						d8[1][j] = b3 ? d4[j] : o;
+					}
+#pragma unroll
+					for (int c = 0; c < 2; c++)
+#pragma unroll
+						for (int j = 0; j < 4; j++) {
+							const float o = __shfl_xor_sync(0xffffffffu, d8[c][j], 16);
+							dd[0][c][j] = b4 ? o : d8[c][j];
+							dd[1][c][j] = b4 ? d8[c][j] : o;
+						}
+#pragma unroll
+					for (int f = 0; f < 2; f++)
+#pragma unroll
+						for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+							for (int h = 0; h < 2; h++)
+#pragma unroll
+								for (int c = 0; c < 2; c++)
+#pragma unroll
+									for (int j = 0; j < 4; j++) gq[f][mt][h] += d[mt][j][2 * h + c] * dd[f][c][j];
+				}
+			}
+		}
+		if constexpr (!LAST) {
+#pragma unroll
+			for (int mt = 0; mt < 2; mt++) store_modes(A, acc[mt], b, y, T, mt, g, t, nullptr);
+		}
+	}
+	if constexpr (LAST && TRAIN) {
+		__shared__ float sq[2 * C + 2];
+		__shared__ double sl[4];
+		for (int i = threadIdx.x; i < 2 * C + 2; i += blockDim.x) sq[i] = 0.f;
+		__syncthreads();
+#pragma unroll
+		for (int f = 0; f < 2; f++)
+#pragma unroll
+			for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+				for (int h = 0; h < 2; h++) {
+					float a = gq[f][mt][h];
+					a += __shfl_xor_sync(0xffffffffu, a, 1);
+					a += __shfl_xor_sync(0xffffffffu, a, 2);
+					if (t == 0) atomicAdd(&sq[f * C + 16 * mt + g + 8 * h], a);
+				}
+#pragma unroll
+		for (int o = 8; o; o >>= 1) gqb += __shfl_xor_sync(0xffffffffu, gqb, o);
+		if ((lane & 15) == 0) atomicAdd(&sq[2 * C + (lane >> 4)], gqb);
+		lacc = warp_sum(lacc);
+		if (lane == 0) sl[threadIdx.x >> 5] = lacc;
+		__syncthreads();
+		for (int i = threadIdx.x; i < 2 * C + 2; i += blockDim.x) atomicAdd(gr + OFF_Q + i, sq[i]);
+		if (threadIdx.x == 0) atomicAdd(loss, (sl[0] + sl[1] + sl[2] + sl[3]) / (double)(2 * (long long)B * npix));
+	}
+}
+static_assert(OFF_QB == OFF_Q + 2 * C, "q follows Q");
+
+// First half of a layer backward, a warp per row: dz = dout gelu'(z) (the last layer:
+// dz = Q^T dy, not stored), written over dout; the x transform of dz, which starts
+// the spectral branch's adjoint; dW += dz v^T and db += dz summed over pixels.
+template <bool FIRST, bool LAST>
+__global__ void __launch_bounds__(128, 4)
+    layer_grad(const float* __restrict__ x, int xvec, const float* __restrict__ v, const float* __restrict__ z, float* dz,
+               const float* __restrict__ dy, const __nv_bfloat16* __restrict__ w, const uint4* __restrict__ fe,
+               const float* __restrict__ sx, float2* __restrict__ A, float* __restrict__ gW, float* __restrict__ gb,
+               long long nrows, int T) {
+	__shared__ float sW[C * C];
+	__shared__ float sb[C];
+	for (int i = threadIdx.x; i < C * C; i += blockDim.x) sW[i] = 0.f;
+	if (threadIdx.x < C) sb[threadIdx.x] = 0.f;
+	__syncthreads();
+	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+	const long long npix = (long long)T * T;
+	float aW[2][4][4], bsum[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, Qr[2][2][2];
+	LiftRow lift[4];
+#pragma unroll
+	for (int mt = 0; mt < 2; mt++) {
+#pragma unroll
+		for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+			for (int k = 0; k < 4; k++) aW[mt][nt][k] = 0.f;
+		if (LAST) {
+#pragma unroll
+			for (int h = 0; h < 2; h++) {
+				Qr[0][mt][h] = wld(w, OFF_Q + 16 * mt + g + 8 * h);
+				Qr[1][mt][h] = wld(w, OFF_Q + C + 16 * mt + g + 8 * h);
+			}
+		}
+	}
+	if (FIRST) {
+#pragma unroll
+		for (int nt = 0; nt < 4; nt++) lift[nt].load(w, 8 * nt + g);
+	}
+	const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+	for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows; r += nw) {
+		const long long b = r / T;
+		const int y = (int)(r - b * T);
+		const long long base = b * C * npix + (long long)y * T, base2 = b * 2 * npix + (long long)y * T;
+		float acc[2][2][4];
+#pragma unroll
+		for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+			for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+				for (int k = 0; k < 4; k++) acc[mt][nt][k] = 0.f;
+		for (int tile = 0; tile < T / PX; tile++) {
+			const int ps = tile * PX + 4 * t;
+			// v^T as B fragments: channel 8 nt + g at the lane's pixels
+			uint32_t vh[2][4][2], vl[2][4][2];
+#pragma unroll
+			for (int nt = 0; nt < 4; nt++) {
+				float4 a, c;
+				if (FIRST) {
+					a = lift[nt].of(ld4u(x + base2 + ps, xvec), ld4u(x + base2 + npix + ps, xvec));
+					c = lift[nt].of(ld4u(x + base2 + ps + 16, xvec), ld4u(x + base2 + npix + ps + 16, xvec));
+				} else {
+					a = ld4(v + base + (8 * nt + g) * npix + ps);
+					c = ld4(v + base + (8 * nt + g) * npix + ps + 16);
+				}
+				split2(a.x, c.x, vh[0][nt][0], vl[0][nt][0]);
+				split2(a.y, c.y, vh[0][nt][1], vl[0][nt][1]);
+				split2(a.z, c.z, vh[1][nt][0], vl[1][nt][0]);
+				split2(a.w, c.w, vh[1][nt][1], vl[1][nt][1]);
+			}
+#pragma unroll
+			for (int mt = 0; mt < 2; mt++) {
+				float d[4][4]; // dz as the accumulators of four n-tiles
+#pragma unroll
+				for (int h = 0; h < 2; h++) {
+					const long long o = base + (16 * mt + g + 8 * h) * npix + ps;
+#pragma unroll
+					for (int c = 0; c < 2; c++) {
+						float4 q;
+						if (LAST) {
+							const float4 e0 = ld4(dy + base2 + ps + 16 * c), e1 = ld4(dy + base2 + npix + ps + 16 * c);
+							const float a0 = Qr[0][mt][h], a1 = Qr[1][mt][h];
+							q = make_float4(a0 * e0.x + a1 * e1.x, a0 * e0.y + a1 * e1.y, a0 * e0.z + a1 * e1.z, a0 * e0.w + a1 * e1.w);
+						} else {
+							const float4 go = ld4(dz + o + 16 * c), zz = ld4(z + o + 16 * c);
+							q = make_float4(go.x * gelu_d(zz.x), go.y * gelu_d(zz.y), go.z * gelu_d(zz.z), go.w * gelu_d(zz.w));
+							st4(dz + o + 16 * c, q.x, q.y, q.z, q.w);
+						}
+						bsum[mt][h] += (q.x + q.y) + (q.z + q.w);
+						d[0][2 * h + c] = q.x;
+						d[1][2 * h + c] = q.y;
+						d[2][2 * h + c] = q.z;
+						d[3][2 * h + c] = q.w;
+					}
+				}
+#pragma unroll
+				for (int ks = 0; ks < 2; ks++) {
+					uint32_t ah[4], al[4];
+#pragma unroll
+					for (int h = 0; h < 2; h++) {
+						split2(d[2 * ks + h][0], d[2 * ks + h][1], ah[2 * h], al[2 * h]);
+						split2(d[2 * ks + h][2], d[2 * ks + h][3], ah[2 * h + 1], al[2 * h + 1]);
+					}
+#pragma unroll
+					for (int nt = 0; nt < 2; nt++) mma_split(acc[mt][nt], ah, al, __ldg(fe + ((tile * 2 + ks) * 2 + nt) * 32 + lane));
+#pragma unroll
+					for (int nt = 0; nt < 4; nt++) {
+						mma_bf16(aW[mt][nt], ah, vh[ks][nt]);
+						mma_bf16(aW[mt][nt], ah, vl[ks][nt]);
+						mma_bf16(aW[mt][nt], al, vh[ks][nt]);
+					}
+				}
+			}
+		}
+#pragma unroll
+		for (int mt = 0; mt < 2; mt++) store_modes(A, acc[mt], b, y, T, mt, g, t, sx);
+	}
+#pragma unroll
+	for (int mt = 0; mt < 2; mt++) {
+#pragma unroll
+		for (int nt = 0; nt < 4; nt++) {
+			const int o = 16 * mt + g, i = 8 * nt + 2 * t;
+			atomicAdd(&sW[o * C + i], aW[mt][nt][0]);
+			atomicAdd(&sW[o * C + i + 1], aW[mt][nt][1]);
+			atomicAdd(&sW[(o + 8) * C + i], aW[mt][nt][2]);
+			atomicAdd(&sW[(o + 8) * C + i + 1], aW[mt][nt][3]);
+		}
+		// bias: the four lanes of a group hold disjoint pixels of the same rows
+#pragma unroll
+		for (int h = 0; h < 2; h++) {
+			float q = bsum[mt][h];
+			q += __shfl_xor_sync(0xffffffffu, q, 1);
+			q += __shfl_xor_sync(0xffffffffu, q, 2);
+			if (t == 0) atomicAdd(&sb[16 * mt + g + 8 * h], q);
+		}
+	}
+	__syncthreads();
+	for (int i = threadIdx.x; i < C * C; i += blockDim.x) atomicAdd(&gW[i], sW[i]);
+	if (threadIdx.x < C) atomicAdd(&gb[threadIdx.x], sb[threadIdx.x]);
+}
+
+// Second half, a warp per row: dv = W^T dz + the x transform's adjoint of the mixed
+// modes, written over dz. LAST: dz = Q^T dy. FIRST: dv is not stored; dP[c][j] +=
+// dv[c] x[j] and dp[c] += dv[c], summed over pixels.
+template <bool FIRST, bool LAST>
+__global__ void __launch_bounds__(128, 3)
+    layer_bwd(const float* __restrict__ x, int xvec, const float* __restrict__ dy, const float2* __restrict__ Aq,
+              const __nv_bfloat16* __restrict__ w, int l, const uint4* __restrict__ ff, float* dz, float* __restrict__ gr,
+              long long nrows, int T) {
+	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+	const long long npix = (long long)T * T;
+	__shared__ uint4 sw[4][32]; // the weights' A fragments (in registers they cost a block per SM)
+	uint32_t aw[2][2][4];
+	float Qk[2][2][4], gp[3][2][2];
+#pragma unroll
+	for (int ks = 0; ks < 2; ks++) {
+		const int o = 16 * ks + 2 * t;
+#pragma unroll
+		for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+			for (int h = 0; h < 2; h++) {
+				const size_t col = off_W(l) + 16 * mt + g + 8 * h; // W[o][i] at col + o C
+				aw[mt][ks][h] = pack_bf16(w, col + (size_t)o * C, col + (size_t)(o + 1) * C);
+				aw[mt][ks][2 + h] = pack_bf16(w, col + (size_t)(o + 8) * C, col + (size_t)(o + 9) * C);
+			}
+		if (LAST) {
+#pragma unroll
+			for (int k = 0; k < 4; k++) {
+				Qk[0][ks][k] = wld(w, OFF_Q + o + (k & 1) + 8 * (k >> 1));
+				Qk[1][ks][k] = wld(w, OFF_Q + C + o + (k & 1) + 8 * (k >> 1));
+			}
+		}
+	}
+	if (threadIdx.x < 32)
+#pragma unroll
+		for (int k = 0; k < 4; k++) sw[k][lane] = make_uint4(aw[k >> 1][k & 1][0], aw[k >> 1][k & 1][1], aw[k >> 1][k & 1][2], aw[k >> 1][k & 1][3]);
+	__syncthreads();
+#pragma unroll
+	for (int j = 0; j < 3; j++)
+#pragma unroll
+		for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+			for (int h = 0; h < 2; h++) gp[j][mt][h] = 0.f;
+	const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+	for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows; r += nw) {
+		const long long b = r / T;
+		const int y = (int)(r - b * T);
+		const long long base = b * C * npix + (long long)y * T, base2 = b * 2 * npix + (long long)y * T;
+		uint32_t mh[2][4], ml[2][4];
+#pragma unroll
+		for (int mt = 0; mt < 2; mt++) load_modes(Aq, b, y, T, mt, g, t, 1.f, 1.f, mh[mt], ml[mt]);
+		for (int tile = 0; tile < T / PX; tile++) {
+			const int pl = tile * PX + px_of(g, 0), ps = tile * PX + 4 * t;
+			float4 vv[2][4];
+			if (LAST) {
+				const float4 e0 = ld4(dy + base2 + pl), e1 = ld4(dy + base2 + npix + pl);
+#pragma unroll
+				for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+					for (int k = 0; k < 4; k++) {
+						const float a0 = Qk[0][ks][k], a1 = Qk[1][ks][k];
+						vv[ks][k] = make_float4(a0 * e0.x + a1 * e1.x, a0 * e0.y + a1 * e1.y, a0 * e0.z + a1 * e1.z, a0 * e0.w + a1 * e1.w);
+					}
+			} else {
+#pragma unroll
+				for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+					for (int k = 0; k < 4; k++) vv[ks][k] = ld4(dz + base + (16 * ks + 2 * t + (k & 1) + 8 * (k >> 1)) * npix + pl);
+			}
+			float d[2][4][4];
+#pragma unroll
+			for (int j = 0; j < 4; j++) {
+				const uint4 f = __ldg(ff + (tile * 4 + j) * 32 + lane);
+#pragma unroll
+				for (int mt = 0; mt < 2; mt++) {
+#pragma unroll
+					for (int k = 0; k < 4; k++) d[mt][j][k] = 0.f;
+					mma_split(d[mt][j], mh[mt], ml[mt], f);
+				}
+#pragma unroll
+				for (int ks = 0; ks < 2; ks++) {
+					uint32_t bh[2], bl[2];
+					split2(at(vv[ks][0], j), at(vv[ks][1], j), bh[0], bl[0]);
+					split2(at(vv[ks][2], j), at(vv[ks][3], j), bh[1], bl[1]);
+#pragma unroll
+					for (int mt = 0; mt < 2; mt++) {
+						uint32_t aq[4];
+						ld_frag(aq, &sw[2 * mt + ks][lane]);
+						mma_bf16(d[mt][j], aq, bh);
+						mma_bf16(d[mt][j], aq, bl);
+					}
+				}
+			}
+			__syncwarp(); // every lane's loads of this block before its stores over it
+#pragma unroll
+			for (int c = 0; c < 2; c++) {
+				float4 x0, x1;
+				if (FIRST) {
+					x0 = ld4u(x + base2 + ps + 16 * c, xvec);
+					x1 = ld4u(x + base2 + npix + ps + 16 * c, xvec);
+				}
+#pragma unroll
+				for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+					for (int h = 0; h < 2; h++) {
+						const float a0 = d[mt][0][2 * h + c], a1 = d[mt][1][2 * h + c], a2 = d[mt][2][2 * h + c], a3 = d[mt][3][2 * h + c];
+						if (FIRST) {
+							gp[0][mt][h] += (a0 * x0.x + a1 * x0.y) + (a2 * x0.z + a3 * x0.w);
+							gp[1][mt][h] += (a0 * x1.x + a1 * x1.y) + (a2 * x1.z + a3 * x1.w);
+							gp[2][mt][h] += (a0 + a1) + (a2 + a3);
+						} else {
+							st4(dz + base + (16 * mt + g + 8 * h) * npix + ps + 16 * c, a0, a1, a2, a3);
+						}
+					}
+			}
+		}
+	}
+	if constexpr (FIRST) {
+		__shared__ float sp[3 * C];
+		for (int i = threadIdx.x; i < 3 * C; i += blockDim.x) sp[i] = 0.f;
+		__syncthreads();
+#pragma unroll
+		for (int j = 0; j < 3; j++)
+#pragma unroll
+			for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+				for (int h = 0; h < 2; h++) {
+					float a = gp[j][mt][h];
+					a += __shfl_xor_sync(0xffffffffu, a, 1);
+					a += __shfl_xor_sync(0xffffffffu, a, 2);
+					const int c = 16 * mt + g + 8 * h;
+					if (t == 0) atomicAdd(&sp[j < 2 ? 2 * c + j : 2 * C + c], a);
+				}
+		__syncthreads();
+		for (int i = threadIdx.x; i < 3 * C; i += blockDim.x) atomicAdd(gr + OFF_P + i, sp[i]);
+	}
+}
+static_assert(OFF_PB == OFF_P + 2 * C, "p follows P");
 
 // The truncated transforms along y, per plane of [rows][MX] complex values:
 //   forward: out[k][m] = sum_y in[y][m] exp(-2 pi i ky(k) y / T), k < MY
@@ -322,6 +906,7 @@ __global__ void __launch_bounds__(32 * DY_WARPS) dft_y_fwd(const float2* __restr
 	for (long long plane = blockIdx.x; plane < nplanes; plane += gridDim.x) {
 		const float2* pin = in + plane * T * MX;
 		float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll 4
 		for (int ks = wp; ks < T / 8; ks += DY_WARPS) {
 			const uint4 fh = __ldg(fdy + (ks * 32 + lane) * 2), fl = __ldg(fdy + (ks * 32 + lane) * 2 + 1);
 			const uint32_t ah[4] = {fh.x, fh.y, fh.z, fh.w}, al[4] = {fl.x, fl.y, fl.z, fl.w};
@@ -371,6 +956,7 @@ __global__ void __launch_bounds__(32 * DY_WARPS) dft_y_inv(const float2* __restr
 				zsplit(pin[(k0 + 4) * MX + m], q, bh[ks][nt][1], bl[ks][nt][1]);
 			}
 		float2* pout = out + plane * T * MX;
+#pragma unroll 2
 		for (int mt = wp; mt < T / 16; mt += DY_WARPS) {
 			float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
@@ -474,330 +1060,6 @@ __global__ void mix_grad(const float2* __restrict__ X, const float2* __restrict_
 	}
 }
 
-// z = W v + b + s; out = gelu(z) (act) or z. One warp per 16-pixel tile:
-// D[pixel][out] = sum_in A[pixel][in] B[in][out] with A = v, B = W^T.
-__global__ void __launch_bounds__(128, 4) pointwise_fwd(const float* __restrict__ v, const float* __restrict__ s,
-                                                     const __nv_bfloat16* __restrict__ w, int l, float* __restrict__ z,
-                                                     float* __restrict__ out, int B, int npix, int act) {
-	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-	uint32_t bw[4][2][2];
-	float bias[4][2];
-#pragma unroll
-	for (int nt = 0; nt < 4; nt++) {
-		const size_t row = off_W(l) + (size_t)(8 * nt + g) * C;
-#pragma unroll
-		for (int ks = 0; ks < 2; ks++) {
-			bw[nt][ks][0] = pack_bf16(w, row + 16 * ks + 2 * t, row + 16 * ks + 2 * t + 1);
-			bw[nt][ks][1] = pack_bf16(w, row + 16 * ks + 2 * t + 8, row + 16 * ks + 2 * t + 9);
-		}
-		bias[nt][0] = wld(w, off_b(l) + 8 * nt + 2 * t);
-		bias[nt][1] = wld(w, off_b(l) + 8 * nt + 2 * t + 1);
-	}
-	const int tpi = npix / 16;
-	const long long ntile = (long long)B * tpi;
-	const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-	for (long long tile = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; tile < ntile; tile += nw) {
-		const long long b = tile / tpi;
-		const long long base = b * C * npix + (tile - b * tpi) * 16;
-		uint32_t ah[2][4], al[2][4];
-#pragma unroll
-		for (int ks = 0; ks < 2; ks++) {
-			const float* c0 = v + base + (long long)(16 * ks + 2 * t) * npix;
-			const float* c1 = c0 + npix;
-			const float* c8 = c0 + 8LL * npix;
-			const float* c9 = c8 + npix;
-			split2(c0[g], c1[g], ah[ks][0], al[ks][0]);
-			split2(c0[g + 8], c1[g + 8], ah[ks][1], al[ks][1]);
-			split2(c8[g], c9[g], ah[ks][2], al[ks][2]);
-			split2(c8[g + 8], c9[g + 8], ah[ks][3], al[ks][3]);
-		}
-#pragma unroll
-		for (int nt = 0; nt < 4; nt++) {
-			const long long o0 = base + (long long)(8 * nt + 2 * t) * npix, o1 = o0 + npix;
-			float d[4] = {bias[nt][0] + s[o0 + g], bias[nt][1] + s[o1 + g], bias[nt][0] + s[o0 + g + 8],
-			              bias[nt][1] + s[o1 + g + 8]};
-#pragma unroll
-			for (int ks = 0; ks < 2; ks++) {
-				mma_bf16(d, ah[ks], bw[nt][ks]);
-				mma_bf16(d, al[ks], bw[nt][ks]);
-			}
-			if (z) {
-				z[o0 + g] = d[0];
-				z[o1 + g] = d[1];
-				z[o0 + g + 8] = d[2];
-				z[o1 + g + 8] = d[3];
-			}
-			out[o0 + g] = act ? gelu(d[0]) : d[0];
-			out[o1 + g] = act ? gelu(d[1]) : d[1];
-			out[o0 + g + 8] = act ? gelu(d[2]) : d[2];
-			out[o1 + g + 8] = act ? gelu(d[3]) : d[3];
-		}
-	}
-}
-
-// dz = dout * g'(z) (also the gradient of the spectral branch); dv = W^T dz:
-// D[pixel][in] = sum_out A[pixel][out] B[out][in] with A = dz, B = W.
-__global__ void __launch_bounds__(128, 4) pointwise_bwd(const float* __restrict__ z, const float* __restrict__ dout,
-                                                     const __nv_bfloat16* __restrict__ w, int l, float* __restrict__ dz,
-                                                     float* __restrict__ dv, int B, int npix, int act) {
-	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-	uint32_t bw[4][2][2];
-#pragma unroll
-	for (int nt = 0; nt < 4; nt++) {
-		const size_t col = off_W(l) + 8 * nt + g; // W[o][i = 8 nt + g] at col + o C
-#pragma unroll
-		for (int ks = 0; ks < 2; ks++) {
-			const int o = 16 * ks + 2 * t;
-			bw[nt][ks][0] = pack_bf16(w, col + (size_t)o * C, col + (size_t)(o + 1) * C);
-			bw[nt][ks][1] = pack_bf16(w, col + (size_t)(o + 8) * C, col + (size_t)(o + 9) * C);
-		}
-	}
-	const int tpi = npix / 16;
-	const long long ntile = (long long)B * tpi;
-	const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-	for (long long tile = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; tile < ntile; tile += nw) {
-		const long long b = tile / tpi;
-		const long long base = b * C * npix + (tile - b * tpi) * 16;
-		uint32_t ah[2][4], al[2][4];
-#pragma unroll
-		for (int ks = 0; ks < 2; ks++) {
-			float dd[8];
-			const int och[4] = {16 * ks + 2 * t, 16 * ks + 2 * t + 1, 16 * ks + 2 * t + 8, 16 * ks + 2 * t + 9};
-#pragma unroll
-			for (int q = 0; q < 4; q++)
-#pragma unroll
-				for (int h = 0; h < 2; h++) {
-					const long long i = base + (long long)och[q] * npix + g + 8 * h;
-					const float gv = dout[i];
-					const float d = act ? gv * gelu_d(z[i]) : gv;
-					dz[i] = d;
-					dd[2 * q + h] = d;
-				}
-			// a0 (g; o, o+1), a1 (g+8; o, o+1), a2 (g; o+8, o+9), a3 (g+8; o+8, o+9)
-			split2(dd[0], dd[2], ah[ks][0], al[ks][0]);
-			split2(dd[1], dd[3], ah[ks][1], al[ks][1]);
-			split2(dd[4], dd[6], ah[ks][2], al[ks][2]);
-			split2(dd[5], dd[7], ah[ks][3], al[ks][3]);
-		}
-#pragma unroll
-		for (int nt = 0; nt < 4; nt++) {
-			float d[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-			for (int ks = 0; ks < 2; ks++) {
-				mma_bf16(d, ah[ks], bw[nt][ks]);
-				mma_bf16(d, al[ks], bw[nt][ks]);
-			}
-			const long long i0 = base + (long long)(8 * nt + 2 * t) * npix, i1 = i0 + npix;
-			dv[i0 + g] = d[0];
-			dv[i1 + g] = d[1];
-			dv[i0 + g + 8] = d[2];
-			dv[i1 + g + 8] = d[3];
-		}
-	}
-}
-
-// dW[o][i] += sum_p dz[o][p] v[i][p], db[o] += sum_p dz[o][p]: D[o][i] = sum_p
-// A[o][p] B[p][i] with A = dz, B = v^T, 16 pixels per step; each warp sums its
-// tiles, the block adds its warps in shared memory, then one atomic per entry.
-constexpr int WG_THREADS = 256;
-__global__ void __launch_bounds__(WG_THREADS) weight_grad(const float* __restrict__ dz, const float* __restrict__ v,
-                                                          float* __restrict__ gW, float* __restrict__ gb, int B,
-                                                          int npix) {
-	__shared__ float sW[C * C];
-	__shared__ float sb[C];
-	for (int i = threadIdx.x; i < C * C; i += blockDim.x) sW[i] = 0.f;
-	if (threadIdx.x < C) sb[threadIdx.x] = 0.f;
-	__syncthreads();
-	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-	float acc[2][4][4];
-#pragma unroll
-	for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-		for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-			for (int k = 0; k < 4; k++) acc[mt][nt][k] = 0.f;
-	float bsum[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-	const int tpi = npix / 16;
-	const long long ntile = (long long)B * tpi;
-	const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-	for (long long tile = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; tile < ntile; tile += nw) {
-		const long long b = tile / tpi;
-		const long long base = b * C * npix + (tile - b * tpi) * 16 + 2 * t;
-		uint32_t ah[2][4], al[2][4], bh[4][2], bl[4][2];
-#pragma unroll
-		for (int mt = 0; mt < 2; mt++) {
-			const float* r0 = dz + base + (long long)(16 * mt + g) * npix;
-			const float* r8 = r0 + 8LL * npix;
-			const float2 x0 = *reinterpret_cast<const float2*>(r0), x1 = *reinterpret_cast<const float2*>(r8);
-			const float2 x2 = *reinterpret_cast<const float2*>(r0 + 8), x3 = *reinterpret_cast<const float2*>(r8 + 8);
-			split2(x0.x, x0.y, ah[mt][0], al[mt][0]);
-			split2(x1.x, x1.y, ah[mt][1], al[mt][1]);
-			split2(x2.x, x2.y, ah[mt][2], al[mt][2]);
-			split2(x3.x, x3.y, ah[mt][3], al[mt][3]);
-			bsum[mt][0] += (x0.x + x0.y) + (x2.x + x2.y);
-			bsum[mt][1] += (x1.x + x1.y) + (x3.x + x3.y);
-		}
-#pragma unroll
-		for (int nt = 0; nt < 4; nt++) {
-			const float* r = v + base + (long long)(8 * nt + g) * npix;
-			const float2 y0 = *reinterpret_cast<const float2*>(r), y1 = *reinterpret_cast<const float2*>(r + 8);
-			split2(y0.x, y0.y, bh[nt][0], bl[nt][0]);
-			split2(y1.x, y1.y, bh[nt][1], bl[nt][1]);
-		}
-#pragma unroll
-		for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-			for (int nt = 0; nt < 4; nt++) {
-				mma_bf16(acc[mt][nt], ah[mt], bh[nt]);
-				mma_bf16(acc[mt][nt], ah[mt], bl[nt]);
-				mma_bf16(acc[mt][nt], al[mt], bh[nt]);
-			}
-	}
-#pragma unroll
-	for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-		for (int nt = 0; nt < 4; nt++) {
-			const int o = 16 * mt + g, i = 8 * nt + 2 * t;
-			atomicAdd(&sW[o * C + i], acc[mt][nt][0]);
-			atomicAdd(&sW[o * C + i + 1], acc[mt][nt][1]);
-			atomicAdd(&sW[(o + 8) * C + i], acc[mt][nt][2]);
-			atomicAdd(&sW[(o + 8) * C + i + 1], acc[mt][nt][3]);
-		}
-	// bias: the four lanes of a group hold disjoint pixels of the same rows
-#pragma unroll
-	for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-		for (int h = 0; h < 2; h++) {
-			float x = bsum[mt][h];
-			x += __shfl_xor_sync(0xffffffffu, x, 1);
-			x += __shfl_xor_sync(0xffffffffu, x, 2);
-			if (t == 0) atomicAdd(&sb[16 * mt + g + 8 * h], x);
-		}
-	__syncthreads();
-	for (int i = threadIdx.x; i < C * C; i += blockDim.x) atomicAdd(&gW[i], sW[i]);
-	if (threadIdx.x < C) atomicAdd(&gb[threadIdx.x], sb[threadIdx.x]);
-}
-
-// y = x + Q v + q; with a target also loss += sum (y - t)^2 / n and dy = 2 (y - t) / n
-__global__ void proj_fwd_loss(const float* __restrict__ x, const float* __restrict__ v, const __nv_bfloat16* __restrict__ w,
-                              float* __restrict__ y, const float* __restrict__ target, float* __restrict__ dy,
-                              double* __restrict__ loss, int B, int npix) {
-	__shared__ float Qs[2 * C + 2];
-	__shared__ double red[32];
-	for (int i = threadIdx.x; i < 2 * C + 2; i += blockDim.x) Qs[i] = wld(w, OFF_Q + i);
-	__syncthreads();
-	const long long n = (long long)B * npix;
-	const float inv = 2.f / (float)(2 * n);
-	double acc = 0.0;
-	for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-		const long long b = t / npix;
-		const int p = (int)(t - b * npix);
-		const float* vb = v + b * C * npix + p;
-		float o0 = Qs[2 * C], o1 = Qs[2 * C + 1];
-#pragma unroll 8
-		for (int c = 0; c < C; c++) {
-			const float vv = vb[(long long)c * npix];
-			o0 += Qs[c] * vv;
-			o1 += Qs[C + c] * vv;
-		}
-		const long long i0 = b * 2 * npix + p, i1 = i0 + npix;
-		const float y0 = x[i0] + o0, y1 = x[i1] + o1;
-		y[i0] = y0;
-		y[i1] = y1;
-		if (target) {
-			const float e0 = y0 - target[i0], e1 = y1 - target[i1];
-			acc += (double)e0 * e0 + (double)e1 * e1;
-			dy[i0] = inv * e0;
-			dy[i1] = inv * e1;
-		}
-	}
-	if (target) {
-		acc = warp_sum(acc);
-		if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-		__syncthreads();
-		if (threadIdx.x < 32) {
-			double a = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-			a = warp_sum(a);
-			if (threadIdx.x == 0) atomicAdd(loss, a / (double)(2 * n));
-		}
-	}
-}
-
-// dv = Q^T dy
-__global__ void proj_bwd(const float* __restrict__ dy, const __nv_bfloat16* __restrict__ w, float* __restrict__ dv, int B,
-                         int npix) {
-	__shared__ float Qs[2 * C];
-	for (int i = threadIdx.x; i < 2 * C; i += blockDim.x) Qs[i] = wld(w, OFF_Q + i);
-	__syncthreads();
-	const long long n = (long long)B * npix;
-	for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-		const long long b = t / npix;
-		const int p = (int)(t - b * npix);
-		const float d0 = dy[b * 2 * npix + p], d1 = dy[b * 2 * npix + npix + p];
-		float* db = dv + b * C * npix + p;
-#pragma unroll 8
-		for (int c = 0; c < C; c++) db[(long long)c * npix] = Qs[c] * d0 + Qs[C + c] * d1;
-	}
-}
-
-// Per-channel sums over all pixels of a[b][c][p] * e[b][j][p] (j = 0, 1; e a
-// two-field tensor) and of a itself. Gradients of the lift (a = dv0, e = x;
-// g_ae = dP [C][2], g_a = dp [C]) and of the projection (a = v_L, e = dy;
-// g_ae = dQ [2][C]). One block row per channel (blockIdx.y).
-__global__ void channel_grad(const float* __restrict__ a, const float* __restrict__ e, float* __restrict__ g_ae,
-                             int stride_c, int stride_j, float* __restrict__ g_a, int B, int npix) {
-	__shared__ float red[3][32];
-	const int c = blockIdx.y;
-	const long long n = (long long)B * npix;
-	float s0 = 0.f, s1 = 0.f, sa = 0.f;
-	for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-		const long long b = t / npix;
-		const int p = (int)(t - b * npix);
-		const float av = a[(b * C + c) * npix + p];
-		s0 += av * e[(b * 2) * npix + p];
-		s1 += av * e[(b * 2 + 1) * npix + p];
-		sa += av;
-	}
-	s0 = warp_sum(s0);
-	s1 = warp_sum(s1);
-	sa = warp_sum(sa);
-	if ((threadIdx.x & 31) == 0) {
-		red[0][threadIdx.x >> 5] = s0;
-		red[1][threadIdx.x >> 5] = s1;
-		red[2][threadIdx.x >> 5] = sa;
-	}
-	__syncthreads();
-	if (threadIdx.x < 32) {
-		const bool in = threadIdx.x < (blockDim.x >> 5);
-		s0 = warp_sum(in ? red[0][threadIdx.x] : 0.f);
-		s1 = warp_sum(in ? red[1][threadIdx.x] : 0.f);
-		sa = warp_sum(in ? red[2][threadIdx.x] : 0.f);
-		if (threadIdx.x == 0) {
-			atomicAdd(&g_ae[c * stride_c], s0);
-			atomicAdd(&g_ae[c * stride_c + stride_j], s1);
-			if (g_a) atomicAdd(&g_a[c], sa);
-		}
-	}
-}
-
-// g[j] += sum over pixels of e[b][j][p], j = 0, 1
-__global__ void sum2_kernel(const float* __restrict__ e, float* __restrict__ g, int B, int npix) {
-	const long long n = (long long)B * npix;
-	float s0 = 0.f, s1 = 0.f;
-	for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-		const long long b = t / npix;
-		const int p = (int)(t - b * npix);
-		s0 += e[b * 2 * npix + p];
-		s1 += e[b * 2 * npix + npix + p];
-	}
-	s0 = warp_sum(s0);
-	s1 = warp_sum(s1);
-	if ((threadIdx.x & 31) == 0) {
-		atomicAdd(&g[0], s0);
-		atomicAdd(&g[1], s1);
-	}
-}
-
 __global__ void to_bf16(const float* __restrict__ a, __nv_bfloat16* __restrict__ b, long long n) {
 	for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
 		b[i] = __float2bfloat16(a[i]);
@@ -818,41 +1080,40 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
 
 // Tiles of a periodic two-field FP64 grid as FP32 network input. Tile j of the
 // batch is block (first + j) of the grid's core x core blocks (row-major over
-// tiles_x columns) plus halo points on each side, wrapped periodically.
+// tiles_x columns) plus halo points on each side, wrapped periodically. One warp
+// per row of a tile and field.
 __global__ void gather_tiles(const double* __restrict__ f, float* __restrict__ out, int Nx, int Ny, int T, int core,
                              int halo, int tiles_x, int first, int count) {
-	const long long per = 2LL * T * T;
-	const long long n = per * count;
-	for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-		const int j = (int)(t / per);
-		const int r = (int)(t - (long long)j * per);
-		const int u = r / (T * T), q = r - u * T * T;
-		const int ty = q / T, tx = q - ty * T;
-		const int tile = first + j;
+	const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+	for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < 2 * T * count; r += nw) {
+		const int ty = r % T, u = (r / T) & 1, tile = first + r / (2 * T);
 		const int by = tile / tiles_x, bx = tile - by * tiles_x;
-		int x = (bx * core - halo + tx) % Nx, y = (by * core - halo + ty) % Ny;
-		if (x < 0) x += Nx;
+		int y = (by * core - halo + ty) % Ny, x0 = (bx * core - halo) % Nx;
 		if (y < 0) y += Ny;
-		out[t] = (float)f[((long long)u * Ny + y) * Nx + x];
+		if (x0 < 0) x0 += Nx;
+		const double* row = f + ((long long)u * Ny + y) * Nx;
+		float* o = out + (long long)r * T;
+		for (int tx = lane; tx < T; tx += 32) {
+			int x = x0 + tx;
+			while (x >= Nx) x -= Nx; // at most T / Nx turns
+			o[tx] = (float)row[x];
+		}
 	}
 }
 
-// Writes each tile's core block of the network output back to the grid.
+// Writes each tile's core block of the network output back to the grid, one warp
+// per row of a core and field.
 __global__ void scatter_tiles(const float* __restrict__ in, double* __restrict__ f, int Nx, int Ny, int T, int core,
                               int halo, int tiles_x, int first, int count) {
-	const long long per = 2LL * core * core;
-	const long long n = per * count;
-	for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-		const int j = (int)(t / per);
-		const int r = (int)(t - (long long)j * per);
-		const int u = r / (core * core), q = r - u * core * core;
-		const int cy = q / core, cx = q - cy * core;
-		const int tile = first + j;
+	const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+	for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < 2 * core * count; r += nw) {
+		const int cy = r % core, u = (r / core) & 1, j = r / (2 * core), tile = first + j;
 		const int by = tile / tiles_x, bx = tile - by * tiles_x;
-		const int x = bx * core + cx, y = by * core + cy;
-		if (x >= Nx || y >= Ny) continue;
-		f[((long long)u * Ny + y) * Nx + x] =
-		    (double)in[(long long)j * 2 * T * T + ((long long)u * T + halo + cy) * T + halo + cx];
+		const int y = by * core + cy, x0 = bx * core;
+		if (y >= Ny) continue;
+		const float* i = in + (((long long)j * 2 + u) * T + halo + cy) * T + halo;
+		double* row = f + ((long long)u * Ny + y) * Nx + x0;
+		for (int cx = lane; cx < core && x0 + cx < Nx; cx += 32) row[cx] = (double)i[cx];
 	}
 }
 
@@ -914,21 +1175,18 @@ struct pfcg_fno {
 	float* av = nullptr;
 	long long adam_t = 0;
 	float2* tw = nullptr;        // twiddles of the tile size
-	uint4* fdx = nullptr;        // mma fragments of the truncated x transforms (dft_frag_kernel)
-	uint4* fix = nullptr;
+	uint4* fe = nullptr;         // mma fragments of the truncated x transforms (dft_frag_kernel)
+	uint4* ff = nullptr;
 	uint4* fdy = nullptr;        // mma fragments of the truncated y transforms (dfty_frag_kernel)
 	uint4* fiy = nullptr;
 	float* sx = nullptr;         // per-kx weights of the truncated irfft2: (kx ? 2 : 1) / T^2
-	float* v[L + 1] = {};        // layer inputs (v[L] feeds the projection)
-	float* z[L] = {};            // pre-activations
-	float* s = nullptr;          // spectral branch output
+	float* v[L] = {};            // inputs of layers 1 .. L-1 (layer 0's is the lift of x)
+	float* z[L - 1] = {};        // pre-activations (the last layer has no activation)
 	float2* A = nullptr;         // [B][C][T][MX] x-transformed rows (and adjoint scratch)
 	float2* X[L] = {};           // [B][C][MY][MX] retained modes of each layer input
 	float2* Y = nullptr;         // [B][C][MY][MX] mixed modes
 	float2* Bq = nullptr;        // [B][C][T][MX] y-inverse rows (and adjoint scratch)
-	float* dv = nullptr;         // gradient scratch
-	float* dv2 = nullptr;
-	float* dz = nullptr;
+	float* dv = nullptr;         // gradient of a layer's output, pre-activation and input in turn
 	float* x = nullptr;          // [B][2][T][T] tile input (apply)
 	float* y = nullptr;          // [B][2][T][T] network output
 	float* dy = nullptr;
@@ -954,60 +1212,78 @@ int ffail(pfcg_fno* f, int code, const std::string& m) {
 		if (e_ != cudaSuccess) return ffail(f, PFCG_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
 	} while (0)
 
-// forward pass over a batch of B tiles; with train the pre-activations are kept for backward
-int forward(pfcg_fno* f, const float* x, int B, const float* target, bool train) {
-	const int T = f->T, npix = T * T;
-	const long long rows = (long long)B * C * T, planes = (long long)B * C;
+int grid_rows(long long nrows) { return grid_for(nrows * 32, 128); }
+
+// forward pass over a batch of B tiles; with a target also the loss, dy, the
+// pre-activations for backward and the projection's gradients (into f->g, cleared here)
+int forward(pfcg_fno* f, const float* x, int B, const float* target) {
+	const int T = f->T;
+	const long long rows = (long long)B * T, planes = (long long)B * C;
+	const int vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
 	cudaStream_t st = f->stream;
-	lift_fwd<<<grid_for((long long)B * npix, 256), 256, 0, st>>>(x, f->w, f->v[0], B, npix);
+	if (target) {
+		FCK(cudaMemsetAsync(f->g, 0, sizeof(float) * NPARAM, st));
+		FCK(cudaMemsetAsync(f->loss, 0, sizeof(double), st));
+	}
+	lift_dft<<<grid_for(rows * 4, 128), 128, 0, st>>>(x, vec, f->w, f->A, f->fe, rows, T);
 	f->launches++;
 	for (int l = 0; l < L; l++) {
-		dft_x<<<grid_for(rows * 2, 256), 256, 0, st>>>(f->v[l], f->A, f->fdx, nullptr, rows, T);
 		dft_y_fwd<<<grid_for(planes * 32 * DY_WARPS, 32 * DY_WARPS), 32 * DY_WARPS, 0, st>>>(f->A, f->X[l], f->fdy, planes, T);
 		mix<<<grid_for((long long)NK * ((B + 15) / 16) * 8 * 32, 128), 128, 0, st>>>(f->X[l], f->Y, f->w, l, B, 0);
 		dft_y_inv<<<grid_for(planes * 32 * DY_WARPS, 32 * DY_WARPS), 32 * DY_WARPS, 0, st>>>(f->Y, f->Bq, f->fiy, planes, T);
-		idft_x<<<grid_for(rows * 2, 256), 256, 0, st>>>(f->Bq, f->s, f->fix, f->sx, rows, T, 0);
-		pointwise_fwd<<<grid_for((long long)B * npix / 16 * 32, 128), 128, 0, st>>>(f->v[l], f->s, f->w, l, train ? f->z[l] : nullptr,
-		                                                                    f->v[l + 1], B, npix, l < L - 1);
-		f->launches += 6;
+#define PFCG_LAYER(FI, LA, TR)                                                                                        \
+	layer_fwd<FI, LA, TR><<<grid_rows(rows), 128, 0, st>>>(x, vec, f->v[l], f->Bq, f->w, l, f->fe, f->ff, f->sx,      \
+	                                                       l < L - 1 ? f->z[l] : nullptr, l < L - 1 ? f->v[l + 1] : nullptr, \
+	                                                       f->A, f->y, target, f->dy, f->loss, f->g, rows, T, B)
+		if (l == 0) {
+			if (target) PFCG_LAYER(true, false, true);
+			else PFCG_LAYER(true, false, false);
+		} else if (l < L - 1) {
+			if (target) PFCG_LAYER(false, false, true);
+			else PFCG_LAYER(false, false, false);
+		} else {
+			if (target) PFCG_LAYER(false, true, true);
+			else PFCG_LAYER(false, true, false);
+		}
+#undef PFCG_LAYER
+		f->launches += 4;
 	}
-	if (target) FCK(cudaMemsetAsync(f->loss, 0, sizeof(double), st));
-	proj_fwd_loss<<<grid_for((long long)B * npix, 256), 256, 0, st>>>(x, f->v[L], f->w, f->y, target, f->dy, f->loss, B,
-	                                                                 npix);
-	f->launches++;
 	FCK(cudaGetLastError());
 	return 0;
 }
 
+// gradients of every parameter after forward() with a target
 int backward(pfcg_fno* f, const float* x, int B) {
-	const int T = f->T, npix = T * T;
-	const long long rows = (long long)B * C * T, planes = (long long)B * C;
+	const int T = f->T;
+	const long long rows = (long long)B * T, planes = (long long)B * C;
+	const int vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
 	cudaStream_t st = f->stream;
-	const dim3 cg(std::min(grid_for((long long)B * npix, 256), 64), C);
-	const int wg = std::min(grid_for((long long)B * npix / 16 / (WG_THREADS / 32), 1), 148 * 4);
-	FCK(cudaMemsetAsync(f->g, 0, sizeof(float) * NPARAM, st));
-	// projection: dQ[j][c] = sum v_L[c] dy[j], dq[j] = sum dy[j], dv_L = Q^T dy
-	channel_grad<<<cg, 256, 0, st>>>(f->v[L], f->dy, f->g + OFF_Q, 1, C, nullptr, B, npix);
-	sum2_kernel<<<grid_for((long long)B * npix, 256), 256, 0, st>>>(f->dy, f->g + OFF_QB, B, npix);
-	proj_bwd<<<grid_for((long long)B * npix, 256), 256, 0, st>>>(f->dy, f->w, f->dv, B, npix);
-	f->launches += 3;
+	// about one row per warp in layer_grad: its tensor-core sums stay short (with 4.6
+	// rows each the gradient was 6.7e-6 from 64 bits instead of 2e-6)
+	const int gr = grid_rows(rows);
 	for (int l = L - 1; l >= 0; l--) {
-		pointwise_bwd<<<grid_for((long long)B * npix / 16 * 32, 128), 128, 0, st>>>(f->z[l], f->dv, f->w, l, f->dz, f->dv2, B, npix,
-		                                                                    l < L - 1);
-		weight_grad<<<wg, WG_THREADS, 0, st>>>(f->dz, f->v[l], f->g + off_W(l), f->g + off_b(l), B, npix);
+		float* gW = f->g + off_W(l);
+		float* gb = f->g + off_b(l);
+		const float* z = l < L - 1 ? f->z[l] : nullptr;
+		if (l == L - 1)
+			layer_grad<false, true><<<gr, 128, 0, st>>>(x, vec, f->v[l], z, f->dv, f->dy, f->w, f->fe, f->sx, f->Bq, gW, gb, rows, T);
+		else if (l > 0)
+			layer_grad<false, false><<<gr, 128, 0, st>>>(x, vec, f->v[l], z, f->dv, f->dy, f->w, f->fe, f->sx, f->Bq, gW, gb, rows, T);
+		else
+			layer_grad<true, false><<<gr, 128, 0, st>>>(x, vec, nullptr, z, f->dv, f->dy, f->w, f->fe, f->sx, f->Bq, gW, gb, rows, T);
 		// spectral branch, in reverse
-		dft_x<<<grid_for(rows * 2, 256), 256, 0, st>>>(f->dz, f->Bq, f->fdx, f->sx, rows, T);
 		dft_y_fwd<<<grid_for(planes * 32 * DY_WARPS, 32 * DY_WARPS), 32 * DY_WARPS, 0, st>>>(f->Bq, f->Y, f->fdy, planes, T);
 		mix_grad<<<grid_for((long long)C * C * NK, 256), 256, 0, st>>>(f->X[l], f->Y, f->g, l, B);
 		mix<<<grid_for((long long)NK * ((B + 15) / 16) * 8 * 32, 128), 128, 0, st>>>(f->Y, f->Bq, f->w, l, B, 1);
 		dft_y_inv<<<grid_for(planes * 32 * DY_WARPS, 32 * DY_WARPS), 32 * DY_WARPS, 0, st>>>(f->Bq, f->A, f->fiy, planes, T);
-		idft_x<<<grid_for(rows * 2, 256), 256, 0, st>>>(f->A, f->dv2, f->fix, nullptr, rows, T, 1);
-		f->launches += 8;
-		std::swap(f->dv, f->dv2);
+		if (l == L - 1)
+			layer_bwd<false, true><<<gr, 128, 0, st>>>(x, vec, f->dy, f->A, f->w, l, f->ff, f->dv, f->g, rows, T);
+		else if (l > 0)
+			layer_bwd<false, false><<<gr, 128, 0, st>>>(x, vec, f->dy, f->A, f->w, l, f->ff, f->dv, f->g, rows, T);
+		else
+			layer_bwd<true, false><<<gr, 128, 0, st>>>(x, vec, f->dy, f->A, f->w, l, f->ff, f->dv, f->g, rows, T);
+		f->launches += 6;
 	}
-	// lift: dP[c][j] = sum dv0[c] x[j], dp[c] = sum dv0[c]
-	channel_grad<<<cg, 256, 0, st>>>(f->dv, x, f->g + OFF_P, 2, 1, f->g + OFF_PB, B, npix);
-	f->launches++;
 	FCK(cudaGetLastError());
 	return 0;
 }
@@ -1025,12 +1301,12 @@ int fno_apply_device(pfcg_fno* f, const double* d_in, double* d_out, int Nx, int
 	FCK(cudaStreamWaitEvent(own, ev, 0));
 	for (int first = 0; first < ntiles; first += f->maxB) {
 		const int count = std::min(f->maxB, ntiles - first);
-		gather_tiles<<<grid_for(2LL * T * T * count, 256), 256, 0, own>>>(d_in, f->x, Nx, Ny, T, core, halo, tx, first,
+		gather_tiles<<<grid_for(2LL * T * count * 32, 256), 256, 0, own>>>(d_in, f->x, Nx, Ny, T, core, halo, tx, first,
 		                                                                  count);
 		f->launches++;
-		int rc = forward(f, f->x, count, nullptr, false);
+		int rc = forward(f, f->x, count, nullptr);
 		if (rc) return rc;
-		scatter_tiles<<<grid_for(2LL * core * core * count, 256), 256, 0, own>>>(f->y, d_out, Nx, Ny, T, core, halo, tx,
+		scatter_tiles<<<grid_for(2LL * core * count * 32, 256), 256, 0, own>>>(f->y, d_out, Nx, Ny, T, core, halo, tx,
 		                                                                         first, count);
 		f->launches++;
 	}
@@ -1087,21 +1363,18 @@ int pfcg_fno_create(int tile, int max_batch, pfcg_fno** out) {
 	add((void**)&f->am, sizeof(float) * NPARAM);
 	add((void**)&f->av, sizeof(float) * NPARAM);
 	add((void**)&f->tw, sizeof(float2) * tile);
-	add((void**)&f->fdx, sizeof(uint4) * (tile / 16) * 2 * 32);
-	add((void**)&f->fix, sizeof(uint4) * (tile / 8) * 32);
+	add((void**)&f->fe, sizeof(uint4) * (tile / PX) * 4 * 32);
+	add((void**)&f->ff, sizeof(uint4) * (tile / PX) * 4 * 32);
 	add((void**)&f->fdy, sizeof(uint4) * (tile / 8) * 32 * 2);
 	add((void**)&f->fiy, sizeof(uint4) * (tile / 16) * 2 * 32 * 2);
 	add((void**)&f->sx, sizeof(float) * MX);
-	for (int l = 0; l <= L; l++) add((void**)&f->v[l], sizeof(float) * nv);
-	for (int l = 0; l < L; l++) add((void**)&f->z[l], sizeof(float) * nv);
+	for (int l = 1; l < L; l++) add((void**)&f->v[l], sizeof(float) * nv);
+	for (int l = 0; l < L - 1; l++) add((void**)&f->z[l], sizeof(float) * nv);
 	for (int l = 0; l < L; l++) add((void**)&f->X[l], sizeof(float2) * max_batch * C * NK);
-	add((void**)&f->s, sizeof(float) * nv);
 	add((void**)&f->A, sizeof(float2) * max_batch * C * tile * MX);
 	add((void**)&f->Y, sizeof(float2) * max_batch * C * NK);
 	add((void**)&f->Bq, sizeof(float2) * max_batch * C * tile * MX);
 	add((void**)&f->dv, sizeof(float) * nv);
-	add((void**)&f->dv2, sizeof(float) * nv);
-	add((void**)&f->dz, sizeof(float) * nv);
 	add((void**)&f->x, sizeof(float) * max_batch * 2 * npix);
 	add((void**)&f->y, sizeof(float) * max_batch * 2 * npix);
 	add((void**)&f->dy, sizeof(float) * max_batch * 2 * npix);
@@ -1116,7 +1389,7 @@ int pfcg_fno_create(int tile, int max_batch, pfcg_fno** out) {
 	for (int m = 0; m < MX; m++) sc[m] = (m == 0 ? 1.f : 2.f) / (float)npix;
 	e = cudaMemcpyAsync(f->sx, sc, sizeof(sc), cudaMemcpyHostToDevice, f->stream);
 	twiddle_kernel<<<1, 256, 0, f->stream>>>(f->tw, tile);
-	dft_frag_kernel<<<(tile * 8 + 255) / 256, 256, 0, f->stream>>>(f->tw, tile, f->fdx, f->fix);
+	dft_frag_kernel<<<(tile * 8 + 255) / 256, 256, 0, f->stream>>>(f->tw, tile, f->fe, f->ff);
 	dfty_frag_kernel<<<(tile * 8 + 255) / 256, 256, 0, f->stream>>>(f->tw, tile, f->fdy, f->fiy);
 	f->launches += 2;
 	for (size_t i = 0; i < 5 && e == cudaSuccess; i++) e = cudaMemsetAsync(*bufs[i], 0, sizes[i], f->stream);
@@ -1133,14 +1406,12 @@ int pfcg_fno_create(int tile, int max_batch, pfcg_fno** out) {
 void pfcg_fno_destroy(pfcg_fno* f) {
 	if (!f) return;
 	if (f->stream) cudaStreamSynchronize(f->stream);
-	void* ptrs[] = {f->p,  f->w,  f->g,  f->am, f->av,   f->tw,        f->sx,   f->s,   f->A,   f->Y,   f->Bq, f->dv,
-	                f->dv2, f->dz, f->x, f->y,  f->dy,   f->loss,      f->field_tmp, f->part, f->fdx, f->fix, f->fdy, f->fiy};
+	void* ptrs[] = {f->p, f->w, f->g, f->am, f->av, f->tw, f->sx, f->A, f->Y, f->Bq, f->dv, f->x, f->y, f->dy, f->loss,
+	                f->field_tmp, f->part, f->fe, f->ff, f->fdy, f->fiy};
 	for (void* q : ptrs) cudaFree(q);
-	for (int l = 0; l <= L; l++) cudaFree(f->v[l]);
-	for (int l = 0; l < L; l++) {
-		cudaFree(f->z[l]);
-		cudaFree(f->X[l]);
-	}
+	for (float* q : f->v) cudaFree(q);
+	for (float* q : f->z) cudaFree(q);
+	for (float2* q : f->X) cudaFree(q);
 	if (f->stream) cudaStreamDestroy(f->stream);
 	delete f;
 }
@@ -1167,7 +1438,7 @@ int pfcg_fno_get_params(pfcg_fno* f, float* host_params) {
 int pfcg_fno_forward(pfcg_fno* f, const float* d_in, float* d_out, int batch) {
 	if (!f || !d_in || !d_out) return ffail(f, PFCG_EARG, "NULL argument");
 	if (batch < 1 || batch > f->maxB) return ffail(f, PFCG_EARG, "batch outside [1, max_batch]");
-	int rc = forward(f, d_in, batch, nullptr, false);
+	int rc = forward(f, d_in, batch, nullptr);
 	if (rc) return rc;
 	FCK(cudaMemcpyAsync(d_out, f->y, sizeof(float) * batch * 2 * f->T * f->T, cudaMemcpyDeviceToDevice, f->stream));
 	FCK(cudaStreamSynchronize(f->stream));
@@ -1178,7 +1449,7 @@ int pfcg_fno_loss_grad(pfcg_fno* f, const float* d_in, const float* d_target, in
                        float* host_grad) {
 	if (!f || !d_in || !d_target) return ffail(f, PFCG_EARG, "NULL argument");
 	if (batch < 1 || batch > f->maxB) return ffail(f, PFCG_EARG, "batch outside [1, max_batch]");
-	int rc = forward(f, d_in, batch, d_target, true);
+	int rc = forward(f, d_in, batch, d_target);
 	if (!rc) rc = backward(f, d_in, batch);
 	if (rc) return rc;
 	if (loss) FCK(cudaMemcpyAsync(loss, f->loss, sizeof(double), cudaMemcpyDeviceToHost, f->stream));

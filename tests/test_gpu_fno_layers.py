@@ -1,0 +1,96 @@
+"""The warm-start network's fused layer kernels (pfc_b200/csrc/fno.cu) where they
+can go wrong: the smallest and larger tiles, one tile, more tiles than a mixing
+block's sixteen rows, and input tensors that start off a 16-byte boundary, against
+the CPU oracle; and the GELU over its whole range through a network whose output
+is the GELU of its input.
+
+Tolerances as in test_gpu_fno: outputs to 1e-4 of the largest value, gradients to
+2e-3 in relative L2 norm per parameter block (FP32 sums with BF16 weights against
+float64)."""
+import numpy as np
+import pytest
+
+from oracle import fno_oracle as O
+from pfc_b200 import fno
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def _params(seed):
+    p = fno.init_params(seed, out_scale=1.0)
+    rng = np.random.default_rng(seed)
+    for k, (o, s) in fno.layout().items():
+        n = int(np.prod(s))
+        if k[:2] in ("Rr", "Ri"):
+            p[o:o + n] = rng.uniform(-1, 1, n) * 0.02
+        if k in ("p", "q") or k[0] == "b":
+            p[o:o + n] = rng.uniform(-0.1, 0.1, n)
+    return p
+
+
+def _off(a, shift):
+    """a on the device, starting `shift` floats after a 512-byte boundary."""
+    buf = torch.empty(a.size + shift, dtype=torch.float32, device="cuda")
+    v = buf[shift:].view(*a.shape)
+    v.copy_(torch.tensor(a))
+    return v
+
+
+@pytest.mark.parametrize("T,B,shift", [(32, 17, 0), (32, 1, 1), (128, 2, 3), (256, 1, 0)])
+def test_layers_match_oracle(T, B, shift):
+    rng = np.random.default_rng(T + B)
+    p = _params(T)
+    x = rng.normal(scale=0.5, size=(B, 2, T, T)).astype(np.float32)
+    t = (x + rng.normal(scale=0.1, size=x.shape)).astype(np.float32)
+    with fno.Network(T, B) as net:
+        net.set_params(p)
+        dx, dt = _off(x, shift), _off(t, shift)
+        dy, dy0 = torch.empty(x.shape, device="cuda"), torch.empty(x.shape, device="cuda")
+        torch.cuda.synchronize()
+        net.forward(_off(x, 0).data_ptr(), dy0.data_ptr(), B)
+        net.forward(dx.data_ptr(), dy.data_ptr(), B)
+        loss, g = net.loss_grad(dx.data_ptr(), dt.data_ptr(), B, want_grad=True)
+    assert torch.equal(dy, dy0)
+    loss_o, g_o, y_o = O.loss_and_grad(fno.bf16_round(p).astype(np.float64), x, t)
+    assert np.abs(dy.cpu().numpy() - y_o).max() < 1e-4 * np.abs(y_o).max()
+    assert abs(loss - loss_o) < 1e-4 * loss_o
+    for k, (o, s) in fno.layout().items():
+        n = int(np.prod(s))
+        err = np.linalg.norm(g[o:o + n] - g_o[o:o + n]) / max(np.linalg.norm(g_o[o:o + n]), 1e-30)
+        assert err < 2e-3, (k, err)
+
+
+def test_gelu_over_its_range():
+    """W0 = I on channel 0, the other layers pass it on far in GELU's linear range:
+    the output less the input is GELU(x0) to FP32 rounding of the added offset."""
+    T = 32
+    p = np.zeros(fno.NPARAM, dtype=np.float32)
+    lay = fno.layout()
+
+    def put(name, idx, v):
+        o, s = lay[name]
+        p[o + np.ravel_multi_index(idx, s)] = v
+
+    put("P", (0, 0), 1.0)
+    for l in range(fno.LAYERS):
+        put("W%d" % l, (0, 0), 1.0)
+    for l in (1, 2):
+        put("b%d" % l, (0,), 16.0)  # GELU(z + 16) = z + 16 to FP32
+    put("b3", (0,), -32.0)
+    put("Q", (1, 0), 1.0)
+    z = np.linspace(-12, 12, T * T, dtype=np.float32).reshape(T, T)
+    x = np.stack([z, np.zeros_like(z)])[None]
+    with fno.Network(T, 1) as net:
+        net.set_params(p)
+        dx = torch.tensor(x, device="cuda")
+        dy = torch.empty_like(dx)
+        torch.cuda.synchronize()
+        net.forward(dx.data_ptr(), dy.data_ptr(), 1)
+    got = dy.cpu().numpy()[0, 1].astype(np.float64)
+    want = torch.nn.functional.gelu(torch.tensor(z, dtype=torch.float64)).numpy()
+    # offsets of 16 and 32 on values up to 12: four roundings at 2^-19, and the products'
+    # BF16 splits, 2^-16 of the largest operand (44) each in four layers
+    assert np.abs(got - want).max() < 4 * 2.0 ** -19 + 4 * 44 * 2.0 ** -16
+    assert np.all(np.isfinite(got))
