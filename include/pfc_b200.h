@@ -330,10 +330,8 @@ void pfcg_fno_destroy(pfcg_fno* f);
  * stream: a cudaStream_t (NULL = the default stream); the call returns after it
  *   has synchronised with that stream.
  * Transforms run in FP32 (means and reductions in FP64), as PFCG_FP32, on the
- * runtime-plan step kernels only: the kernels specialised on a length need
- * per-pass twiddle tables that this call does not build, so at those lengths a
- * step costs more than through a handle (512^2 U=1: about 59 us against 24 us
- * on a B200).
+ * step kernels of run-time lengths only: the kernels specialised on a length need
+ * per-pass twiddle tables that this call does not build.
  * The workspace is a file-scope array of PFCG_NOALLOC_SCRATCH_BYTES (32 MiB)
  * that every GPU loading the library holds until exit; grids needing more,
  * about 2 * U * (Nx/2+1) * Ny * 8 bytes plus 32 * Ny bytes and a few KB, are

@@ -1767,6 +1767,15 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[PFCG_NOALLOC_SC
 
 size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
+// exp(-2 pi i k / n), k < n, the same way
+__global__ void noalloc_roots_kernel(float2* tw, int n) {
+	for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+		double sn, cs;
+		sincospi(-2.0 * (double)k / (double)n, &sn, &cs);
+		tw[k] = make_float2((float)cs, (float)sn);
+	}
+}
+
 // the plan's twiddles in FP32 from a double-precision sincospi
 __global__ void noalloc_twiddles_kernel(float2* tw, const FftPlan p) {
 	for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < p.ntw; k += gridDim.x * blockDim.x) {
@@ -1836,14 +1845,17 @@ extern "C" int pfcg_relax_noalloc(const pfcg_params* p, int Nx, int Ny, double d
 	set_dk(&h);
 	h.celem = sizeof(float2);
 	h.stream = (cudaStream_t)stream;
+	h.widetab = true; // three and four fields: their tables share the plans' memory, one after the other
 	int rc = 0;
 	if (!make_plan(Nx, false, &h.px) || !make_plan(Ny, false, &h.py))
 		rc = fail(&h, PFCG_ESIZE, "bad factorisation");
 	if (!rc) rc = choose_layout(&h);
 	if (rc) return fail(nullptr, rc, h.err);
 	// the runtime-plan STEP kernels (the specialised ones need per-pass tables)
-	h.geom.CC = h.ccr;
-	use_rt_steps(&h);
+	if (!is_wide(&h)) {
+		h.geom.CC = h.ccr;
+		use_rt_steps(&h);
+	}
 
 	unsigned char* base = (unsigned char*)scratch;
 	const size_t nspec = (size_t)h.H * Ny;
@@ -1860,13 +1872,13 @@ extern "C" int pfcg_relax_noalloc(const pfcg_params* p, int Nx, int Ny, double d
 	h.flag = (int*)carve(sizeof(int));
 	h.d_part = (double*)carve(sizeof(double) * MAXU * MEAN_BLOCKS);
 	h.nlpart = (double*)carve(sizeof(double) * MAXU * Ny);
-	h.twx = carve(sizeof(float2) * Nx);
-	h.twy = carve(sizeof(float2) * Ny);
+	h.twx = h.wtwx = carve(sizeof(float2) * Nx);
+	h.twy = h.wtwy = carve(sizeof(float2) * Ny);
 	h.d_real = fields; // the caller's buffer is both input and output
 
 	auto done = [&](int code) {
 		// the handle's pointers are views of the static workspace: nothing to free
-		h.spec = h.work = h.twx = h.twy = nullptr;
+		h.spec = h.work = h.twx = h.twy = h.wtwx = h.wtwy = nullptr;
 		h.mean = h.acc = h.d_part = h.nlpart = nullptr;
 		h.flag = nullptr;
 		h.d_real = nullptr;
@@ -1881,23 +1893,36 @@ extern "C" int pfcg_relax_noalloc(const pfcg_params* p, int Nx, int Ny, double d
 	// the workspace keeps the previous call's contents: clear what must start at zero
 	CKN(cudaMemsetAsync(h.acc, 0, sizeof(double) * ACC_N, h.stream));
 	CKN(cudaMemsetAsync(h.flag, 0, sizeof(int), h.stream));
-	noalloc_twiddles_kernel<<<(Nx + 255) / 256, 256, 0, h.stream>>>((float2*)h.twx, h.px);
-	CKN(cudaGetLastError());
-	noalloc_twiddles_kernel<<<(Ny + 255) / 256, 256, 0, h.stream>>>((float2*)h.twy, h.py);
+	const bool wide = is_wide(&h);
+	if (wide) {
+		noalloc_roots_kernel<<<(Nx + 255) / 256, 256, 0, h.stream>>>((float2*)h.wtwx, Nx);
+		CKN(cudaGetLastError());
+		noalloc_roots_kernel<<<(Ny + 255) / 256, 256, 0, h.stream>>>((float2*)h.wtwy, Ny);
+	} else {
+		noalloc_twiddles_kernel<<<(Nx + 255) / 256, 256, 0, h.stream>>>((float2*)h.twx, h.px);
+		CKN(cudaGetLastError());
+		noalloc_twiddles_kernel<<<(Ny + 255) / 256, 256, 0, h.stream>>>((float2*)h.twy, h.py);
+	}
 	CKN(cudaGetLastError());
 
 	// upload (means, r2c along x, FFT along y), steps, download
 	CKN(launch_field_means(fields, h.U, (long long)Nx * Ny, h.d_part, MEAN_BLOCKS, h.mean, h.stream));
 	XArgs<float> xa = xargs<float>(&h);
-	YArgs<float> ya = yargs<float>(&h);
-	if ((rc = run_xpass<float>(&h, XP_R2C, xa, h.cx))) return done(rc);
-	if ((rc = run_ypass<float>(&h, YP_INIT, ya, h.cy))) return done(rc);
+	YArgs<float> ya = yargs<float>(&h, true);
+	LaunchCfg cy = h.cys;
+	cy.grid--; // no k = 0 update
+	if ((rc = run_xpass<float>(&h, XP_R2C, xa, h.cxs))) return done(rc);
+	if ((rc = run_ypass<float>(&h, YP_INIT, ya, cy))) return done(rc);
 	xa.acc = h.acc + ACC_NL;
 	for (int s = 0; s < nsteps; s++) {
 		if ((rc = run_xpass<float>(&h, XP_STEP, xa, h.cxs))) return done(rc);
 		if ((rc = run_ypass<float>(&h, YP_STEP, ya, h.cys))) return done(rc);
 	}
 	xa.acc = h.acc;
+	if (wide) { // the last transform is the plan's
+		noalloc_twiddles_kernel<<<(Nx + 255) / 256, 256, 0, h.stream>>>((float2*)h.twx, h.px);
+		CKN(cudaGetLastError());
+	}
 	if ((rc = run_xpass<float>(&h, XP_C2R, xa, h.cx))) return done(rc);
 	int nan = 0;
 	CKN(cudaMemcpyAsync(&nan, h.flag, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
