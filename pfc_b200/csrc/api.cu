@@ -80,6 +80,8 @@ struct pfcg_handle {
 	void* wtwx = nullptr;
 	void* wtwy = nullptr;
 	int wsbx = 1, wsby = 1;
+	int early = 0, warm = 0; // choose_early
+	bool no_early = false;  // in a batch, whose launches are plain
 	int ccr = 1;            // columns per CTA of the run-time y-pass modes (geom.CC: the STEP kernel's)
 	double* d_real = nullptr;   // U*Ny*Nx doubles
 	double* d_fields = nullptr; // f(r) work fields
@@ -239,6 +241,29 @@ void use_rt_steps(pfcg_handle* h) {
 	h->cys.grid++;
 }
 
+// Grids that are on the chip at once beside the other pass's: each pass then starts
+// while the other still runs, and does before its wait what does not depend on it
+// (rt_xpass, rt_ypass). Needs the registers, shared memory and threads of both on
+// every SM; otherwise the early work would only lengthen a CTA that starts late, and
+// fewer threads per CTA to make room cost more than it gives (512^2 U=3 FP64: 38 us
+// per step instead of 29). 128^2 FP64: 14.0 us per step without, 11.9 with;
+// 256^2 U=2 FP64 18.8 and 16.1; 512^2 FP64 16.6 and 15.4. The x-pass's part pays
+// where an SM has one of its CTAs (128^2: 12.7 and 11.9; 360 x 500 FP32, two: 21.9
+// and 25.5).
+void choose_early(pfcg_handle* h) {
+	h->early = 0;
+	if (h->no_early) return;
+	const int regs = h->prec == PFCG_FP64 ? 128 : 64;
+	const int nx = (h->cxs.grid + h->nsm - 1) / h->nsm, ny = (h->cys.grid + h->nsm - 1) / h->nsm;
+	const int smy = h->cys.smem + rt_early_elems(h->U, h->geom.CC, h->Ny) * (int)h->celem / 2;
+	if (nx * (h->cxs.smem + 1024) + ny * (smy + 1024) > 227 * 1024 || nx + ny > 32) return;
+	const int tx = nx * h->cxs.block, ty = ny * h->cys.block;
+	if ((tx + ty) * regs > 65536 || tx + ty > 2048) return;
+	h->cys.smem = smy;
+	h->early = 1;
+	h->warm = nx == 1;
+}
+
 // launch shapes of the kernels of run-time lengths for row tile R and column group CC
 void set_generic_configs(pfcg_handle* h, int R, int CC) {
 	const int U = h->U;
@@ -251,6 +276,8 @@ void set_generic_configs(pfcg_handle* h, int R, int CC) {
 	h->cy = rt_config(h, h->py, U * h->ccr, groups, &h->sby);
 	h->cy1 = rt_config(h, h->py, h->ccr, groups, &h->sby1);
 	use_rt_steps(h);
+	h->early = 0;
+	if (!is_wide(h)) choose_early(h);
 	if (is_wide(h)) {
 		int nt;
 		const int P = (U * R + 1) / 2, S = U * CC;
@@ -266,13 +293,15 @@ void set_generic_configs(pfcg_handle* h, int R, int CC) {
 // long row leave one CTA per SM (4096^2 U=2: 827 us per step at R = 1, 887 at 2)
 // and short rows only lose latency by sharing a CTA. FP32: four rows, whose 32
 // bytes per column are a whole sector of the y-pass's gather (3000 x 2700 U=2:
-// 238 us at R = 4, 247 at 2, 259 at 1), two where four would leave SMs without a
-// tile (512^2 U=1: 15.4 us at both).
+// 246 us at R = 4, 254 at 2, 267 at 1; U=1 1000^2: 30.5 and 31.7), two where four
+// would leave SMs without a tile, or with one only of four sequences (U = 2:
+// 720^2 31.7 us at R = 4 and 28.8 at 2, 1440 x 900 52.1 and 46.3; 1600^2, 400
+// tiles, 75.6 and 78.8).
 int rt_rows(const pfcg_handle* h) {
 	const int least = h->U % 2 ? 2 : 1;
 	if (h->prec == PFCG_FP32)
 		for (int r : {4, 2})
-			if (r > least && x_tile_ok(h, r) && h->Ny / r >= h->nsm) return r;
+			if (r > least && x_tile_ok(h, r) && h->Ny / r >= h->nsm * (h->U * r > 4 ? 2 : 1)) return r;
 	return x_tile_ok(h, least) ? least : x_tile_ok(h, 1) ? 1 : 0;
 }
 
@@ -296,6 +325,10 @@ int choose_layout(pfcg_handle* h) {
 	if (!R) return fail(h, PFCG_ESIZE, "no x-pass tile fits shared memory for this Nx");
 	if (!y_group_ok(h, 1)) return fail(h, PFCG_ESIZE, "no y-pass column group fits shared memory for this Ny");
 	set_generic_configs(h, R, CC);
+	if (allow_spec && (xspec || (spec_cols(U, h->Ny) && spec_rows(U, h->Ny) == R))) {
+		h->early = 0;
+		use_rt_steps(h);
+	}
 	if (xspec) h->cxs = {h->Ny / R, spec_x_threads(U, h->Nx), spec_x_smem(U, h->Nx), 1};
 	if (allow_spec && spec_cols(U, h->Ny) && spec_rows(U, h->Ny) == R) {
 		CC = h->geom.CC = spec_cols(U, h->Ny);
@@ -489,6 +522,7 @@ template <typename T> XArgs<T> xargs(pfcg_handle* h) {
 	a.g = h->geom;
 	a.part = h->nlpart;
 	a.k = host_nl_k<T>(h->model);
+	a.warm = h->early && h->warm;
 	if (is_wide(h)) {
 		a.wtw = (const cplx<T>*)h->wtwx;
 		a.wplan = radix_plan(h->Nx);
@@ -513,6 +547,7 @@ template <typename T> YArgs<T> yargs(pfcg_handle* h, bool step = false) {
 	a.m = h->model;
 	a.g = h->geom;
 	if (!step) a.g.CC = h->ccr;
+	a.early = step ? h->early : 0;
 	if (is_wide(h)) {
 		a.wtw = (const cplx<T>*)h->wtwy;
 		a.wplan = radix_plan(h->Ny);
@@ -1647,10 +1682,8 @@ int pfcg_batch_create(int nprob, const pfcg_params* params, const int* Nx, const
 		// sizes with specialised kernels run them in their fixed shape; the
 		// others run the runtime-plan kernels, in the shape the autotuner picks
 		if (batch_ct(h)) continue;
-		if (h->cxs.spec || h->cys.spec) {
-			h->geom.CC = h->ccr;
-			use_rt_steps(h);
-		}
+		h->no_early = true;
+		set_generic_configs(h, h->geom.R, is_wide(h) ? h->geom.CC : h->ccr);
 		if (autotune) {
 			const int r2 = pfcg_autotune(h, 5);
 			if (r2) {
@@ -1852,10 +1885,7 @@ extern "C" int pfcg_relax_noalloc(const pfcg_params* p, int Nx, int Ny, double d
 	if (!rc) rc = choose_layout(&h);
 	if (rc) return fail(nullptr, rc, h.err);
 	// the runtime-plan STEP kernels (the specialised ones need per-pass tables)
-	if (!is_wide(&h)) {
-		h.geom.CC = h.ccr;
-		use_rt_steps(&h);
-	}
+	if (!is_wide(&h)) set_generic_configs(&h, h.geom.R, h.ccr);
 
 	unsigned char* base = (unsigned char*)scratch;
 	const size_t nspec = (size_t)h.H * Ny;

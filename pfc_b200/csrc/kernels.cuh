@@ -108,6 +108,7 @@ template <typename T> struct XArgs {
 	const cplx<T>* twct;    // per-pass twiddle table of the specialised kernels
 	FftPlan plan;
 	int sb;                 // channel pairs per FFT call
+	int warm;               // STEP, run-time lengths: a transform of nothing before the wait (rt_xpass)
 	NlK<T> k;               // STEP, run-time lengths: the nonlinear term's constants
 	const cplx<T>* wtw;     // FP32, U >= 3: n-entry twiddle table of kernels_wide.cuh (nullptr: kernels_rt.cuh)
 	RadixPlan wplan;
@@ -145,6 +146,7 @@ template <typename T> struct YArgs {
 	const cplx<T>* twct;    // per-pass twiddle table of the specialised kernels
 	FftPlan plan;
 	int sb;                 // sequences per FFT call
+	int early;              // STEP, run-time lengths: what does not depend on the x-pass before the wait (rt_ypass)
 	const cplx<T>* wtw;     // as in XArgs
 	RadixPlan wplan;
 	int wsb;
@@ -188,6 +190,9 @@ int spec_y_smem(int U, int N);
 int spec_twiddles(int N);
 // 1 if that y-pass reads its input columns straight from memory (TMA-capable)
 int spec_y_regio(int U, int N);
+
+// shared-memory elements (of T) that rt_ypass needs beyond its sequences with `early`
+int rt_early_elems(int U, int CC, int Ny);
 
 // Host-side launchers; return cudaGetLastError().
 template <typename T> cudaError_t launch_xpass(int mode, const XArgs<T>& a, const LaunchCfg& c, cudaStream_t s);

@@ -58,6 +58,12 @@ int spec_x_smem(int U, int N) {
 }
 int spec_y_smem(int U, int N) { return (U * spec_cols(U, N) * padded_len<float>(N) + spec_twiddles(N)) * 8; }
 
+// the spectral state of CC columns, and per pair of entries (one more per column
+// for ky = Ny / 2) two coefficients per field and one per pair of fields
+int rt_early_elems(int U, int CC, int Ny) {
+	return 2 + 2 * U * CC * Ny + (2 * U + U * (U - 1) / 2) * (CC * Ny / 2 + CC);
+}
+
 // ------------------------------------------------------ energy density --
 template <int U>
 __global__ void energy_density_kernel(const double* __restrict__ mf, const double* __restrict__ pn,

@@ -100,89 +100,98 @@ __device__ __forceinline__ void rt_xpass(const XArgs<T>& a, const int mode_, con
 	const bool byrow = U % 2 == 1 && R > 1;    // rows paired
 	T offT[U];
 	double off[U];
-#pragma unroll
-	for (int u = 0; u < U; u++) {
-		off[u] = a.off ? a.off[u] : 0.0;
-		offT[u] = (T)off[u];
-	}
-
-	if (mode == XP_R2C) {
-		// real rows less their mean, two to a sequence
-		if (byrow) {
-#pragma unroll
-			for (int u = 0; u < U; u++)
-				for (int e = tid; e < Nx * hq; e += nt) {
-					const int q = hq > 1 ? rt_div(e, a.plan.mn) : 0, x = e - q * Nx;
-					const double* r = a.real + ((long long)u * Ny + y0 + 2 * q) * Nx + x;
-					sm[(u * hq + q) * ld + rt_pad(x, sh)] = mk<T>((T)(r[0] - off[u]), (T)(r[Nx] - off[u]));
-				}
-		} else {
-			for (int e = tid; e < Nx * R; e += nt) {
-				const int r = R > 1 ? rt_div(e, a.plan.mn) : 0, x = e - r * Nx;
-				const double* v = a.real + ((long long)(y0 + r)) * Nx + x;
-#pragma unroll
-				for (int h = 0; h < F; h++) {
-					const double v0 = v[(long long)(2 * h) * Ny * Nx] - off[2 * h];
-					const double v1 = 2 * h + 1 < U ? v[(long long)(2 * h + 1) * Ny * Nx] - off[2 * h + 1 < U ? 2 * h + 1 : 0] : 0.0;
-					sm[(r * F + h) * ld + rt_pad(x, sh)] = mk<T>((T)v0, (T)v1);
-				}
-			}
-		}
-	} else {
-		// Hermitian-extended spectra of the pairs, C = A + iB on 0 .. Nx/2 and
-		// conj A + i conj B above, swapped; the imaginary parts of the kx = 0 and
-		// kx = Nx/2 entries are dropped like a c2r transform does
-		auto put = [&](cplx<T>* s, int k, cplx<T> A, cplx<T> B) {
-			if (k == 0 || 2 * k == Nx) { A.y = (T)0; B.y = (T)0; }
-			s[rt_pad(k, sh)] = mk<T>(A.y + B.x, A.x - B.y);
-			if (k > 0 && 2 * k < Nx) s[rt_pad(Nx - k, sh)] = mk<T>(B.x - A.y, A.x + B.y);
-		};
-		if (byrow) {
-#pragma unroll
-			for (int u = 0; u < U; u++) {
-				const cplx<T>* src = a.work + u * a.wstride + tofs;
-#pragma unroll 4
-				for (int e = tid; e < H << lq; e += nt) {
-					cplx<T> A, B;
-					ld2(src + 2 * e, A, B);
-					put(sm + (u * hq + (e & (hq - 1))) * ld, e >> lq, A, B);
-				}
-			}
-		} else if (U % 2 == 0 && R > 1) {
-#pragma unroll
-			for (int h = 0; h < F; h++) {
-				const cplx<T>* src = a.work + (2 * h) * a.wstride + tofs;
-#pragma unroll 4
-				for (int e = tid; e < H << lq; e += nt) {
-					cplx<T> A0, A1, B0, B1;
-					ld2(src + 2 * e, A0, A1);
-					ld2(src + a.wstride + 2 * e, B0, B1);
-					cplx<T>* s = sm + (2 * (e & (hq - 1)) * F + h) * ld;
-					put(s, e >> lq, A0, B0);
-					put(s + F * ld, e >> lq, A1, B1);
-				}
-			}
-		} else {
-#pragma unroll
-			for (int h = 0; h < F; h++) {
-				const cplx<T>* s0 = a.work + (2 * h) * a.wstride + tofs;
-				const cplx<T>* s1 = s0 + a.wstride;
-#pragma unroll 4
-				for (int k = tid; k < H; k += nt) put(sm + h * ld, k, s0[k], 2 * h + 1 < U ? s1[k] : mk<T>((T)0, (T)0));
-			}
-		}
-	}
-
-	// The first transform (the inverse one, or R2C's forward one), then the
-	// pointwise work, then the second one: one copy of the transform's code
 	constexpr int NACC = STEP ? U : 1 + U;
 	double acc[NACC];
 #pragma unroll
 	for (int i = 0; i < NACC; i++) acc[i] = 0.0;
 	bool nan = false;
+	// The first transform (the inverse one, or R2C's forward one), then the
+	// pointwise work, then the second one: one copy of the transform's code.
+	// With `warm` a turn before them transforms whatever shared memory holds, to
+	// fetch that code, the plan's constants and the twiddles while the previous
+	// kernel still runs (cold, the first transform of 512 points took 4700 cycles,
+	// the second 2900).
 #pragma unroll 1
-	for (int turn = 0; turn < 2; turn++) {
-		if (turn == 1) {
+	for (int turn = STEP && a.warm ? -1 : 0; turn < 2; turn++) {
+		if (turn == 0) {
+			// programmatic dependent launch (pdl_launch): the previous kernel's results
+			// are complete and visible after this wait; a plain launch returns at once
+			asm volatile("griddepcontrol.wait;" ::: "memory");
+			asm volatile("griddepcontrol.launch_dependents;");
+#pragma unroll
+			for (int u = 0; u < U; u++) {
+				off[u] = a.off ? a.off[u] : 0.0;
+				offT[u] = (T)off[u];
+			}
+
+			if (mode == XP_R2C) {
+				// real rows less their mean, two to a sequence
+				if (byrow) {
+#pragma unroll
+					for (int u = 0; u < U; u++)
+						for (int e = tid; e < Nx * hq; e += nt) {
+							const int q = hq > 1 ? rt_div(e, a.plan.mn) : 0, x = e - q * Nx;
+							const double* r = a.real + ((long long)u * Ny + y0 + 2 * q) * Nx + x;
+							sm[(u * hq + q) * ld + rt_pad(x, sh)] = mk<T>((T)(r[0] - off[u]), (T)(r[Nx] - off[u]));
+						}
+				} else {
+					for (int e = tid; e < Nx * R; e += nt) {
+						const int r = R > 1 ? rt_div(e, a.plan.mn) : 0, x = e - r * Nx;
+						const double* v = a.real + ((long long)(y0 + r)) * Nx + x;
+#pragma unroll
+						for (int h = 0; h < F; h++) {
+							const double v0 = v[(long long)(2 * h) * Ny * Nx] - off[2 * h];
+							const double v1 = 2 * h + 1 < U ? v[(long long)(2 * h + 1) * Ny * Nx] - off[2 * h + 1 < U ? 2 * h + 1 : 0] : 0.0;
+							sm[(r * F + h) * ld + rt_pad(x, sh)] = mk<T>((T)v0, (T)v1);
+						}
+					}
+				}
+			} else {
+				// Hermitian-extended spectra of the pairs, C = A + iB on 0 .. Nx/2 and
+				// conj A + i conj B above, swapped; the imaginary parts of the kx = 0 and
+				// kx = Nx/2 entries are dropped like a c2r transform does
+				auto put = [&](cplx<T>* s, int k, cplx<T> A, cplx<T> B) {
+					if (k == 0 || 2 * k == Nx) { A.y = (T)0; B.y = (T)0; }
+					s[rt_pad(k, sh)] = mk<T>(A.y + B.x, A.x - B.y);
+					if (k > 0 && 2 * k < Nx) s[rt_pad(Nx - k, sh)] = mk<T>(B.x - A.y, A.x + B.y);
+				};
+				if (byrow) {
+#pragma unroll
+					for (int u = 0; u < U; u++) {
+						const cplx<T>* src = a.work + u * a.wstride + tofs;
+#pragma unroll 4
+						for (int e = tid; e < H << lq; e += nt) {
+							cplx<T> A, B;
+							ld2(src + 2 * e, A, B);
+							put(sm + (u * hq + (e & (hq - 1))) * ld, e >> lq, A, B);
+						}
+					}
+				} else if (U % 2 == 0 && R > 1) {
+#pragma unroll
+					for (int h = 0; h < F; h++) {
+						const cplx<T>* src = a.work + (2 * h) * a.wstride + tofs;
+#pragma unroll 4
+						for (int e = tid; e < H << lq; e += nt) {
+							cplx<T> A0, A1, B0, B1;
+							ld2(src + 2 * e, A0, A1);
+							ld2(src + a.wstride + 2 * e, B0, B1);
+							cplx<T>* s = sm + (2 * (e & (hq - 1)) * F + h) * ld;
+							put(s, e >> lq, A0, B0);
+							put(s + F * ld, e >> lq, A1, B1);
+						}
+					}
+				} else {
+#pragma unroll
+					for (int h = 0; h < F; h++) {
+						const cplx<T>* s0 = a.work + (2 * h) * a.wstride + tofs;
+						const cplx<T>* s1 = s0 + a.wstride;
+#pragma unroll 4
+						for (int k = tid; k < H; k += nt) put(sm + h * ld, k, s0[k], 2 * h + 1 < U ? s1[k] : mk<T>((T)0, (T)0));
+					}
+				}
+			}
+
+		} else if (turn == 1) {
 			// the real fields: item (q, x) holds two rows of every field, or item (r, x) one
 			if (byrow) {
 				for (int e = tid; e < Nx * hq; e += nt) {
@@ -389,6 +398,8 @@ __device__ __forceinline__ void rt_ypass(const YArgs<T>& a, const int mode_, con
 	const int tid = threadIdx.x, nt = blockDim.x;
 	const int S = U * CC, kx0 = grp * CC;
 	if (STEP && kx0 >= H) { // the CTA of the k = 0 update
+		asm volatile("griddepcontrol.wait;" ::: "memory"); // as in rt_xpass
+		asm volatile("griddepcontrol.launch_dependents;");
 		ypass_mean_update<T, U>(a, tid, nt);
 		return;
 	}
@@ -397,44 +408,83 @@ __device__ __forceinline__ void rt_ypass(const YArgs<T>& a, const int mode_, con
 	const int lR = __ffs(R) - 1, lC = __ffs(CC) - 1;
 	const int nh = Ny / 2;
 
-	if (STEP) {
-		// this group's spectral state into L2 while the forward transform runs
-		const int lines = ncol * Ny * (int)sizeof(cplx<T>) / 128;
+	// With `early`, before the wait for the x-pass: the spectral state into shared
+	// memory (asynchronous copies), the update's coefficients, and a transform of
+	// nothing as in rt_xpass. The state is that of the y-pass before: the x-pass in
+	// between lets this kernel start only after its own wait for that y-pass.
+	cplx<T>* eN = sm + ((S * ld + 1) & ~1);                 // [u][c][ky], on 16 bytes
+	T* eK = reinterpret_cast<T*>(eN + S * Ny);              // [coefficient][pair]
+	const int nk = (nh << lC) + CC;
+	if (STEP && a.early) {
 #pragma unroll
 		for (int u = 0; u < U; u++) {
-			const char* p = reinterpret_cast<const char*>(a.spec + u * a.sstride + (long long)kx0 * Ny);
-			for (int i = tid; i < lines; i += nt) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i * 128));
+			const char* src = reinterpret_cast<const char*>(a.spec + u * a.sstride + (long long)kx0 * Ny);
+			const unsigned dst = (unsigned)__cvta_generic_to_shared(eN + u * CC * Ny);
+			for (int i = tid * 16; i < ncol * Ny * (int)sizeof(cplx<T>); i += nt * 16)
+				asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i), "l"(src + i) : "memory");
+		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
+		for (int e = tid; e < nk; e += nt) {
+			const bool second = e >= nh << lC; // ky = Ny / 2 of column e - CC nh
+			const int c = second ? e - (nh << lC) : CC > 1 ? rt_div(e, a.plan.mnh) : 0;
+			T A[U], Bn[U], cu[npairs<T, U>()];
+			entry_coef<T, U>(a.k, k2_step<T>(kx0 + c, second ? nh : e - c * nh, Ny, a.k.dkx, a.k.dky), A, Bn, cu);
+#pragma unroll
+			for (int u = 0; u < U; u++) {
+				eK[u * nk + e] = A[u];
+				eK[(U + u) * nk + e] = Bn[u];
+			}
+#pragma unroll
+			for (int p = 0; p < U * (U - 1) / 2; p++) eK[(2 * U + p) * nk + e] = cu[p];
 		}
 	}
-	if (mode != YP_WEIGHT) {
-		// CC columns of every row tile of `work`, two rows at a time where the tile has them
+
+#pragma unroll 1
+	for (int turn = STEP && a.early ? -1 : 0; turn < 2; turn++) {
+		if (turn == 0) {
+			asm volatile("griddepcontrol.wait;" ::: "memory"); // as in rt_xpass
+			asm volatile("griddepcontrol.launch_dependents;");
+			if (mode == YP_WEIGHT) continue;
+			if (STEP && !a.early) {
+				// this group's spectral state into L2 while the forward transform runs
+				const int lines = ncol * Ny * (int)sizeof(cplx<T>) / 128;
 #pragma unroll
-		for (int u = 0; u < U; u++) {
-			const cplx<T>* src = a.work + u * a.wstride + (long long)kx0 * R;
-			cplx<T>* dst = sm + u * CC * ld;
-			if (R > 1) {
-#pragma unroll 4
-				for (int i = tid; i < nh << lC; i += nt) {
-					const int e = 2 * i, r = e & (R - 1), c = (e >> lR) & (CC - 1), t = e >> (lR + lC);
-					cplx<T> v0 = mk<T>((T)0, (T)0), v1 = v0;
-					if (c < ncol) ld2(src + t * tileH + c * R + r, v0, v1);
-					cplx<T>* d = dst + c * ld + rt_pad(t * R + r, sh);
-					d[0] = v0;
-					d[1] = v1;
-				}
-			} else {
-#pragma unroll 4
-				for (int e = tid; e < Ny << lC; e += nt) {
-					const int c = e & (CC - 1), t = e >> lC;
-					dst[c * ld + rt_pad(t, sh)] = c < ncol ? src[t * tileH + c] : mk<T>((T)0, (T)0);
+				for (int u = 0; u < U; u++) {
+					const char* p = reinterpret_cast<const char*>(a.spec + u * a.sstride + (long long)kx0 * Ny);
+					for (int i = tid; i < lines; i += nt) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i * 128));
 				}
 			}
-		}
-	}
-#pragma unroll 1
-	for (int turn = mode == YP_WEIGHT ? 1 : 0; turn < 2; turn++) {
-		if (turn == 1) {
+			{
+				// CC columns of every row tile of `work`, two rows at a time where the tile has them
+#pragma unroll
+				for (int u = 0; u < U; u++) {
+					const cplx<T>* src = a.work + u * a.wstride + (long long)kx0 * R;
+					cplx<T>* dst = sm + u * CC * ld;
+					if (R > 1) {
+#pragma unroll 4
+						for (int i = tid; i < nh << lC; i += nt) {
+							const int e = 2 * i, r = e & (R - 1), c = (e >> lR) & (CC - 1), t = e >> (lR + lC);
+							cplx<T> v0 = mk<T>((T)0, (T)0), v1 = v0;
+							if (c < ncol) ld2(src + t * tileH + c * R + r, v0, v1);
+							cplx<T>* d = dst + c * ld + rt_pad(t * R + r, sh);
+							d[0] = v0;
+							d[1] = v1;
+						}
+					} else {
+#pragma unroll 4
+						for (int e = tid; e < Ny << lC; e += nt) {
+							const int c = e & (CC - 1), t = e >> lC;
+							dst[c * ld + rt_pad(t, sh)] = c < ncol ? src[t * tileH + c] : mk<T>((T)0, (T)0);
+						}
+					}
+				}
+			}
+		} else if (turn == 1) {
 			if (STEP) {
+				if (a.early) {
+					asm volatile("cp.async.wait_all;" ::: "memory");
+					__syncthreads();
+				}
 				// coupling and update of pfc-relax.c:1215-1244 for the entries ky = h and
 				// Ny - h (h = 0: 0 and Ny / 2, whose k^2 differ) of column c
 				const StepK<T>& K = a.k;
@@ -444,13 +494,32 @@ __device__ __forceinline__ void rt_ypass(const YArgs<T>& a, const int mode_, con
 					const int kx = kx0 + c, k2nd = h ? Ny - h : nh;
 					cplx<T>* sp = a.spec + (long long)kx * Ny;
 					cplx<T> N0[U], N1[U];
-#pragma unroll
-					for (int u = 0; u < U; u++) {
-						N0[u] = __ldcs(sp + u * a.sstride + h);
-						N1[u] = __ldcs(sp + u * a.sstride + k2nd);
-					}
 					T A[U], Bn[U], cu[npairs<T, U>()];
-					entry_coef<T, U>(K, k2_step<T>(kx, h, Ny, K.dkx, K.dky), A, Bn, cu);
+					auto stored = [&](int at) {
+#pragma unroll
+						for (int u = 0; u < U; u++) {
+							A[u] = eK[u * nk + at];
+							Bn[u] = eK[(U + u) * nk + at];
+						}
+#pragma unroll
+						for (int p = 0; p < U * (U - 1) / 2; p++) cu[p] = eK[(2 * U + p) * nk + at];
+					};
+					if (a.early) {
+						const cplx<T>* s = eN + c * Ny;
+#pragma unroll
+						for (int u = 0; u < U; u++) {
+							N0[u] = s[u * CC * Ny + h];
+							N1[u] = s[u * CC * Ny + k2nd];
+						}
+						stored(e);
+					} else {
+#pragma unroll
+						for (int u = 0; u < U; u++) {
+							N0[u] = __ldcs(sp + u * a.sstride + h);
+							N1[u] = __ldcs(sp + u * a.sstride + k2nd);
+						}
+						entry_coef<T, U>(K, k2_step<T>(kx, h, Ny, K.dkx, K.dky), A, Bn, cu);
+					}
 					auto apply = [&](int ky, const cplx<T>(&N)[U]) {
 						cplx<T> M[U];
 						cplx<T>* s = sm + c * ld + rt_pad(ky, sh);
@@ -475,7 +544,10 @@ __device__ __forceinline__ void rt_ypass(const YArgs<T>& a, const int mode_, con
 						}
 					};
 					apply(h, N0);
-					if (h == 0) entry_coef<T, U>(K, k2_step<T>(kx, nh, Ny, K.dkx, K.dky), A, Bn, cu);
+					if (h == 0) {
+						if (a.early) stored((nh << lC) + c);
+						else entry_coef<T, U>(K, k2_step<T>(kx, nh, Ny, K.dkx, K.dky), A, Bn, cu);
+					}
 					apply(k2nd, N1);
 				}
 			} else {
@@ -517,7 +589,7 @@ __device__ __forceinline__ void rt_ypass(const YArgs<T>& a, const int mode_, con
 		}
 		__syncthreads();
 		rt_fft<T>(sm, a.plan, S, a.sb, a.tw, tid, nt);
-	}
+		}
 #pragma unroll
 	for (int u = 0; u < U; u++) {
 		cplx<T>* dst = a.work + u * a.wstride + (long long)kx0 * R;
@@ -546,17 +618,11 @@ template <typename T> constexpr int RT_MINB = sizeof(T) == 4 ? 2 : 1;
 
 template <typename T, int U, bool STEP> __global__ void __launch_bounds__(MAXNT, RT_MINB<T>) xrt_kernel(const XArgs<T> a, int mode) {
 	rt_warm_twiddles<T>(a.tw, a.plan.ntw, threadIdx.x, blockDim.x);
-	// programmatic dependent launch (pdl_launch): the previous kernel's results
-	// are complete and visible after this wait; a plain launch returns at once
-	asm volatile("griddepcontrol.wait;" ::: "memory");
-	asm volatile("griddepcontrol.launch_dependents;");
 	rt_xpass<T, U, STEP>(a, mode, blockIdx.x);
 }
 
 template <typename T, int U, bool STEP> __global__ void __launch_bounds__(MAXNT, RT_MINB<T>) yrt_kernel(const YArgs<T> a, int mode) {
 	rt_warm_twiddles<T>(a.tw, a.plan.ntw, threadIdx.x, blockDim.x);
-	asm volatile("griddepcontrol.wait;" ::: "memory");
-	asm volatile("griddepcontrol.launch_dependents;");
 	rt_ypass<T, U, STEP>(a, mode, blockIdx.x);
 }
 

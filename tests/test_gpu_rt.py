@@ -67,3 +67,12 @@ def test_run_time_lengths_match_oracle(U, Nx, Ny, monkeypatch):
         assert np.abs(ng - no).max() < 1e-12
         # f(r) is a polynomial of degree four in fields of order one with coefficients below 3
         assert np.abs(frg - fr).max() < 20 * tol, (prec, np.abs(frg - fr).max())
+
+
+@pytest.mark.parametrize("U,Nx,Ny", [(1, 128, 128), (2, 256, 150), (1, 300, 640), (1, 360, 500), (2, 64, 256), (3, 90, 294),
+                                     (4, 60, 150)])
+def test_work_before_the_wait_matches_oracle(U, Nx, Ny, monkeypatch):
+    """A small problem by itself takes its state and coefficients, and turns a
+    transform, before the wait for the previous pass: one CTA of a pass per SM, one
+    CTA more than SMs, two, and grids just too large for it. Bounds as above."""
+    test_run_time_lengths_match_oracle(U, Nx, Ny, monkeypatch)
