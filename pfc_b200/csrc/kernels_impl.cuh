@@ -123,6 +123,18 @@ __device__ __forceinline__ float phi1f(float x, float A) {
 	return (A - 1.f) / x;
 }
 
+// CTAs of NT threads per SM that the kernels of length N leave registers for. A
+// single problem's: as many as put its grid of `ctas` on the chip at once, up to
+// 1024 threads (64 registers each; radix 3 and 6 spill there and stop at 640), and
+// no more, since a lone CTA is faster with more registers (768^2 18.0 us per step,
+// 21.8 with 1024 threads for every size; 1024^2 U=2 24.4 and 25.9). A batch's: 1024
+// threads, for the most CTAs in flight (24 problems of 256^2 .. 1536^2: 8.4 ms, 10.6
+// with 512).
+__host__ __device__ constexpr int minb(int N, int NT, int ctas) {
+	const int want = (ctas + 147) / 148, most = (N % 3 == 0 ? 640 : 1024) / NT;
+	return want > most ? (most < 2 ? 2 : most) : want < 2 ? 2 : want;
+}
+
 // Launch shapes of the kernels specialised on a compile-time length NC (NC = 0:
 // runtime length and plan). P / S resident sequences, NSUB per FFT call, NT threads.
 template <typename T, int U, int NC, int RC> struct XCfg {
@@ -132,7 +144,8 @@ template <typename T, int U, int NC, int RC> struct XCfg {
 	static constexpr int LD = NC + (NC >> Pad<T>::SHIFT) + 1;
 	static constexpr int NSUB = CT ? (P * NC / MAXE <= MAXNT ? P : MAXNT * MAXE / NC) : 1;
 	static constexpr int NT = CT ? NSUB * NC / MAXE : MAXNT;
-	static constexpr int MINB = (CT && sizeof(T) == 4) ? 2 : 1;
+	static constexpr int MINB = minb(NC, NT, NC / RC);
+	static constexpr int MINB_BATCH = 1024 / NT;
 	static constexpr int TWN = CT ? CtPlan<NC, MAXE>::TWN : 0;
 };
 
@@ -146,7 +159,8 @@ template <typename T, int U, int NC, int CCC, int RC, bool FUSEDK = true> struct
 	static constexpr int NSUB = CT ? (FUSED ? S : (S * NC / MAXE <= MAXNT ? S : MAXNT * MAXE / NC)) : 1;
 	// fused: thread t holds butterfly t mod N/MAXE of column t / (N/MAXE) for every field
 	static constexpr int NT = CT ? (FUSED ? U * CCC * NC / MAXE : NSUB * NC / MAXE) : MAXNT;
-	static constexpr int MINB = (CT && sizeof(T) == 4) ? 2 : 1;
+	static constexpr int MINB = minb(NC, NT, (NC / 2 + CCC) / CCC + 1);
+	static constexpr int MINB_BATCH = 1024 / NT;
 	static constexpr int TWN = CT ? CtPlan<NC, MAXE>::TWN : 0;
 };
 
@@ -343,14 +357,16 @@ __device__ __forceinline__ void xpass_step_fused(const XArgs<T>& a, cplx<T>* sm,
 		const int k = tid + it * NT;
 		if (k >= H) break;
 		cplx<T> y[CH];
-		if constexpr (sizeof(T) == 4 && RC == 2) {
-			// both rows of a field at k are one 16-byte word
+		if constexpr (sizeof(T) == 4 && RC % 2 == 0) {
+			// two rows of a field at k are one 16-byte word
 #pragma unroll
-			for (int u = 0; u < U; u++) {
-				const float4 q = *reinterpret_cast<const float4*>(a.work + u * a.wstride + tofs + (long long)k * RC);
-				y[u] = mk<T>(q.x, q.y);
-				y[U + u] = mk<T>(q.z, q.w);
-			}
+			for (int u = 0; u < U; u++)
+#pragma unroll
+				for (int r = 0; r < RC; r += 2) {
+					const float4 q = *reinterpret_cast<const float4*>(a.work + u * a.wstride + tofs + (long long)k * RC + r);
+					y[r * U + u] = mk<T>(q.x, q.y);
+					y[(r + 1) * U + u] = mk<T>(q.z, q.w);
+				}
 		} else {
 #pragma unroll
 			for (int c = 0; c < CH; c++) y[c] = a.work[(c % U) * a.wstride + tofs + (long long)k * RC + c / U];
@@ -428,11 +444,14 @@ __device__ __forceinline__ void xpass_step_fused(const XArgs<T>& a, cplx<T>* sm,
 			zz[2 * p] = mk<T>(half * (Ck.x + Cm.x), half * (Ck.y - Cm.y));
 			zz[2 * p + 1] = mk<T>(half * (Ck.y + Cm.y), half * (Cm.x - Ck.x));
 		}
-		if constexpr (sizeof(T) == 4 && RC == 2) {
+		if constexpr (sizeof(T) == 4 && RC % 2 == 0) {
 #pragma unroll
 			for (int u = 0; u < U; u++)
-				*reinterpret_cast<float4*>(a.work + u * a.wstride + tofs + (long long)k * RC) =
-				    make_float4(zz[u].x, zz[u].y, zz[U + u].x, zz[U + u].y);
+#pragma unroll
+				for (int r = 0; r < RC; r += 2) {
+					const cplx<T> p = zz[r * U + u], q = zz[(r + 1) * U + u];
+					*reinterpret_cast<float4*>(a.work + u * a.wstride + tofs + (long long)k * RC + r) = make_float4(p.x, p.y, q.x, q.y);
+				}
 		} else {
 #pragma unroll
 			for (int c = 0; c < CH; c++) a.work[(c % U) * a.wstride + tofs + (long long)k * RC + c / U] = zz[c];
@@ -964,14 +983,14 @@ __global__ void __launch_bounds__(YCfg<T, U, NC, CCC, RC, FUSEDK>::NT, YCfg<T, U
 // the launch belongs to a problem of that length and field count (one launch
 // per such class of a batch), so the body is the single-problem one.
 template <typename T, int U, int NC, int RC>
-__global__ void __launch_bounds__(XCfg<T, U, NC, RC>::NT, XCfg<T, U, NC, RC>::MINB)
+__global__ void __launch_bounds__(XCfg<T, U, NC, RC>::NT, XCfg<T, U, NC, RC>::MINB_BATCH)
     xpass_ct_batch_kernel(const XArgs<T>* __restrict__ probs, const int* __restrict__ blk_prob,
                           const int* __restrict__ blk_local) {
 	xpass_body<T, U, NC, RC>(probs[blk_prob[blockIdx.x]], blk_local[blockIdx.x]);
 }
 
 template <typename T, int U, int NC, int CCC, int RC, bool FUSEDK>
-__global__ void __launch_bounds__(YCfg<T, U, NC, CCC, RC, FUSEDK>::NT, YCfg<T, U, NC, CCC, RC, FUSEDK>::MINB)
+__global__ void __launch_bounds__(YCfg<T, U, NC, CCC, RC, FUSEDK>::NT, YCfg<T, U, NC, CCC, RC, FUSEDK>::MINB_BATCH)
     ypass_ct_batch_kernel(const YArgs<T>* __restrict__ probs, const int* __restrict__ blk_prob,
                           const int* __restrict__ blk_local) {
 	ypass_body<T, U, NC, CCC, RC, FUSEDK>(probs[blk_prob[blockIdx.x]], blk_local[blockIdx.x]);
@@ -1045,21 +1064,25 @@ static cudaError_t ylaunch(const YArgs<T>& a, const LaunchCfg& c, cudaStream_t s
 
 template <typename T> struct Spec;
 // Rows per x-pass tile (xr) and columns per y-pass group (ycc) of the kernels
-// specialised on a compile-time length N, 0 where there is none. The row tile
-// is also the layout of `work` for the runtime-plan modes (evaluate, c2r, r2c),
-// so U * xr stays within MAX_CH: an FP32 x-pass CTA runs U * xr * N / (2 M)
-// threads for the main radix M = ct_maxe (512 at N = 4096 and 2048, N / 4
-// below with M = 16, 192 at N = 384). A y-pass CTA runs U * ycc * N / M
-// threads: 512, or 384 at N = 384, 768 and 1536 (8^2 * 6, 16^2 * 3, 16^2 * 6).
+// specialised on a compile-time length N, 0 where there is none. The row tile is
+// also the layout of `work` for the run-time-length modes (evaluate, c2r, r2c). A
+// CTA runs a thread per M = ct_maxe points of its sequences, so few sequences make
+// small CTAs: more of them per grid, and barriers that fewer warps wait at.
+// 512 threads everywhere left 512^2 17 y-pass CTAs and 1024^2 65 for 148 SMs. us per
+// step with (rows, columns) of 512-thread CTAs and with these: 256^2 U=1 16.4
+// (8, 32) and 11.6; 512^2 19.2 (8, 16) and 13.6, U=2 28.3 (4, 8) and 15.4;
+// 768^2 22.0 (8, 8) and 18.0, U=2 33.4 (4, 4) and 23.5; 1024^2 34.4 (8, 8) and 18.4,
+// U=2 36.7 (4, 4) and 24.4; 2048^2 52.1 (8, 4) and 41.3, U=2 92.6 (4, 2) and 77.2;
+// 4096^2 157.9 (4, 2) and 140. Fewer still lose: 1024^2 U=2 one row, one column
+// 39.6; 4096^2 U=2 one row (8 bytes per column and tile) 409, two rows 282.
 template <> struct Spec<float> {
-	static constexpr int x1(int N) {
-		return N == 4096 ? 4 : (N == 2048 || N == 1536 || N == 1024 || N == 768 || N == 512 || N == 384 || N == 256) ? 8 : 0;
+	static constexpr bool has(int U, int N) {
+		return (U == 1 || U == 2) && (N == 4096 || N == 2048 || N == 1536 || N == 1024 || N == 768 || N == 512 || N == 384 || N == 256);
 	}
-	static constexpr int y1(int N) {
-		return N == 4096 ? 2 : N == 2048 || N == 1536 ? 4 : N == 1024 || N == 768 || N == 384 ? 8 : N == 512 ? 16 : N == 256 ? 32 : 0;
+	static constexpr int xr(int U, int N) { return !has(U, N) ? 0 : N == 4096 ? 2 : (N == 512 || N == 256 ? 8 : 4) / U; }
+	static constexpr int ycc(int U, int N) {
+		return !has(U, N) ? 0 : N == 1024 || N == 768 ? 2 : (N == 4096 ? 2 : N == 256 ? 8 : 4) / U;
 	}
-	static constexpr int xr(int U, int N) { return U == 1 ? x1(N) : U == 2 ? x1(N) / 2 : 0; }
-	static constexpr int ycc(int U, int N) { return U == 1 ? y1(N) : U == 2 ? y1(N) / 2 : 0; }
 };
 template <typename T, int U> static bool x_is_spec(const XArgs<T>& a) {
 	return Spec<T>::xr(U, a.g.Nx) > 0 && a.g.R == Spec<T>::xr(U, a.g.Nx);
