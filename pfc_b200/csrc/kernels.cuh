@@ -10,7 +10,9 @@
 //   work[u]  the mixed (kx, y) representation between the two passes, complex,
 //            tiled by R rows: element (kx, y) at ((y/R)*H + kx)*R + y%R, so one
 //            row tile is contiguous for the x-pass and CC adjacent columns of
-//            one tile are contiguous for the y-pass.
+//            one tile are contiguous for the y-pass. In FP64 with an even number of
+//            fields (WORK_IL) the fields of a (row tile, kx) are adjacent instead of
+//            U arrays: element (u, kx, y) at (((y/R)*H + kx)*U + u)*R + y%R.
 //
 // One time step is two kernels:
 //   x-pass (one CTA per R-row tile, all U fields): c2r along x of work,
@@ -31,6 +33,14 @@
 namespace pfcg {
 
 constexpr int MAXU = 4;
+
+// FP64 tiles of even U hold one row, 16 bytes of a field per (tile, kx): half a
+// sector, of which the y-pass of one column used no more. Two fields side by side
+// fill it (4096^2 U=2: y-pass 552 -> 505 us, step 837 -> 806; 1000^2 61.5 -> 55.3).
+// Odd U has two rows, a sector, already. FP32 keeps arrays: its specialised x-pass
+// reads 16-byte words of adjacent kx, and lost more at 32 bytes apart than the
+// y-pass gained (4096^2 U=2 119 + 172 -> 129 + 168 us).
+template <typename T, int U> constexpr bool WORK_IL = sizeof(T) == 8 && U % 2 == 0;
 constexpr int MAXW = 4;
 constexpr int MAX_CH = 8;     // real rows (channels) per x-pass CTA; odd counts pad with a zero channel
 constexpr int MAX_TRIAL = 5;  // box sizes per Parseval reduction
@@ -98,7 +108,7 @@ struct RadixPlan {
 };
 
 template <typename T> struct XArgs {
-	cplx<T>* work;          // U arrays at stride wstride
+	cplx<T>* work;          // U arrays at stride wstride (WORK_IL: one)
 	long long wstride;
 	const double* off;      // per-field value added after c2r / subtracted before r2c (the mean)
 	double* real;           // XP_C2R output / XP_R2C input: U fields of Ny*Nx doubles

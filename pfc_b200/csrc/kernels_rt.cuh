@@ -95,7 +95,8 @@ __device__ __forceinline__ void rt_xpass(const XArgs<T>& a, const int mode_, con
 	const int P = (U * R + 1) >> 1;
 	const int hq = R >> 1, lq = R > 1 ? __ffs(hq) - 1 : 0; // row pairs of a tile
 	const int y0 = tile * R;
-	const long long tofs = (long long)tile * H * R;
+	constexpr bool IL = WORK_IL<T, U>;
+	const long long tofs = (long long)tile * H * (IL ? U * R : R), us = IL ? R : a.wstride;
 	constexpr int F = (U + 1) / 2;             // sequences per row when fields are paired
 	const bool byrow = U % 2 == 1 && R > 1;    // rows paired
 	T offT[U];
@@ -169,12 +170,13 @@ __device__ __forceinline__ void rt_xpass(const XArgs<T>& a, const int mode_, con
 				} else if (U % 2 == 0 && R > 1) {
 #pragma unroll
 					for (int h = 0; h < F; h++) {
-						const cplx<T>* src = a.work + (2 * h) * a.wstride + tofs;
+						const cplx<T>* src = a.work + (2 * h) * us + tofs;
 #pragma unroll 4
 						for (int e = tid; e < H << lq; e += nt) {
+							const int at = 2 * (IL ? e + (e >> lq) * (U - 1) * hq : e);
 							cplx<T> A0, A1, B0, B1;
-							ld2(src + 2 * e, A0, A1);
-							ld2(src + a.wstride + 2 * e, B0, B1);
+							ld2(src + at, A0, A1);
+							ld2(src + us + at, B0, B1);
 							cplx<T>* s = sm + (2 * (e & (hq - 1)) * F + h) * ld;
 							put(s, e >> lq, A0, B0);
 							put(s + F * ld, e >> lq, A1, B1);
@@ -183,10 +185,11 @@ __device__ __forceinline__ void rt_xpass(const XArgs<T>& a, const int mode_, con
 				} else {
 #pragma unroll
 					for (int h = 0; h < F; h++) {
-						const cplx<T>* s0 = a.work + (2 * h) * a.wstride + tofs;
-						const cplx<T>* s1 = s0 + a.wstride;
+						const cplx<T>* s0 = a.work + (2 * h) * us + tofs;
+						const cplx<T>* s1 = s0 + us;
+						constexpr int ks = IL ? U : 1;
 #pragma unroll 4
-						for (int k = tid; k < H; k += nt) put(sm + h * ld, k, s0[k], 2 * h + 1 < U ? s1[k] : mk<T>((T)0, (T)0));
+						for (int k = tid; k < H; k += nt) put(sm + h * ld, k, s0[k * ks], 2 * h + 1 < U ? s1[k * ks] : mk<T>((T)0, (T)0));
 					}
 				}
 			}
@@ -301,25 +304,27 @@ __device__ __forceinline__ void rt_xpass(const XArgs<T>& a, const int mode_, con
 		} else if (U % 2 == 0 && R > 1) {
 #pragma unroll
 			for (int h = 0; h < F; h++) {
-				cplx<T>* dst = a.work + (2 * h) * a.wstride + tofs;
+				cplx<T>* dst = a.work + (2 * h) * us + tofs;
 				for (int e = tid; e < H << lq; e += nt) {
+					const int at = 2 * (IL ? e + (e >> lq) * (U - 1) * hq : e);
 					cplx<T> a0, a1, b0, b1;
 					const cplx<T>* s = sm + (2 * (e & (hq - 1)) * F + h) * ld;
 					split(s, e >> lq, a0, b0);
 					split(s + F * ld, e >> lq, a1, b1);
-					st2(dst + 2 * e, a0, a1);
-					st2(dst + a.wstride + 2 * e, b0, b1);
+					st2(dst + at, a0, a1);
+					st2(dst + us + at, b0, b1);
 				}
 			}
 		} else {
 #pragma unroll
 			for (int h = 0; h < F; h++) {
-				cplx<T>* d0 = a.work + (2 * h) * a.wstride + tofs;
+				cplx<T>* d0 = a.work + (2 * h) * us + tofs;
+				constexpr int ks = IL ? U : 1;
 				for (int k = tid; k < H; k += nt) {
 					cplx<T> za, zb;
 					split(sm + h * ld, k, za, zb);
-					d0[k] = za;
-					if (2 * h + 1 < U) d0[a.wstride + k] = zb;
+					d0[k * ks] = za;
+					if (2 * h + 1 < U) d0[us + k * ks] = zb;
 				}
 			}
 		}
@@ -404,7 +409,7 @@ __device__ __forceinline__ void rt_ypass(const YArgs<T>& a, const int mode_, con
 		return;
 	}
 	const int ncol = min(CC, H - kx0);
-	const long long tileH = (long long)H * R;
+	const long long tileH = (long long)H * (WORK_IL<T, U> ? U * R : R);
 	const int lR = __ffs(R) - 1, lC = __ffs(CC) - 1;
 	const int nh = Ny / 2;
 
@@ -454,8 +459,27 @@ __device__ __forceinline__ void rt_ypass(const YArgs<T>& a, const int mode_, con
 					for (int i = tid; i < lines; i += nt) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i * 128));
 				}
 			}
-			{
-				// CC columns of every row tile of `work`, two rows at a time where the tile has them
+			// CC columns of every row tile of `work`, two rows at a time where the tile has them
+			if constexpr (WORK_IL<T, U>) {
+				const cplx<T>* src = a.work + kx0 * U * R;
+				if (R > 1) {
+#pragma unroll 4
+					for (int e = tid; e < nh * U << lC; e += nt) {
+						const int r = 2 * e & (R - 1), i = e >> (lR - 1), u = i % U, c = i / U & (CC - 1), t = i / U >> lC;
+						cplx<T> v0 = mk<T>((T)0, (T)0), v1 = v0;
+						if (c < ncol) ld2(src + t * tileH + (c * U + u) * R + r, v0, v1);
+						cplx<T>* d = sm + (u * CC + c) * ld + rt_pad(t * R + r, sh);
+						d[0] = v0;
+						d[1] = v1;
+					}
+				} else {
+#pragma unroll 4
+					for (int e = tid; e < Ny * U << lC; e += nt) {
+						const int u = e % U, c = e / U & (CC - 1), t = e / U >> lC;
+						sm[(u * CC + c) * ld + rt_pad(t, sh)] = c < ncol ? src[t * tileH + c * U + u] : mk<T>((T)0, (T)0);
+					}
+				}
+			} else {
 #pragma unroll
 				for (int u = 0; u < U; u++) {
 					const cplx<T>* src = a.work + u * a.wstride + (long long)kx0 * R;
@@ -590,21 +614,38 @@ __device__ __forceinline__ void rt_ypass(const YArgs<T>& a, const int mode_, con
 		__syncthreads();
 		rt_fft<T>(sm, a.plan, S, a.sb, a.tw, tid, nt);
 		}
-#pragma unroll
-	for (int u = 0; u < U; u++) {
-		cplx<T>* dst = a.work + u * a.wstride + (long long)kx0 * R;
-		const cplx<T>* src = sm + u * CC * ld;
+	if constexpr (WORK_IL<T, U>) {
+		cplx<T>* dst = a.work + kx0 * U * R;
 		if (R > 1) {
-			for (int i = tid; i < nh << lC; i += nt) {
-				const int e = 2 * i, r = e & (R - 1), c = (e >> lR) & (CC - 1), t = e >> (lR + lC);
-				const cplx<T>* s = src + c * ld + rt_pad(t * R + r, sh);
-				if (c < ncol) st2(dst + t * tileH + c * R + r, mk<T>(s[0].y, s[0].x), mk<T>(s[1].y, s[1].x));
+			for (int e = tid; e < nh * U << lC; e += nt) {
+				const int r = 2 * e & (R - 1), i = e >> (lR - 1), u = i % U, c = i / U & (CC - 1), t = i / U >> lC;
+				const cplx<T>* s = sm + (u * CC + c) * ld + rt_pad(t * R + r, sh);
+				if (c < ncol) st2(dst + t * tileH + (c * U + u) * R + r, mk<T>(s[0].y, s[0].x), mk<T>(s[1].y, s[1].x));
 			}
 		} else {
-			for (int e = tid; e < Ny << lC; e += nt) {
-				const int c = e & (CC - 1), t = e >> lC;
-				const cplx<T> v = src[c * ld + rt_pad(t, sh)];
-				if (c < ncol) dst[t * tileH + c] = mk<T>(v.y, v.x);
+			for (int e = tid; e < Ny * U << lC; e += nt) {
+				const int u = e % U, c = e / U & (CC - 1), t = e / U >> lC;
+				const cplx<T> v = sm[(u * CC + c) * ld + rt_pad(t, sh)];
+				if (c < ncol) dst[t * tileH + c * U + u] = mk<T>(v.y, v.x);
+			}
+		}
+	} else {
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			cplx<T>* dst = a.work + u * a.wstride + (long long)kx0 * R;
+			const cplx<T>* src = sm + u * CC * ld;
+			if (R > 1) {
+				for (int i = tid; i < nh << lC; i += nt) {
+					const int e = 2 * i, r = e & (R - 1), c = (e >> lR) & (CC - 1), t = e >> (lR + lC);
+					const cplx<T>* s = src + c * ld + rt_pad(t * R + r, sh);
+					if (c < ncol) st2(dst + t * tileH + c * R + r, mk<T>(s[0].y, s[0].x), mk<T>(s[1].y, s[1].x));
+				}
+			} else {
+				for (int e = tid; e < Ny << lC; e += nt) {
+					const int c = e & (CC - 1), t = e >> lC;
+					const cplx<T> v = src[c * ld + rt_pad(t, sh)];
+					if (c < ncol) dst[t * tileH + c] = mk<T>(v.y, v.x);
+				}
 			}
 		}
 	}
