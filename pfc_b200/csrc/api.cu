@@ -26,6 +26,7 @@
 
 #include "../../include/pfc_b200.h"
 #include "fno.cuh"
+#include "host_copy.h"
 #include "kernels.cuh"
 
 using namespace pfcg;
@@ -82,6 +83,7 @@ struct pfcg_handle {
 	int wsbx = 1, wsby = 1;
 	int early = 0, warm = 0; // choose_early
 	bool no_early = false;  // in a batch, whose launches are plain
+	bool staged = false;    // holds host_copy's chunks
 	int ccr = 1;            // columns per CTA of the run-time y-pass modes (geom.CC: the STEP kernel's)
 	double* d_real = nullptr;   // U*Ny*Nx doubles
 	double* d_fields = nullptr; // f(r) work fields
@@ -649,7 +651,7 @@ template <typename T> int spectral_from_real(pfcg_handle* h) {
 template <typename T> int do_upload(pfcg_handle* h, const double* fields, cudaMemcpyKind kind) {
 	int rc = ensure_real(h);
 	if (rc) return rc;
-	CK(h, cudaMemcpyAsync(h->d_real, fields, sizeof(double) * h->U * (size_t)h->Nx * h->Ny, kind, h->stream));
+	CK(h, host_copy(h->d_real, fields, sizeof(double) * h->U * (size_t)h->Nx * h->Ny, kind, h->stream, h->dev, &h->staged));
 	rc = spectral_from_real<T>(h);
 	if (rc) return rc;
 	h->t = 0;
@@ -677,7 +679,7 @@ template <typename T> int do_download(pfcg_handle* h, double* fields, cudaMemcpy
 	XArgs<T> xa = xargs<T>(h);
 	rc = run_xpass<T>(h, XP_C2R, xa, h->cx);
 	if (rc) return rc;
-	CK(h, cudaMemcpyAsync(fields, h->d_real, sizeof(double) * h->U * (size_t)h->Nx * h->Ny, kind, h->stream));
+	CK(h, host_copy(fields, h->d_real, sizeof(double) * h->U * (size_t)h->Nx * h->Ny, kind, h->stream, h->dev, &h->staged));
 	CK(h, cudaStreamSynchronize(h->stream));
 	return 0;
 }
@@ -811,7 +813,7 @@ template <typename T> int do_smooth(pfcg_handle* h, int u, double* out, cudaMemc
 	x1.real = h->d_real;
 	rc = run_xpass<T>(h, XP_C2R, x1, h->cx1);
 	if (rc) return rc;
-	CK(h, cudaMemcpyAsync(out, h->d_real, sizeof(double) * (size_t)h->Nx * h->Ny, kind, h->stream));
+	CK(h, host_copy(out, h->d_real, sizeof(double) * (size_t)h->Nx * h->Ny, kind, h->stream, h->dev, &h->staged));
 	CK(h, cudaStreamSynchronize(h->stream));
 	return 0;
 }
@@ -909,7 +911,7 @@ template <typename T> int energy_field(pfcg_handle* h, double* f_host) {
 			if ((rc = weighted(W_Q, v, u, v, q + pair * npts, k))) return rc;
 	h->launches++;
 	CK(h, launch_energy_density(mf, pn, eta, q, npair, h->model, npts, f, h->stream));
-	CK(h, cudaMemcpyAsync(f_host, f, sizeof(double) * npts, cudaMemcpyDeviceToHost, h->stream));
+	CK(h, host_copy(f_host, f, sizeof(double) * npts, cudaMemcpyDeviceToHost, h->stream, h->dev, &h->staged));
 	CK(h, cudaStreamSynchronize(h->stream));
 	return 0;
 }
@@ -1114,6 +1116,7 @@ void pfcg_destroy(pfcg_handle* h) {
 	if (h->h_buf) cudaFreeHost(h->h_buf);
 	if (h->sgraph) cudaGraphExecDestroy(h->sgraph);
 	if (h->stream) cudaStreamDestroy(h->stream);
+	host_copy_release(&h->staged);
 	delete h;
 }
 
