@@ -622,18 +622,46 @@ template <typename T> int run_ypass(pfcg_handle* h, int mode, const YArgs<T>& a,
 	return 0;
 }
 
-// Spectral state from the real fields in d_real (device): FP64 means, then the
-// forward transforms of the fluctuations.
-template <typename T> int spectral_from_real(pfcg_handle* h) {
+// The caller's array of n doubles as the kernels' own, where it lies in one
+// allocation of this device, so that the fields cross memory once instead of three
+// times (4096^2 U=2 FP32: upload_device 478 -> 395 us, download_device 208 -> 121;
+// 128^2: 43 -> 40, 27 -> 21); otherwise nullptr, and a copy
+// finds out what the array is.
+double* own_array(pfcg_handle* h, const double* p, size_t n) {
+	static const PFN_cuMemGetAddressRange_v3020 range = [] {
+		cudaDriverEntryPointQueryResult q;
+		void* fn = nullptr;
+		if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &q) != cudaSuccess) {
+			cudaGetLastError();
+			fn = nullptr;
+		}
+		return (PFN_cuMemGetAddressRange_v3020)fn;
+	}();
+	cudaPointerAttributes at;
+	if (!range || (uintptr_t)p % 16) return nullptr;
+	if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+		cudaGetLastError();
+		return nullptr;
+	}
+	CUdeviceptr base = 0;
+	size_t size = 0;
+	if (at.type != cudaMemoryTypeDevice || at.device != h->dev || range(&base, &size, (CUdeviceptr)p) != CUDA_SUCCESS) return nullptr;
+	return (CUdeviceptr)p + n * sizeof(double) <= base + size ? const_cast<double*>(p) : nullptr;
+}
+
+// Spectral state from the real fields (device): FP64 means, then the forward
+// transforms of the fluctuations.
+template <typename T> int spectral_from_real(pfcg_handle* h, double* real) {
 	const size_t npts = (size_t)h->Nx * h->Ny;
 	int rc = 0;
 	// the mean (k = 0 mode) in FP64, by a fixed-order reduction on the device
 	h->launches += 2;
 	{
 		ProfScope ps(h, 2);
-		CK(h, launch_field_means(h->d_real, h->U, (long long)npts, h->d_part, MEAN_BLOCKS, h->mean, h->stream));
+		CK(h, launch_field_means(real, h->U, (long long)npts, h->d_part, MEAN_BLOCKS, h->mean, h->stream));
 	}
 	XArgs<T> xa = xargs<T>(h);
+	xa.real = real;
 	rc = run_xpass<T>(h, XP_R2C, xa, is_wide(h) ? h->cxs : h->cx);
 	if (rc) return rc;
 	YArgs<T> ya = yargs<T>(h, is_wide(h));
@@ -649,10 +677,12 @@ template <typename T> int spectral_from_real(pfcg_handle* h) {
 }
 
 template <typename T> int do_upload(pfcg_handle* h, const double* fields, cudaMemcpyKind kind) {
-	int rc = ensure_real(h);
+	const size_t n = h->U * (size_t)h->Nx * h->Ny;
+	double* own = kind == cudaMemcpyDeviceToDevice ? own_array(h, fields, n) : nullptr;
+	int rc = own ? 0 : ensure_real(h);
 	if (rc) return rc;
-	CK(h, host_copy(h->d_real, fields, sizeof(double) * h->U * (size_t)h->Nx * h->Ny, kind, h->stream, h->dev, &h->staged));
-	rc = spectral_from_real<T>(h);
+	if (!own) CK(h, host_copy(h->d_real, fields, sizeof(double) * n, kind, h->stream, h->dev, &h->staged));
+	rc = spectral_from_real<T>(h, own ? own : h->d_real);
 	if (rc) return rc;
 	h->t = 0;
 	return 0;
@@ -670,16 +700,19 @@ template <typename T> int do_warmstart(pfcg_handle* h, pfcg_fno* f) {
 	if (fno_scratch_grid(f, n, &tmp) || fno_apply_device(f, h->d_real, tmp, h->Nx, h->Ny, h->stream))
 		return fail(h, PFCG_ECUDA, std::string("warm start: ") + fno_error(f));
 	CK(h, cudaMemcpyAsync(h->d_real, tmp, sizeof(double) * n, cudaMemcpyDeviceToDevice, h->stream));
-	return spectral_from_real<T>(h);
+	return spectral_from_real<T>(h, h->d_real);
 }
 
 template <typename T> int do_download(pfcg_handle* h, double* fields, cudaMemcpyKind kind) {
-	int rc = ensure_real(h);
+	const size_t n = h->U * (size_t)h->Nx * h->Ny;
+	double* own = kind == cudaMemcpyDeviceToDevice ? own_array(h, fields, n) : nullptr;
+	int rc = own ? 0 : ensure_real(h);
 	if (rc) return rc;
 	XArgs<T> xa = xargs<T>(h);
+	if (own) xa.real = own;
 	rc = run_xpass<T>(h, XP_C2R, xa, h->cx);
 	if (rc) return rc;
-	CK(h, host_copy(fields, h->d_real, sizeof(double) * h->U * (size_t)h->Nx * h->Ny, kind, h->stream, h->dev, &h->staged));
+	if (!own) CK(h, host_copy(fields, h->d_real, sizeof(double) * n, kind, h->stream, h->dev, &h->staged));
 	CK(h, cudaStreamSynchronize(h->stream));
 	return 0;
 }
@@ -1189,7 +1222,7 @@ static int fields_impl(pfcg_handle* h, const double* density, int fold, double s
 			break;
 		}
 		h->launches++;
-		if ((rc = spectral_from_real<double>(h))) break;
+		if ((rc = spectral_from_real<double>(h, h->d_real))) break;
 		if ((rc = host_means(h, m))) break;
 		wp = WParams{};
 		wp.gs = sb;
@@ -1219,7 +1252,7 @@ static int fields_impl(pfcg_handle* h, const double* density, int fold, double s
 			break;
 		}
 		h->launches++;
-		if ((rc = spectral_from_real<double>(h))) break;
+		if ((rc = spectral_from_real<double>(h, h->d_real))) break;
 		if ((rc = host_means(h, m))) break;
 		double* acc = d_g + n;
 		if (cudaMemsetAsync(acc, 0, sizeof(double) * n, h->stream) != cudaSuccess) {

@@ -55,3 +55,30 @@ def test_two_threads_at_once():
         for ref, got, a, b in out:
             np.testing.assert_array_equal(got, ref)
             np.testing.assert_array_equal(b[2], a[2])
+
+
+@pytest.mark.parametrize("prec,U", [("fp32", 1), ("fp32", 3), ("fp64", 2), ("fp64", 4)])
+def test_device_arrays_of_any_alignment(prec, U):
+    """The kernels read and write a device array in place where it is aligned to 16
+    bytes, and a copy of it at 8: equal to the bit, and nothing beside it is touched."""
+    import torch
+
+    from test_gpu_rt import MEANS, _params
+
+    Nx, Ny = 120, 90
+    n = U * Nx * Ny
+    f0 = np.array([synth.noise_state(Nx, Ny, MEANS[u] if U > 1 else 0.25, 0.05, 3, stream=u) for u in range(U)])
+    got = []
+    with lib.Relaxation(_params(U), Nx, Ny, 0.7, 0.7, prec) as r:
+        for shift in (0, 1, 2):
+            d = torch.full((n + 4,), 7.5, dtype=torch.float64, device="cuda")
+            d[shift:shift + n] = torch.from_numpy(f0.reshape(-1)).cuda()
+            torch.cuda.synchronize()
+            r.upload_device(d.data_ptr() + 8 * shift)
+            r.step(3)
+            r.download_device(d.data_ptr() + 8 * shift)
+            out = d.cpu().numpy()
+            assert (out[:shift] == 7.5).all() and (out[shift + n:] == 7.5).all()
+            got.append(out[shift:shift + n])
+    np.testing.assert_array_equal(got[1], got[0])
+    np.testing.assert_array_equal(got[2], got[0])
