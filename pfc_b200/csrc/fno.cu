@@ -573,19 +573,25 @@ __global__ void __launch_bounds__(128, 4)
                long long nrows, int T) {
 	__shared__ float sW[C * C];
 	__shared__ float sb[C];
+	// A warp's weight sums, [accumulator][lane]. They leave the tensor core after
+	// every 32 pixels: its additions are not rounded to nearest, and sums of whole
+	// rows there left the gradient 1.7e-6 from 64 bits at any batch (512^2; now
+	// 5e-7 at one tile, 8e-7 at 16). A second set of registers spilled (6.6 ms an
+	// iteration, 5.2 this way, 4.6 with the long sums).
+	__shared__ float sacc[4][32][32];
+	float* const mine = &sacc[threadIdx.x >> 5][0][threadIdx.x & 31];
+	const unsigned at = (unsigned)__cvta_generic_to_shared(mine);
+#pragma unroll
+	for (int i = 0; i < 32; i++) mine[32 * i] = 0.f;
 	for (int i = threadIdx.x; i < C * C; i += blockDim.x) sW[i] = 0.f;
 	if (threadIdx.x < C) sb[threadIdx.x] = 0.f;
 	__syncthreads();
 	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 	const long long npix = (long long)T * T;
-	float aW[2][4][4], bsum[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, Qr[2][2][2];
+	float bsum[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, Qr[2][2][2];
 	LiftRow lift[4];
 #pragma unroll
 	for (int mt = 0; mt < 2; mt++) {
-#pragma unroll
-		for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-			for (int k = 0; k < 4; k++) aW[mt][nt][k] = 0.f;
 		if (LAST) {
 #pragma unroll
 			for (int h = 0; h < 2; h++) {
@@ -654,6 +660,7 @@ __global__ void __launch_bounds__(128, 4)
 						d[3][2 * h + c] = q.w;
 					}
 				}
+				float dW[4][4] = {};
 #pragma unroll
 				for (int ks = 0; ks < 2; ks++) {
 					uint32_t ah[4], al[4];
@@ -666,25 +673,34 @@ __global__ void __launch_bounds__(128, 4)
 					for (int nt = 0; nt < 2; nt++) mma_split(acc[mt][nt], ah, al, __ldg(fe + ((tile * 2 + ks) * 2 + nt) * 32 + lane));
 #pragma unroll
 					for (int nt = 0; nt < 4; nt++) {
-						mma_bf16(aW[mt][nt], ah, vh[ks][nt]);
-						mma_bf16(aW[mt][nt], ah, vl[ks][nt]);
-						mma_bf16(aW[mt][nt], al, vh[ks][nt]);
+						mma_bf16(dW[nt], ah, vh[ks][nt]);
+						mma_bf16(dW[nt], ah, vl[ks][nt]);
+						mma_bf16(dW[nt], al, vh[ks][nt]);
 					}
+				}
+#pragma unroll
+				for (int i = 0; i < 16; i++) {
+					// no other thread's and no other access: nothing to order global loads by
+					float q;
+					asm volatile("ld.shared.f32 %0, [%1];" : "=f"(q) : "r"(at + 128 * (16 * mt + i)));
+					q += dW[i >> 2][i & 3];
+					asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + 128 * (16 * mt + i)), "f"(q));
 				}
 			}
 		}
 #pragma unroll
 		for (int mt = 0; mt < 2; mt++) store_modes(A, acc[mt], b, y, T, mt, g, t, sx);
 	}
+	asm volatile("" ::: "memory"); // mine[] was written behind the compiler's back
 #pragma unroll
 	for (int mt = 0; mt < 2; mt++) {
 #pragma unroll
 		for (int nt = 0; nt < 4; nt++) {
 			const int o = 16 * mt + g, i = 8 * nt + 2 * t;
-			atomicAdd(&sW[o * C + i], aW[mt][nt][0]);
-			atomicAdd(&sW[o * C + i + 1], aW[mt][nt][1]);
-			atomicAdd(&sW[(o + 8) * C + i], aW[mt][nt][2]);
-			atomicAdd(&sW[(o + 8) * C + i + 1], aW[mt][nt][3]);
+			atomicAdd(&sW[o * C + i], mine[32 * (16 * mt + 4 * nt + 0)]);
+			atomicAdd(&sW[o * C + i + 1], mine[32 * (16 * mt + 4 * nt + 1)]);
+			atomicAdd(&sW[(o + 8) * C + i], mine[32 * (16 * mt + 4 * nt + 2)]);
+			atomicAdd(&sW[(o + 8) * C + i + 1], mine[32 * (16 * mt + 4 * nt + 3)]);
 		}
 		// bias: the four lanes of a group hold disjoint pixels of the same rows
 #pragma unroll
@@ -1258,8 +1274,6 @@ int backward(pfcg_fno* f, const float* x, int B) {
 	const long long rows = (long long)B * T, planes = (long long)B * C;
 	const int vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
 	cudaStream_t st = f->stream;
-	// about one row per warp in layer_grad: its tensor-core sums stay short (with 4.6
-	// rows each the gradient was 6.7e-6 from 64 bits instead of 2e-6)
 	const int gr = grid_rows(rows);
 	for (int l = L - 1; l >= 0; l--) {
 		float* gW = f->g + off_W(l);
