@@ -241,20 +241,21 @@ int pfcg_set_device(int device);
 int pfcg_set_profiling(pfcg_handle* h, int on);
 int pfcg_profile_read(pfcg_handle* h, double* ms, long long* launches, int nkinds);
 
-/* Measures the launch shapes the runtime-plan kernels can take for this
+/* Measures the launch shapes the kernels of run-time lengths can take for this
  * handle's size (rows per x-pass tile, columns per y-pass group) over nsteps
  * steps each and keeps the fastest; results are cached per (precision, U, Nx,
  * Ny) for the process. Call before pfcg_upload: the timing steps run on the
  * handle's buffers, which are cleared afterwards. Sizes with compile-time
- * specialised kernels (FP32: 256, 384, 512, 768, 1024, 1536, 2048, 4096) keep their fixed shape. No counterpart in
- * the reference (FFTW_MEASURE planning, pfc-relax.c:227-231, is the nearest). */
+ * specialised kernels (one or two FP32 fields: 256, 384, 512, 768, 1024, 1536,
+ * 2048, 4096) keep their fixed shape. No counterpart in the reference
+ * (FFTW_MEASURE planning, pfc-relax.c:227-231, is the nearest). */
 int pfcg_autotune(pfcg_handle* h, int nsteps);
 
 /* Many independent relaxations (sizes, fields and parameters may differ)
  * stepped together. The problems fall into classes: one per (U, N) with
  * N = Nx = Ny a length with specialised kernels (pfcg_autotune lists them), in
- * their fixed launch shape, and one for all other problems, on the
- * runtime-plan kernels. A step of a class is two kernel launches (a batched
+ * their fixed launch shape, or 2048 or 4096 in FP64 with U <= 2, and one for all
+ * other problems, on the kernels of run-time lengths. A step of a class is two kernel launches (a batched
  * x-pass and a batched y-pass over per-problem tables); pfcg_batch_step
  * captures nsteps steps into one CUDA graph (cached per nsteps), each class a
  * chain of its own that runs beside the others, and launches it.

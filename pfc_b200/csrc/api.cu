@@ -1496,7 +1496,7 @@ struct BatchClass {
 	bool ct = false;
 	int U = 0, N = 0;
 	LaunchCfg cx{}, cy{};      // ct: the specialised launch shapes of its problems
-	int threads = 0, smem = 0; // runtime-plan class: the largest of its problems'
+	int threads = 0, smem = 0; // class of run-time lengths: the largest of its problems'
 	int xoff = 0, xn = 0, yoff = 0, yn = 0;
 	cudaStream_t stream = nullptr;
 	cudaEvent_t done = nullptr;
@@ -1716,7 +1716,7 @@ int pfcg_batch_create(int nprob, const pfcg_params* params, const int* Nx, const
 		if (rc) return bail(rc);
 		b->h.push_back(h);
 		// sizes with specialised kernels run them in their fixed shape; the
-		// others run the runtime-plan kernels, in the shape the autotuner picks
+		// others run the kernels of run-time lengths, in the shape the autotuner picks
 		if (batch_ct(h)) continue;
 		h->no_early = true;
 		set_generic_configs(h, h->geom.R, is_wide(h) ? h->geom.CC : h->ccr);
@@ -1920,7 +1920,7 @@ extern "C" int pfcg_relax_noalloc(const pfcg_params* p, int Nx, int Ny, double d
 		rc = fail(&h, PFCG_ESIZE, "bad factorisation");
 	if (!rc) rc = choose_layout(&h);
 	if (rc) return fail(nullptr, rc, h.err);
-	// the runtime-plan STEP kernels (the specialised ones need per-pass tables)
+	// the STEP kernels of run-time lengths (the specialised ones need per-pass tables)
 	if (!is_wide(&h)) set_generic_configs(&h, h.geom.R, h.ccr);
 
 	unsigned char* base = (unsigned char*)scratch;

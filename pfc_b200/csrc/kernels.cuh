@@ -212,7 +212,7 @@ template <typename T> cudaError_t launch_ypass(int mode, const YArgs<T>& a, cons
 // device memory (XArgs<T> or YArgs<T> array) and per-block (problem, tile or
 // column group) tables of nblk blocks. launch_ct_batch: every block's problem
 // has U fields and length N, which has specialised kernels (launch shape c of
-// those problems); launch_generic_batch: the runtime-plan kernels, any sizes.
+// those problems); launch_generic_batch: the kernels of run-time lengths, any sizes.
 // nblk = 0 only prepares the kernels' shared-memory limits (call it before
 // capturing a graph).
 cudaError_t launch_ct_batch(int pass, int U, int N, const void* probs, const int* bp, const int* bl, int nblk,

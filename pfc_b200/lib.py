@@ -270,7 +270,7 @@ class Relaxation:
         return s.value or 0
 
     def autotune(self, nsteps: int = 5) -> None:
-        """Measure the runtime-plan launch shapes and keep the fastest (before upload)."""
+        """Measure the launch shapes of the run-time-length kernels and keep the fastest (before upload)."""
         self._check(self.L.pfcg_autotune(self.h, nsteps))
 
     def set_profiling(self, on: bool) -> None:
