@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(128, 4)
 	// every 32 pixels: its additions are not rounded to nearest, and sums of whole
 	// rows there left the gradient 1.7e-6 from 64 bits at any batch (512^2; now
 	// 5e-7 at one tile, 8e-7 at 16). A second set of registers spilled (6.6 ms an
-	// iteration, 5.2 this way, 4.6 with the long sums).
+	// iteration, 5.2 to 5.6 this way, 4.6 with the long sums).
 	__shared__ float sacc[4][32][32];
 	float* const mine = &sacc[threadIdx.x >> 5][0][threadIdx.x & 31];
 	const unsigned at = (unsigned)__cvta_generic_to_shared(mine);
