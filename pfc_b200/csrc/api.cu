@@ -1985,9 +1985,10 @@ extern "C" int pfcg_relax_noalloc(const pfcg_params* p, int Nx, int Ny, double d
 		if ((rc = run_ypass<float>(&h, YP_STEP, ya, h.cys))) return done(rc);
 	}
 	xa.acc = h.acc;
-	if (wide) { // the last transform is the plan's
+	if (wide) { // the last transform is the plan's; its kernel reads the table before its wait
 		noalloc_twiddles_kernel<<<(Nx + 255) / 256, 256, 0, h.stream>>>((float2*)h.twx, h.px);
 		CKN(cudaGetLastError());
+		h.cx.plain = 1;
 	}
 	if ((rc = run_xpass<float>(&h, XP_C2R, xa, h.cx))) return done(rc);
 	int nan = 0;

@@ -186,6 +186,7 @@ constexpr int FLAG_TIMEOUT = 2;
 struct LaunchCfg {
 	int grid, block, smem;
 	int spec;  // 1: the compile-time specialised STEP kernel for this shape (2: never the fused y-pass)
+	int plain; // 1: launched after the previous kernel's end, whose results this one reads before its wait (rt_warm_twiddles)
 };
 
 // Shapes of the compile-time specialised STEP kernels (FP32, kernels_impl.cuh):

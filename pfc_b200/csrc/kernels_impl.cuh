@@ -1015,7 +1015,8 @@ template <typename K> static void smem_attr(K k, unsigned long long& mask) {
 // next pass's CTAs may be scheduled while the last wave of the previous one
 // drains, and each kernel waits for the previous kernel's completion and
 // memory (griddepcontrol.wait) before touching anything that kernel writes.
-// PFCG_PDL=0 launches them plainly.
+// PFCG_PDL=0 launches them plainly, as `plain` does a kernel that reads something of
+// the previous one before that wait.
 static bool pdl_on() {
 	static const int on = [] {
 		const char* e = std::getenv("PFCG_PDL");
@@ -1025,8 +1026,8 @@ static bool pdl_on() {
 }
 
 template <typename K, typename A>
-static cudaError_t pdl_launch(K k, int grid, int block, int smem, cudaStream_t s, const A& a, int n) {
-	if (!pdl_on()) {
+static cudaError_t pdl_launch(K k, int grid, int block, int smem, cudaStream_t s, const A& a, int n, bool plain = false) {
+	if (plain || !pdl_on()) {
 		k<<<grid, block, smem, s>>>(a, n);
 		return cudaGetLastError();
 	}

@@ -37,7 +37,9 @@ __device__ __forceinline__ void st2(double2* p, double2 a, double2 b) {
 }
 
 // Brings the plan's twiddles into L1 (one load per 128-byte line). Issued before
-// the wait for the previous kernel, on which the table does not depend.
+// the wait for the previous kernel, which must not be the one that writes the table:
+// tables are written when a handle is made, and a launch that follows a kernel
+// writing one is plain (LaunchCfg), since L1 could keep the lines of before.
 template <typename T> __device__ __forceinline__ void rt_warm_twiddles(const cplx<T>* tw, int ntw, int t, int nt) {
 	const char* p = reinterpret_cast<const char*>(tw);
 	const int bytes = ntw * (int)sizeof(cplx<T>);
@@ -671,13 +673,13 @@ template <typename T, int U, bool STEP> cudaError_t xrt_launch(int mode, const X
 	auto k = xrt_kernel<T, U, STEP>;
 	static unsigned long long mask = 0;
 	smem_attr(k, mask);
-	return pdl_launch(k, c.grid, c.block, c.smem, s, a, mode);
+	return pdl_launch(k, c.grid, c.block, c.smem, s, a, mode, c.plain);
 }
 template <typename T, int U, bool STEP> cudaError_t yrt_launch(int mode, const YArgs<T>& a, const LaunchCfg& c, cudaStream_t s) {
 	auto k = yrt_kernel<T, U, STEP>;
 	static unsigned long long mask = 0;
 	smem_attr(k, mask);
-	return pdl_launch(k, c.grid, c.block, c.smem, s, a, mode);
+	return pdl_launch(k, c.grid, c.block, c.smem, s, a, mode, c.plain);
 }
 
 // launchers of one precision and field count, instantiated in kernels_rt_<f32|f64>_<U>.cu

@@ -111,3 +111,31 @@ def test_noalloc_nan_then_clean_call():
     dev = torch.tensor(np.ascontiguousarray(good), dtype=torch.float64, device="cuda")
     torch.cuda.synchronize()
     assert lib.relax_noalloc(p, Nx, Ny, 0.7, 0.7, 5, dev.data_ptr(), 0) == 0, lib.last_error()
+
+
+@pytest.mark.parametrize("U,Nx,Ny", [(3, 128, 96), (4, 60, 84), (3, 640, 36), (4, 1000, 50)])
+def test_noalloc_three_and_four_fields(U, Nx, Ny):
+    """Three and four fields: the step kernels' table and the download's share memory,
+    one written over the other between two launches. Twice in a row with other
+    inputs, against the allocating path (the same kernels, tables of their own) and
+    the oracle, at the FP32 parity bound 2e-5 over five steps; a line of the wrong
+    table would show at the size of the fields."""
+    import torch
+
+    import pyoracle
+    from test_gpu_rt import MEANS, _params
+
+    p, dx, dy, nsteps = _params(U), 0.7, 0.65, 5
+    for seed in (61, 62):
+        f0 = np.array([synth.noise_state(Nx, Ny, MEANS[u], 0.05, seed, stream=u) for u in range(U)])
+        o = pyoracle.Oracle(p, Nx, Ny, dx, dy)
+        o.upload(f0)
+        o.step(nsteps)
+        ref = o.download()
+        o.close()
+        dev = torch.tensor(f0, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        assert lib.relax_noalloc(p, Nx, Ny, dx, dy, nsteps, dev.data_ptr(), 0) == 0, lib.last_error()
+        got = dev.cpu().numpy().reshape(ref.shape)
+        assert np.abs(got - ref).max() < 2e-5
+        assert np.abs(got - reference_run(p, Nx, Ny, dx, dy, f0, nsteps)).max() < 2e-5
