@@ -98,7 +98,11 @@ int pfcg_upload(pfcg_handle* h, const double* fields);
 int pfcg_download(pfcg_handle* h, double* fields);
 
 /* As pfcg_upload / pfcg_download, with the fields in DEVICE memory (for data
- * that is generated or consumed on the GPU). */
+ * that is generated or consumed on the GPU). The kernels read or write the array
+ * itself (one that is not aligned to 16 bytes or not in one allocation of the
+ * handle's device is copied), on the handle's own stream (pfcg_stream), and the call
+ * returns when they have. That stream waits for no other: work that the caller has
+ * queued elsewhere on the array must have finished before the call. */
 int pfcg_upload_device(pfcg_handle* h, const double* d_fields);
 int pfcg_download_device(pfcg_handle* h, double* d_fields);
 

@@ -245,7 +245,7 @@ def make_pairs(n: int, N: int = 512, steps=(10000,), seed0: int = 1, chunk: int 
                 for j in range(m):
                     b.problems[j].download_device(buf.data_ptr())
                     Ys[s][c0 + j].copy_(buf)
-                torch.cuda.synchronize()
+                    torch.cuda.synchronize()  # the next problem writes buf on a stream of its own
         log("pairs %d/%d  %.1f s" % (c0 + m, n, time.time() - t0))
     return X, Ys
 

@@ -207,11 +207,11 @@ class Relaxation:
         return out
 
     def upload_device(self, ptr: int) -> None:
-        """Uploads U*Ny*Nx doubles from DEVICE memory at ptr."""
+        """Uploads U*Ny*Nx doubles from DEVICE memory at ptr, whose writers must have finished."""
         self._check(self.L.pfcg_upload_device(self.h, ctypes.c_void_p(ptr)))
 
     def download_device(self, ptr: int) -> None:
-        """Downloads the fields to U*Ny*Nx doubles of DEVICE memory at ptr."""
+        """Downloads the fields to U*Ny*Nx doubles of DEVICE memory at ptr, whose readers must have finished."""
         self._check(self.L.pfcg_download_device(self.h, ctypes.c_void_p(ptr)))
 
     def smooth(self, u: int = 0) -> np.ndarray:
