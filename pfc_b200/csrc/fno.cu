@@ -257,45 +257,72 @@ __device__ __forceinline__ void store_modes(float2* __restrict__ out, const floa
 }
 
 // x transform of the lifted input: v0 = P x + p is linear, so its modes are P times
-// those of x's two fields, plus p T at m = 0. One warp per eight rows, whose two
-// fields are the sixteen rows of an A operand.
-__global__ void __launch_bounds__(128) lift_dft(const float* __restrict__ x, int xvec, const __nv_bfloat16* __restrict__ w,
-                                                float2* __restrict__ out, const uint4* __restrict__ fe, long long nrows, int T) {
+// those of x's two fields, plus p T at m = 0. These sums are FP32: every channel takes
+// their error times its two weights, so that one of BF16 splits would add up over the
+// channels where those of 32 transforms average out (network applied to 2048^2: 8.3e-6
+// from 64 bits with split products here, 8.0e-6 with one transform per channel and with
+// these; 4096^2 takes 20.9 ms either way).
+// One warp per row; pixel 32 i + lane, w = exp(-2 pi i / T):
+//   X[m] = sum_lane w^(m lane) sum_i x[32 i + lane] w^(32 m i),
+// the inner twiddles the same for every lane.
+__global__ void __launch_bounds__(128) lift_dft(const float* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                float* __restrict__ out, const float2* __restrict__ tw, long long nrows, int T) {
 	__shared__ float Ps[3 * C];
+	__shared__ float2 ti[MAXT / 32][MX];
 	for (int i = threadIdx.x; i < 3 * C; i += blockDim.x) Ps[i] = wld(w, OFF_P + i);
+	for (int i = threadIdx.x; i < T / 32 * MX; i += blockDim.x) ti[i / MX][i % MX] = tw[(32 * (i / MX) * (i % MX)) & (T - 1)];
 	__syncthreads();
-	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+	const int lane = threadIdx.x & 31;
+	float2 tl[MX];
+#pragma unroll
+	for (int m = 0; m < MX; m++) tl[m] = tw[(m * lane) & (T - 1)];
 	const long long npix = (long long)T * T, nw = ((long long)gridDim.x * blockDim.x) >> 5;
-	for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows / 8; r += nw) {
-		const long long b = r * 8 / T;
-		const int y = (int)(r * 8 - b * T) + g;
-		const float* p = x + b * 2 * npix + (long long)y * T + 4 * t;
-		float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll 2
-		for (int tile = 0; tile < T / PX; tile++) {
-			float d[4][4];
+	for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows; r += nw) {
+		const long long b = r / T;
+		const int y = (int)(r - b * T);
+		const float* p = x + b * 2 * npix + (long long)y * T + lane;
+		float a[2 * 2 * MX]; // [field][mode][Re, Im]
 #pragma unroll
-			for (int c = 0; c < 2; c++)
+		for (int k = 0; k < 4 * MX; k++) a[k] = 0.f;
+#pragma unroll 4
+		for (int i = 0; i < T / 32; i++) {
+			const float v[2] = {p[32 * i], p[npix + 32 * i]};
 #pragma unroll
-				for (int h = 0; h < 2; h++) {
-					const float4 q = ld4u(p + h * npix + tile * PX + 16 * c, xvec);
-					d[0][2 * h + c] = q.x;
-					d[1][2 * h + c] = q.y;
-					d[2][2 * h + c] = q.z;
-					d[3][2 * h + c] = q.w;
+			for (int m = 0; m < MX; m++) {
+				const float2 c = ti[i][m];
+#pragma unroll
+				for (int f = 0; f < 2; f++) {
+					a[2 * (MX * f + m)] = fmaf(v[f], c.x, a[2 * (MX * f + m)]);
+					a[2 * (MX * f + m) + 1] = fmaf(v[f], -c.y, a[2 * (MX * f + m) + 1]);
 				}
-			add_dft(acc, d, fe, tile, lane);
+			}
 		}
-		float2* o = out + (b * C * T + y) * MX + t;
-		for (int c = 0; c < C; c++) {
-			const float p0 = Ps[2 * c], p1 = Ps[2 * c + 1], pc = t == 0 ? Ps[2 * C + c] * (float)T : 0.f;
-			float2* q = o + (long long)c * T * MX;
-			q[0] = make_float2(p0 * acc[0][0] + p1 * acc[0][2] + pc, p0 * acc[0][1] + p1 * acc[0][3]);
-			q[4] = make_float2(p0 * acc[1][0] + p1 * acc[1][2], p0 * acc[1][1] + p1 * acc[1][3]);
+#pragma unroll
+		for (int k = 0; k < 2 * MX; k++) {
+			const float2 c = tl[k % MX];
+			const float re = a[2 * k], im = a[2 * k + 1];
+			a[2 * k] = re * c.x + im * c.y;
+			a[2 * k + 1] = im * c.x - re * c.y;
 		}
+		// over the lanes, halving what a lane keeps: it ends with element `lane`
+#pragma unroll
+		for (int o = 16; o; o >>= 1)
+#pragma unroll
+			for (int k = 0; k < o; k++) {
+				const bool up = lane & o;
+				const float keep = up ? a[o + k] : a[k], send = up ? a[k] : a[o + k];
+				a[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+			}
+		const float other = __shfl_xor_sync(0xffffffffu, a[0], 16);
+		const int e = lane & 15, h = lane >> 4; // (Re, Im) of mode e / 2; this half's channels
+		const float x0 = h ? other : a[0], x1 = h ? a[0] : other;
+		float* o = out + ((b * C + h) * T + y) * (2 * MX) + e;
+#pragma unroll 4
+		for (int c = h; c < C; c += 2, o += 2LL * T * (2 * MX))
+			*o = Ps[2 * c] * x0 + Ps[2 * c + 1] * x1 + (e == 0 ? Ps[2 * C + c] * (float)T : 0.f);
 	}
 }
-
+static_assert(4 * MX == 32, "an element of the sums per lane");
 
 // Two-field pixel values of a lane's column for all four n-tiles (channel values of
 // the lift's output), v0[c][px] = P[c][0] x0 + P[c][1] x1 + p[c]
@@ -1241,7 +1268,7 @@ int forward(pfcg_fno* f, const float* x, int B, const float* target) {
 		FCK(cudaMemsetAsync(f->g, 0, sizeof(float) * NPARAM, st));
 		FCK(cudaMemsetAsync(f->loss, 0, sizeof(double), st));
 	}
-	lift_dft<<<grid_for(rows * 4, 128), 128, 0, st>>>(x, vec, f->w, f->A, f->fe, rows, T);
+	lift_dft<<<grid_rows(rows), 128, 0, st>>>(x, f->w, reinterpret_cast<float*>(f->A), f->tw, rows, T);
 	f->launches++;
 	for (int l = 0; l < L; l++) {
 		dft_y_fwd<<<grid_for(planes * 32 * DY_WARPS, 32 * DY_WARPS), 32 * DY_WARPS, 0, st>>>(f->A, f->X[l], f->fdy, planes, T);

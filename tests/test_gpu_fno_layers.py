@@ -94,3 +94,39 @@ def test_gelu_over_its_range():
     # BF16 splits, 2^-16 of the largest operand (44) each in four layers
     assert np.abs(got - want).max() < 4 * 2.0 ** -19 + 4 * 44 * 2.0 ** -16
     assert np.all(np.isfinite(got))
+
+
+def test_lifted_modes_are_fp32_sums():
+    """The modes of the lifted input are FP32 sums, which all channels share: of a wave
+    above the retained modes they are zero but for rounding. With W0 = 0 and one
+    channel's K0 = 1 the first layer's z is the field of those errors. A row's sum of 64
+    products in FP32 is off by about 2^-25 of its partial sums, 40 of them in rms, which
+    makes 128 modes of 64 rows 5e-8 of the field in rms; sums of BF16 pairs (2^-18 a
+    product) make 4.7e-7. Three GELUs near zero halve it each."""
+    T = 64
+    p = np.zeros(fno.NPARAM, dtype=np.float32)
+    lay = fno.layout()
+
+    def put(name, idx, v):
+        o, s = lay[name]
+        p[o + np.ravel_multi_index(idx, s)] = v
+
+    put("P", (0, 0), 1.0)
+    for ky in range(16):
+        for kx in range(8):
+            put("Rr0", (0, 0, ky, kx), 1.0)
+    for l in (1, 2, 3):
+        put("W%d" % l, (0, 0), 1.0)
+    put("Q", (1, 0), 1.0)
+    x = np.zeros((1, 2, T, T), dtype=np.float32)
+    i = np.arange(T)
+    x[0, 0] = np.cos(2 * np.pi * (20 * i[None, :] + 9 * i[:, None]) / T + 0.3)
+    with fno.Network(T, 1) as net:
+        net.set_params(p)
+        dx = torch.tensor(x, device="cuda")
+        dy = torch.empty_like(dx)
+        torch.cuda.synchronize()
+        net.forward(dx.data_ptr(), dy.data_ptr(), 1)
+    want = O.loss_and_grad(fno.bf16_round(p).astype(np.float64), x, x)[2][0, 1]
+    err = np.abs(dy.cpu().numpy()[0, 1] - want).max() * 8
+    assert err < 1.5e-7, err
