@@ -130,3 +130,39 @@ def test_lifted_modes_are_fp32_sums():
     want = O.loss_and_grad(fno.bf16_round(p).astype(np.float64), x, x)[2][0, 1]
     err = np.abs(dy.cpu().numpy()[0, 1] - want).max() * 8
     assert err < 1.5e-7, err
+
+
+@pytest.mark.parametrize("T", [32, 128])
+def test_transform_and_bias_round_once(T):
+    """A layer's inverse transform is a sum of its own, added to the bias in FP32: with
+    W3 = 0, b3 = 1 and a transform of a few 2^-13 the last layer's z = 1 + s is off by
+    half a unit in the last place, 2^-24, and by s's own error, 2^-16 of 2^-12 (products
+    of values split into BF16 pairs). Sums that carry the bias through the tensor
+    core, which does not round to nearest, are off by several times as much."""
+    p = np.zeros(fno.NPARAM, dtype=np.float32)
+    lay = fno.layout()
+
+    def put(name, idx, v):
+        o, s = lay[name]
+        p[o + np.ravel_multi_index(idx, s)] = v
+
+    put("P", (0, 0), 1.0)
+    for l in range(3):
+        put("W%d" % l, (0, 0), 1.0)
+    put("b3", (0,), 1.0)
+    for k in range(1, 7):
+        put("Rr3", (0, 0, k, k), 2.0 ** -11)
+        put("Ri3", (0, 0, k, 7 - k), -2.0 ** -11)
+    put("Q", (1, 0), 1.0)
+    x = np.zeros((1, 2, T, T), dtype=np.float32)
+    x[0, 0] = np.random.default_rng(T).normal(scale=1.0, size=(T, T))
+    with fno.Network(T, 1) as net:
+        net.set_params(p)
+        dx = torch.tensor(x, device="cuda")
+        dy = torch.empty_like(dx)
+        torch.cuda.synchronize()
+        net.forward(dx.data_ptr(), dy.data_ptr(), 1)
+    want = O.loss_and_grad(fno.bf16_round(p).astype(np.float64), x, x)[2][0, 1]
+    s = np.abs(want - 1).max()
+    assert 2.0 ** -16 < s < 2.0 ** -12, s
+    assert np.abs(dy.cpu().numpy()[0, 1] - want).max() < 2.0 ** -24 + 2.0 ** -26
