@@ -27,8 +27,12 @@
 
 #include "../../include/pfc_b200.h"
 #include "fno.cuh"
+#include "fno_gelu.cuh"
 
 namespace {
+
+using pfcg::gelu;
+using pfcg::gelu_d;
 
 constexpr int C = PFCG_FNO_CHANNELS;
 constexpr int L = PFCG_FNO_LAYERS;
@@ -55,43 +59,6 @@ __host__ __device__ constexpr size_t off_Ri(int l) { return off_Rr(l) + (size_t)
 constexpr int MAXT = 512; // largest tile (twiddle table in shared memory)
 
 __device__ __forceinline__ float wld(const __nv_bfloat16* w, size_t i) { return __bfloat162float(w[i]); }
-
-// The normal distribution's lower tail at -u and the density's exponential, u = |z|
-// (clamped where both are zero in FP32): Phi(-u) = exp(-u^2 / 2) R(u), and R(u) =
-// t Q(t) with t = 1 / (1 + 0.21 u) and Q of degree 8, fitted here by iteratively
-// reweighted least squares to 1.4e-8 relative over u < 13.5. GELU from it is within
-// 2.4e-7 of FP64 on [-9, 9] (rms 4.7e-8), from erff 4.5e-7 (6.3e-8), in 16
-// instructions and two special-function ones instead of about 22; the derivative
-// shares both parts. GELU was half of a layer's instructions.
-struct Tail {
-	float u, phi, e;
-	__device__ __forceinline__ explicit Tail(float z) {
-		float t;
-		u = fminf(fabsf(z), 20.f);
-		asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.21f, u, 1.f)));
-		asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-0.72134752f * u * u));
-		float q = -0.07203336f;
-		q = fmaf(q, t, 0.28545034f);
-		q = fmaf(q, t, -0.33418325f);
-		q = fmaf(q, t, 0.35402617f);
-		q = fmaf(q, t, -0.097240396f);
-		q = fmaf(q, t, 0.1263528f);
-		q = fmaf(q, t, 0.068790667f);
-		q = fmaf(q, t, 0.085129313f);
-		q = fmaf(q, t, 0.083707705f);
-		phi = q * t * e;
-	}
-};
-__device__ __forceinline__ float gelu(float z) {
-	const Tail p(z);
-	float r; // max(z, 0), NaN kept
-	asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(z));
-	return fmaf(-p.u, p.phi, r);
-}
-__device__ __forceinline__ float gelu_d(float z) {
-	const Tail p(z);
-	return fmaf(z * 0.39894228040143268f, p.e, z < 0.f ? p.phi : 1.f - p.phi);
-}
 
 // wave number of retained row k along y
 __device__ __forceinline__ int ky_of(int k, int T) { return k < MY / 2 ? k : T - MY + k; }
