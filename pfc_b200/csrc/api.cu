@@ -1420,9 +1420,11 @@ const char* pfcg_last_error(const pfcg_handle* h) { return h ? h->err.c_str() : 
 // --------------------------------------------------------------- autotune ---
 namespace {
 
-// measured (R, CC) per (precision, U, Nx, Ny), shared by every handle of the process
+// measured (R, CC) per (device, in a batch, precision, U, Nx, Ny), shared by every handle
+// of the process. A batch's problems are timed on their own: they do nothing before the
+// previous pass has ended (choose_early), which other shapes suit.
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int, int>, std::pair<int, int>> g_tune;
+std::map<std::tuple<int, bool, int, int, int, int>, std::pair<int, int>> g_tune;
 
 template <typename T> int time_steps(pfcg_handle* h, int nsteps, float* ms) {
 	XArgs<T> xa = xargs<T>(h);
@@ -1450,7 +1452,7 @@ template <typename T> int time_steps(pfcg_handle* h, int nsteps, float* ms) {
 extern "C" int pfcg_autotune(pfcg_handle* h, int nsteps) {
 	if (!h || nsteps < 1) return fail(h, PFCG_EARG, "bad argument");
 	if (h->cxs.spec || h->cys.spec) return 0; // the specialised kernels have a fixed shape
-	const auto key = std::make_tuple((int)h->prec, h->U, h->Nx, h->Ny);
+	const auto key = std::make_tuple(h->dev, h->no_early, (int)h->prec, h->U, h->Nx, h->Ny);
 	{
 		std::lock_guard<std::mutex> lk(g_tune_mu);
 		auto it = g_tune.find(key);

@@ -96,3 +96,24 @@ def test_batch_specialised_2048(precision, tol):
             r.step(4)
             ref = r.download()
         assert np.abs(g - ref).max() < tol
+
+
+@pytest.mark.parametrize("N,batch_first", [(140, True), (150, False)])
+def test_autotune_times_batch_and_single_apart(N, batch_first):
+    """A batch's problem and a handle by itself run the same size differently, so each is
+    timed; a second one of either kind takes the shape that was found."""
+    p = P.make_params(P.honeycomb_1c(-0.25), 1.0, 1.0)
+
+    def single():
+        with lib.Relaxation(p, N, N, 0.8, 0.8, "fp64") as r:
+            r.autotune(2)
+            return r.launches
+
+    def batch():
+        with lib.Batch([(p, N, N, 0.8, 0.8)], "fp64", autotune=True) as b:
+            return b.problems[0].launches
+
+    first, second = (batch, single) if batch_first else (single, batch)
+    assert first() > 0
+    assert second() > 0
+    assert first() == 0 and second() == 0
