@@ -83,7 +83,7 @@ struct pfcg_handle {
 	int wsbx = 1, wsby = 1;
 	int early = 0, warm = 0; // choose_early
 	bool no_early = false;  // in a batch, whose launches are plain
-	bool staged = false;    // holds host_copy's chunks
+	HostHold staged;        // host_copy's chunks
 	int ccr = 1;            // columns per CTA of the run-time y-pass modes (geom.CC: the STEP kernel's)
 	double* d_real = nullptr;   // U*Ny*Nx doubles
 	double* d_fields = nullptr; // f(r) work fields
