@@ -27,9 +27,14 @@ namespace {
 
 constexpr size_t CHUNK = 1 << 20;
 constexpr int WORKERS = 4, SLOTS = 2;
-// Below this the threads' start (some 15 us each) outweighs the faster copy.
-constexpr size_t LEAST = 4 << 20;
-// A caller's bytes from which the chunks are made: 64 MB gain 1.1 ms up and 1.9 down,
+// Below LEAST_UP the threads' start (some 15 us each) outweighs the faster copy. Down, a
+// copy by several cores stalls in about half of the calls for 0.5 to 0.7 ms that neither
+// fewer threads, other chunks nor one thread for all driver calls avoid (8 MB: 0.33 or 1.1
+// ms, the driver alone 0.5; 16 MB: 0.5 or 1.1, the driver 0.9 to 1.05; 32 MB: 0.9 or 1.6, the
+// driver 1.7 to 2.0 and 7.5 into an array that is new), so it is left to the driver below
+// LEAST_DOWN, from where the mean of both gains.
+constexpr size_t LEAST_UP = 4 << 20, LEAST_DOWN = 16 << 20;
+// A caller's bytes from which the chunks are made: 64 MB gain 1 to 2 ms,
 // the chunks cost 1.3 to 2.4 to make and give back.
 constexpr size_t PAYS = 64 << 20;
 constexpr size_t POOL = WORKERS * SLOTS * CHUNK, HUGE = 2 << 20;
@@ -115,7 +120,7 @@ private:
 
 cudaError_t host_copy(void* dst, const void* src, size_t n, cudaMemcpyKind kind, cudaStream_t s, int dev, HostHold* hold) {
 	const bool up = kind == cudaMemcpyHostToDevice;
-	if (n < LEAST || (!up && kind != cudaMemcpyDeviceToHost)) return cudaMemcpyAsync(dst, src, n, kind, s);
+	if (n < (up ? LEAST_UP : LEAST_DOWN) || (!up && kind != cudaMemcpyDeviceToHost)) return cudaMemcpyAsync(dst, src, n, kind, s);
 	cudaPointerAttributes at;
 	cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
 	const bool known = cudaPointerGetAttributes(&at, up ? src : dst) == cudaSuccess && cudaStreamIsCapturing(s, &cap) == cudaSuccess;
