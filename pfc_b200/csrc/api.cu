@@ -211,28 +211,32 @@ bool y_group_ok(const pfcg_handle* h, int c) {
 	return (size_t)S * padded(h->Ny, fp64) * h->celem <= budget;
 }
 
-// CTAs of nt threads and smem bytes that run at once on an SM, at the register
-// counts the kernels of run-time lengths are compiled for (RT_MINB)
-int rt_resident(const pfcg_handle* h, int nt, int smem) {
-	const int regs = h->prec == PFCG_FP64 ? 128 : 64;
+// CTAs of nt threads and smem bytes that run at once on an SM with regs registers a thread
+int rt_resident(int nt, int smem, int regs) {
 	return std::max(1, std::min({65536 / (regs * nt), 227 * 1024 / (smem + 1024), 2048 / nt, 32}));
 }
 
-// Launch shape of the kernels of run-time lengths: S sequences of plan p per
-// CTA. More threads than the passes need shorten the chain (a thread per
-// butterfly, more loads in flight between the transforms) until the grid takes
-// another wave: 1024^2 U=1 FP64 steps in 31 us with 128 threads (one wave) and
-// 46 us with 256 (two); 1440 x 900 U=2 FP32 in 45.6 us with 256 and 47.6 with 224.
+// Threads of a CTA of the kernels of run-time lengths whose passes need nt. More of
+// them, up to `most`, shorten the chain (a thread per butterfly, more loads in flight
+// between the transforms) until the grid takes another wave: 1024^2 U=1 FP64 steps in
+// 31 us with 128 threads (one wave) and 46 us with 256 (two); 1440 x 900 U=2 FP32 in
+// 45.6 us with 256 and 47.6 with 224.
+int rt_more_threads(const pfcg_handle* h, int nt, int most, int smem, int grid, int regs) {
+	auto waves = [&](int n) {
+		const int once = h->nsm * rt_resident(n, smem, regs);
+		return (grid + once - 1) / once;
+	};
+	for (int n : {256, 128, 64})
+		if (n > nt && n <= most && waves(n) <= waves(nt)) return n;
+	return nt;
+}
+
+// Launch shape of those kernels for one problem: S sequences of plan p per CTA, at the
+// register counts that they are compiled for (RT_MINB).
 LaunchCfg rt_config(const pfcg_handle* h, const FftPlan& p, int S, int grid, int* sb) {
 	*sb = sub_batch(p, S);
 	const int smem = (int)(S * p.ld * h->celem);
-	int nt = rt_plan_threads(p, *sb);
-	auto waves = [&](int n) { return (grid + h->nsm * rt_resident(h, n, smem) - 1) / (h->nsm * rt_resident(h, n, smem)); };
-	for (int n : {256, 128, 64})
-		if (n > nt && n <= S * p.n / 4 && waves(n) <= waves(nt)) {
-			nt = n;
-			break;
-		}
+	const int nt = rt_more_threads(h, rt_plan_threads(p, *sb), S * p.n / 4, smem, grid, h->prec == PFCG_FP64 ? 128 : 64);
 	return {grid, nt, smem, 0};
 }
 
@@ -1496,9 +1500,8 @@ extern "C" int pfcg_autotune(pfcg_handle* h, int nsteps) {
 // own stream, independent of the other classes' chains.
 struct BatchClass {
 	bool ct = false;
-	int U = 0, N = 0;
-	LaunchCfg cx{}, cy{};      // ct: the specialised launch shapes of its problems
-	int threads = 0, smem = 0; // class of run-time lengths: the largest of its problems'
+	int U = 0, N = 0;          // U: 0 where the problems' differ
+	LaunchCfg c[2] = {};       // x- and y-pass: threads and shared memory of its blocks
 	int xoff = 0, xn = 0, yoff = 0, yn = 0;
 	cudaStream_t stream = nullptr;
 	cudaEvent_t done = nullptr;
@@ -1528,6 +1531,12 @@ static bool batch_ct(const pfcg_handle* h) { return h->cxs.spec && h->cys.spec &
 // smaller problem in the launch
 static bool batch_own_class(const pfcg_handle* h) {
 	return batch_ct(h) || (h->prec == PFCG_FP64 && h->Nx == h->Ny && h->U <= 2 && (h->Nx == 2048 || h->Nx == 4096));
+}
+// Rows per tile of such a problem: two fields have two in a class of their own, whose
+// grids fill the chip many times over (us per step, one row and two: 2048^2 FP64 228 and
+// 217, two of them 445 and 433, 4096^2 988 and 979); else what suits one problem by itself.
+static int batch_rows(const pfcg_handle* h) {
+	return batch_own_class(h) && h->U == 2 && x_tile_ok(h, 2) ? 2 : h->geom.R;
 }
 
 namespace {
@@ -1570,6 +1579,30 @@ template <typename T> int batch_refresh_args(pfcg_batch* b) {
 	return 0;
 }
 
+// Launch shape of a class of run-time lengths: per pass the largest shared memory of its
+// problems, and threads as rt_config chooses them, but by the waves of all the class's
+// blocks and at the 128 registers its kernels take. With every problem's own threads,
+// chosen for its grid alone, and one shape for both passes, idle threads and the y-pass's
+// shared memory kept blocks off the chip (us per step, FP64: 32 of 256^2 84 and 61, 32 of
+// 256^2 with two fields 202 and 102, 64 of 512^2 614 and 384; FP32 without specialised
+// kernels 8 of 1000^2 199 and 163).
+void batch_rt_shape(const pfcg_batch* b, const std::vector<int>& members, BatchClass* k) {
+	for (int pass = 0; pass < 2; pass++) {
+		LaunchCfg& c = k->c[pass];
+		int most = 0;
+		c.grid = pass ? k->yn : k->xn;
+		for (int i : members) {
+			const pfcg_handle* h = b->h[i];
+			const LaunchCfg& own = pass ? h->cys : h->cxs;
+			const FftPlan& p = pass ? h->py : h->px;
+			c.smem = std::max(c.smem, own.smem);
+			c.block = std::max(c.block, is_wide(h) ? own.block : rt_plan_threads(p, pass ? h->sby : h->sbx));
+			most = std::max(most, is_wide(h) ? 0 : own.smem / (int)(p.ld * h->celem) * p.n / 4);
+		}
+		c.block = rt_more_threads(b->h[members[0]], c.block, most, c.smem, c.grid, 128);
+	}
+}
+
 template <typename T> int batch_build(pfcg_batch* b) {
 	const int n = (int)b->h.size();
 	auto bfail = [&](cudaError_t e, const char* what) {
@@ -1595,8 +1628,10 @@ template <typename T> int batch_build(pfcg_batch* b) {
 				k.ct = batch_ct(h);
 				k.U = h->U;
 				k.N = h->Nx;
-				k.cx = h->cxs;
-				k.cy = h->cys;
+				if (k.ct) {
+					k.c[0] = h->cxs;
+					k.c[1] = h->cys;
+				}
 				b->cls.push_back(k);
 				members.emplace_back();
 			} else {
@@ -1609,11 +1644,6 @@ template <typename T> int batch_build(pfcg_batch* b) {
 				members.emplace_back();
 			}
 			c = generic;
-		}
-		if (!b->cls[c].ct) {
-			BatchClass& k = b->cls[c];
-			k.threads = std::max(k.threads, std::max(h->cxs.block, h->cys.block));
-			k.smem = std::max(k.smem, std::max(h->cxs.smem, h->cys.smem));
 		}
 		members[c].push_back(i);
 	}
@@ -1634,12 +1664,18 @@ template <typename T> int batch_build(pfcg_batch* b) {
 		}
 		k.xn = (int)xp.size() - k.xoff;
 		k.yn = (int)yp.size() - k.yoff;
+		if (!k.ct) {
+			k.U = b->h[m[0]]->U;
+			for (int i : m)
+				if (b->h[i]->U != k.U) k.U = 0;
+			batch_rt_shape(b, m, &k);
+		}
 		cudaError_t e = cudaStreamCreateWithFlags(&k.stream, cudaStreamNonBlocking);
 		if (e == cudaSuccess) e = cudaEventCreateWithFlags(&k.done, cudaEventDisableTiming);
 		// the kernels' shared-memory limits are set here, outside any capture
 		for (int pass = 0; pass < 2 && e == cudaSuccess; pass++)
-			e = k.ct ? launch_ct_batch(pass, k.U, k.N, nullptr, nullptr, nullptr, 0, pass ? k.cy : k.cx, k.stream)
-			         : launch_generic_batch<T>(pass, nullptr, nullptr, nullptr, 0, k.threads, k.smem, k.stream);
+			e = k.ct ? launch_ct_batch(pass, k.U, k.N, nullptr, nullptr, nullptr, 0, k.c[pass], k.stream)
+			         : launch_generic_batch<T>(pass, k.U, nullptr, nullptr, nullptr, 0, k.c[pass], k.stream);
 		if (e != cudaSuccess) return bfail(e, "batch class");
 	}
 	b->xblocks = (int)xp.size();
@@ -1677,13 +1713,13 @@ template <typename T> int batch_launch_steps(pfcg_batch* b, int nsteps) {
 		if (e == cudaSuccess) e = cudaStreamWaitEvent(k.stream, b->fork, 0);
 		for (int s = 0; s < nsteps && e == cudaSuccess; s++) {
 			if (k.ct) {
-				e = launch_ct_batch(0, k.U, k.N, b->d_xargs, xp + k.xoff, xl + k.xoff, k.xn, k.cx, k.stream);
+				e = launch_ct_batch(0, k.U, k.N, b->d_xargs, xp + k.xoff, xl + k.xoff, k.xn, k.c[0], k.stream);
 				if (e == cudaSuccess)
-					e = launch_ct_batch(1, k.U, k.N, b->d_yargs, yp + k.yoff, yl + k.yoff, k.yn, k.cy, k.stream);
+					e = launch_ct_batch(1, k.U, k.N, b->d_yargs, yp + k.yoff, yl + k.yoff, k.yn, k.c[1], k.stream);
 			} else {
-				e = launch_generic_batch<T>(0, b->d_xargs, xp + k.xoff, xl + k.xoff, k.xn, k.threads, k.smem, k.stream);
+				e = launch_generic_batch<T>(0, k.U, b->d_xargs, xp + k.xoff, xl + k.xoff, k.xn, k.c[0], k.stream);
 				if (e == cudaSuccess)
-					e = launch_generic_batch<T>(1, b->d_yargs, yp + k.yoff, yl + k.yoff, k.yn, k.threads, k.smem, k.stream);
+					e = launch_generic_batch<T>(1, k.U, b->d_yargs, yp + k.yoff, yl + k.yoff, k.yn, k.c[1], k.stream);
 			}
 		}
 		// joined even after an error, so that the capture can end
@@ -1721,7 +1757,7 @@ int pfcg_batch_create(int nprob, const pfcg_params* params, const int* Nx, const
 		// others run the kernels of run-time lengths, in the shape the autotuner picks
 		if (batch_ct(h)) continue;
 		h->no_early = true;
-		set_generic_configs(h, h->geom.R, is_wide(h) ? h->geom.CC : h->ccr);
+		set_generic_configs(h, batch_rows(h), is_wide(h) ? h->geom.CC : h->ccr);
 		if (autotune) {
 			const int r2 = pfcg_autotune(h, 5);
 			if (r2) {

@@ -213,14 +213,15 @@ template <typename T> cudaError_t launch_ypass(int mode, const YArgs<T>& a, cons
 // device memory (XArgs<T> or YArgs<T> array) and per-block (problem, tile or
 // column group) tables of nblk blocks. launch_ct_batch: every block's problem
 // has U fields and length N, which has specialised kernels (launch shape c of
-// those problems); launch_generic_batch: the kernels of run-time lengths, any sizes.
+// those problems); launch_generic_batch: the kernels of run-time lengths, any sizes, of U
+// fields or (U = 0) any.
 // nblk = 0 only prepares the kernels' shared-memory limits (call it before
 // capturing a graph).
 cudaError_t launch_ct_batch(int pass, int U, int N, const void* probs, const int* bp, const int* bl, int nblk,
                             const LaunchCfg& c, cudaStream_t s);
 template <typename T>
-cudaError_t launch_generic_batch(int pass, const void* probs, const int* bp, const int* bl, int nblk, int threads,
-                                 int smem, cudaStream_t s);
+cudaError_t launch_generic_batch(int pass, int U, const void* probs, const int* bp, const int* bl, int nblk,
+                                 const LaunchCfg& c, cudaStream_t s);
 
 // Parseval sums for up to MAX_TRIAL box sizes: out[t] = ... With part
 // (MAX_TRIAL * KSPACE_MAX_BLOCKS doubles) the blocks' sums are added in a fixed

@@ -55,16 +55,41 @@ __global__ void __launch_bounds__(MAXNT, 1)
 	}
 }
 
-template <typename T>
-cudaError_t launch_generic_batch(int pass, const void* probs, const int* bp, const int* bl, int nblk, int threads,
-                                 int smem, cudaStream_t s) {
-	static unsigned long long mx = 0, my = 0;
-	smem_attr(xrt_batch_kernel<T>, mx);
-	smem_attr(yrt_batch_kernel<T>, my);
-	if (nblk <= 0) return cudaGetLastError();
-	if (pass == 0) xrt_batch_kernel<T><<<nblk, threads, smem, s>>>((const XArgs<T>*)probs, bp, bl);
-	else yrt_batch_kernel<T><<<nblk, threads, smem, s>>>((const YArgs<T>*)probs, bp, bl);
+// The same where every block's problem has U fields: those kernels need no more
+// registers than U takes.
+template <typename T, int U>
+__global__ void __launch_bounds__(MAXNT, 1)
+    xrt_batch_kernel_u(const XArgs<T>* __restrict__ probs, const int* __restrict__ blk_prob, const int* __restrict__ blk_local) {
+	rt_xpass<T, U, true>(probs[blk_prob[blockIdx.x]], XP_STEP, blk_local[blockIdx.x]);
+}
+template <typename T, int U>
+__global__ void __launch_bounds__(MAXNT, 1)
+    yrt_batch_kernel_u(const YArgs<T>* __restrict__ probs, const int* __restrict__ blk_prob, const int* __restrict__ blk_local) {
+	rt_ypass<T, U, true>(probs[blk_prob[blockIdx.x]], YP_STEP, blk_local[blockIdx.x]);
+}
+
+template <typename A, typename K>
+static cudaError_t batch_launch(K k, unsigned long long& mask, const void* probs, const int* bp, const int* bl, int nblk,
+                                const LaunchCfg& c, cudaStream_t s) {
+	smem_attr(k, mask);
+	if (nblk > 0) k<<<nblk, c.block, c.smem, s>>>((const A*)probs, bp, bl);
 	return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_generic_batch(int pass, int U, const void* probs, const int* bp, const int* bl, int nblk, const LaunchCfg& c,
+                                 cudaStream_t s) {
+	static unsigned long long m[6] = {};
+	if constexpr (sizeof(T) == 8) {
+		if (U == 1)
+			return pass ? batch_launch<YArgs<T>>(yrt_batch_kernel_u<T, 1>, m[0], probs, bp, bl, nblk, c, s)
+			            : batch_launch<XArgs<T>>(xrt_batch_kernel_u<T, 1>, m[1], probs, bp, bl, nblk, c, s);
+		if (U == 2)
+			return pass ? batch_launch<YArgs<T>>(yrt_batch_kernel_u<T, 2>, m[2], probs, bp, bl, nblk, c, s)
+			            : batch_launch<XArgs<T>>(xrt_batch_kernel_u<T, 2>, m[3], probs, bp, bl, nblk, c, s);
+	}
+	return pass ? batch_launch<YArgs<T>>(yrt_batch_kernel<T>, m[4], probs, bp, bl, nblk, c, s)
+	            : batch_launch<XArgs<T>>(xrt_batch_kernel<T>, m[5], probs, bp, bl, nblk, c, s);
 }
 
 } // namespace pfcg

@@ -3,6 +3,7 @@
 
 namespace pfcg {
 
-template cudaError_t launch_generic_batch<float>(int, const void*, const int*, const int*, int, int, int, cudaStream_t);
+template cudaError_t launch_generic_batch<float>(int, int, const void*, const int*, const int*, int, const LaunchCfg&,
+                                           cudaStream_t);
 
 } // namespace pfcg
