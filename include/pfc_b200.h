@@ -247,8 +247,8 @@ int pfcg_profile_read(pfcg_handle* h, double* ms, long long* launches, int nkind
 
 /* Measures the launch shapes the kernels of run-time lengths can take for this
  * handle's size (rows per x-pass tile, columns per y-pass group) over nsteps
- * steps each and keeps the fastest; results are cached per (precision, U, Nx,
- * Ny) for the process. Call before pfcg_upload: the timing steps run on the
+ * steps each and keeps the fastest; results are cached per (device, precision, U,
+ * Nx, Ny) for the process, single handles and a batch's problems apart. Call before pfcg_upload: the timing steps run on the
  * handle's buffers, which are cleared afterwards. Sizes with compile-time
  * specialised kernels (one or two FP32 fields: 256, 384, 512, 768, 1024, 1536,
  * 2048, 4096) keep their fixed shape. No counterpart in the reference
@@ -335,8 +335,9 @@ void pfcg_fno_destroy(pfcg_fno* f);
  * stream: a cudaStream_t (NULL = the default stream); the call returns after it
  *   has synchronised with that stream.
  * Transforms run in FP32 (means and reductions in FP64), as PFCG_FP32, on the
- * step kernels of run-time lengths only: the kernels specialised on a length need
- * per-pass twiddle tables that this call does not build.
+ * step kernels of run-time lengths (one and two fields) or those of three and four
+ * fields: the kernels specialised on a length need per-pass twiddle tables that this
+ * call does not build.
  * The workspace is a file-scope array of PFCG_NOALLOC_SCRATCH_BYTES (32 MiB)
  * that every GPU loading the library holds until exit; grids needing more,
  * about 2 * U * (Nx/2+1) * Ny * 8 bytes plus 32 * Ny bytes and a few KB, are

@@ -135,8 +135,8 @@ __host__ __device__ constexpr int minb(int N, int NT, int ctas) {
 	return want > most ? (most < 2 ? 2 : most) : want < 2 ? 2 : want;
 }
 
-// Launch shapes of the kernels specialised on a compile-time length NC (NC = 0:
-// runtime length and plan). P / S resident sequences, NSUB per FFT call, NT threads.
+// Launch shapes of the kernels specialised on a compile-time length NC. P / S resident
+// sequences, NSUB per FFT call, NT threads.
 template <typename T, int U, int NC, int RC> struct XCfg {
 	static constexpr bool CT = NC > 0;
 	static constexpr int MAXE = CT ? ct_maxe<T>(NC) : RT_MAXE;
@@ -615,13 +615,9 @@ __device__ __forceinline__ void xpass_body(const XArgs<T>& a, const int tile, co
 }
 #pragma nv_diag_default 128
 
-// ----------------------------------------------------------------- y-pass --
-
-
-
-// Row tiles blockIdx.x, + gridDim.x, ... < ntiles: a grid of fewer CTAs than
-// tiles keeps each CTA resident over several tiles, loading the per-pass
-// twiddle table of the specialised kernels once.
+// Row tiles blockIdx.x, + gridDim.x, ... < ntiles. Grids have a CTA per tile, so that
+// the loop runs once; in the y-pass it stays because the compiler allots the registers
+// better with it there (4096^2 U=2: 282.2 us per step, 284.9 without).
 template <typename T, int U, int NC, int RC>
 __global__ void __launch_bounds__(XCfg<T, U, NC, RC>::NT, XCfg<T, U, NC, RC>::MINB)
     xpass_kernel(const XArgs<T> a, int ntiles) {
@@ -636,7 +632,7 @@ __global__ void __launch_bounds__(XCfg<T, U, NC, RC>::NT, XCfg<T, U, NC, RC>::MI
 }
 
 // Body of the y-pass for column group `grp`; called by ypass_kernel and by
-// ypass_batch_kernel.
+// ypass_ct_batch_kernel.
 // ------------------------------------------------------ TMA column loads --
 // The y-pass's input columns are R-row pieces of every row tile of `work`
 // (16 bytes per tile and column at 4096^2 U=2 FP32), a gather that costs the

@@ -1,4 +1,4 @@
-// x- and y-pass kernels of runtime lengths (fft_rt.cuh's plans): every mode at
+// x- and y-pass kernels of run-time lengths (fft_rt.cuh's plans): every mode at
 // sizes without specialised STEP kernels, and the other modes (evaluate, c2r,
 // r2c, the first spectrum, weighted spectra) at every size.
 //

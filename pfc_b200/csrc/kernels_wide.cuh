@@ -1,10 +1,12 @@
 // FP32 STEP, r2c and first-spectrum kernels of systems of three and four fields.
 //
-// They keep the arithmetic that these systems' FP32 results were made with, to
-// the last bit: passes of radix 16, then the power-of-two rest, then 3, 5 and 7,
-// twiddles from an n-entry table, inverse transforms with their own signs, field
-// pairs in the order of the row tile, sums of two products fused as the compiler
-// chooses. The kernels of kernels_rt.cuh step them about three times as fast and
+// They keep the order of operations that these systems' FP32 results were made
+// with: passes of radix 16, then the power-of-two rest, then 3, 5 and 7, twiddles
+// from an n-entry table, inverse transforms with their own signs, field pairs in the
+// order of the row tile. Which products are fused is the compiler's choice, and
+// pfcg_autotune may take another row tile, so the last bits can differ between
+// builds, a single problem and a batch, and tuned and untuned handles.
+// The kernels of kernels_rt.cuh step these systems about three times as fast and
 // are as close to 64 bits (1.5e-5 against 1.4e-5 after 50 steps), but three or
 // four coupled fields amplify a difference in rounding of 1e-7 to 4e-5 of the
 // field and 2e-3 of a point within 100 steps, which no longer counts as the same
