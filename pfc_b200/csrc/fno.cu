@@ -176,7 +176,7 @@ __device__ __forceinline__ void ld_frag(uint32_t (&a)[4], const uint4* p) {
 // a += c, b += c, rounded to nearest. What a tensor core's sum starts from is not: each of
 // its products added to a bias of 1 cost up to 2^-23, so the bias, and in the backward
 // pass the channel product, is added to the transform's own sum (4096^2 applied 20.9 ms,
-// 21.4 with scalar and 20.5 with paired additions; a training iteration 5.7 and 5.8).
+// 21.4 with scalar and 20.5 with paired additions, 20.1 since; a training iteration 5.7 and 5.8, 4.9 since).
 __device__ __forceinline__ void add2(float& a, float& b, float c) {
 	asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %2};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
 	    : "+f"(a), "+f"(b)
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(128, 4)
 	// every 32 pixels: its additions are not rounded to nearest, and sums of whole
 	// rows there left the gradient 1.7e-6 from 64 bits at any batch (512^2; now
 	// 5e-7 at one tile, 8e-7 at 16). A second set of registers spilled (6.6 ms an
-	// iteration, 5.2 to 5.6 this way, 4.6 with the long sums).
+	// iteration, 5.2 to 5.6 this way, 4.6 with the long sums; 4.55 since GELU's derivative needs no clamp).
 	__shared__ float sacc[4][32][32];
 	float* const mine = &sacc[threadIdx.x >> 5][0][threadIdx.x & 31];
 	const unsigned at = (unsigned)__cvta_generic_to_shared(mine);
