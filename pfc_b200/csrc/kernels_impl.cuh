@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(XCfg<T, U, NC, RC>::NT, XCfg<T, U, NC, RC>::MI
 }
 
 // Body of the y-pass for column group `grp`; called by ypass_kernel and by
-// ypass_ct_batch_kernel.
+// ypass_ct_batch_kernel (MEAN: for the k = 0 update too, which is the last group).
 // ------------------------------------------------------ TMA column loads --
 // The y-pass's input columns are R-row pieces of every row tile of `work`
 // (16 bytes per tile and column at 4096^2 U=2 FP32), a gather that costs the
@@ -677,7 +677,7 @@ __device__ __forceinline__ bool tma_wait(unsigned bar, unsigned parity, unsigned
 	}
 }
 
-template <typename T, int U, int NC, int CCC, int RC, bool FUSEDK = true>
+template <typename T, int U, int NC, int CCC, int RC, bool FUSEDK = true, bool MEAN = false>
 __device__ __forceinline__ void ypass_body(const YArgs<T>& a, const int grp, const bool load_tw = true, const int iter = 0) {
 	using C = YCfg<T, U, NC, CCC, RC, FUSEDK>;
 	constexpr int MAXE = C::MAXE;
@@ -686,7 +686,7 @@ __device__ __forceinline__ void ypass_body(const YArgs<T>& a, const int grp, con
 	const int Nx = a.g.Nx, H = a.g.H;
 	const int kx0 = grp * CCC;
 	const int tid = threadIdx.x;
-	if (kx0 >= H) { // the CTA of the k = 0 update
+	if (MEAN && kx0 >= H) {
 		ypass_mean_update<T, U>(a, tid, C::NT);
 		return;
 	}
@@ -967,6 +967,14 @@ __global__ void __launch_bounds__(YCfg<T, U, NC, CCC, RC, FUSEDK>::NT, YCfg<T, U
     ypass_kernel(const YArgs<T> a, int ngroups) {
 	asm volatile("griddepcontrol.wait;" ::: "memory"); // as in xpass_kernel
 	asm volatile("griddepcontrol.launch_dependents;");
+	// The last CTA does the k = 0 update. Told apart here: in the body it cost the column
+	// groups 2 % (4096^2 U=2: y-pass 174.6 us, 171.2 here; a step 281.9 and 280.5, 512^2
+	// 13.5 and 13.3, U=2 15.3 and 15.0, 2048^2 U=2 76.2 and 76.6). A batch's kernels, whose
+	// arguments are in memory, gain nothing by it.
+	if ((int)blockIdx.x == ngroups - 1) {
+		ypass_mean_update<T, U>(a, threadIdx.x, YCfg<T, U, NC, CCC, RC, FUSEDK>::NT);
+		return;
+	}
 	// column groups blockIdx.x, + gridDim.x, ... (as the x-pass's tiles)
 	for (int g = blockIdx.x; g < ngroups; g += gridDim.x) {
 		if (g != (int)blockIdx.x) __syncthreads();
@@ -989,7 +997,7 @@ template <typename T, int U, int NC, int CCC, int RC, bool FUSEDK>
 __global__ void __launch_bounds__(YCfg<T, U, NC, CCC, RC, FUSEDK>::NT, YCfg<T, U, NC, CCC, RC, FUSEDK>::MINB_BATCH)
     ypass_ct_batch_kernel(const YArgs<T>* __restrict__ probs, const int* __restrict__ blk_prob,
                           const int* __restrict__ blk_local) {
-	ypass_body<T, U, NC, CCC, RC, FUSEDK>(probs[blk_prob[blockIdx.x]], blk_local[blockIdx.x]);
+	ypass_body<T, U, NC, CCC, RC, FUSEDK, true>(probs[blk_prob[blockIdx.x]], blk_local[blockIdx.x]);
 }
 
 // Raises the dynamic shared-memory limit of a kernel once per device.
