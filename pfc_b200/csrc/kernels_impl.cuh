@@ -617,7 +617,8 @@ __device__ __forceinline__ void xpass_body(const XArgs<T>& a, const int tile, co
 
 // Row tiles blockIdx.x, + gridDim.x, ... < ntiles. Grids have a CTA per tile, so that
 // the loop runs once; in the y-pass it stays because the compiler allots the registers
-// better with it there (4096^2 U=2: 282.2 us per step, 284.9 without).
+// better with it there (4096^2 U=2: 282.2 us per step, 284.9 without, with the k = 0 update in
+// its body).
 template <typename T, int U, int NC, int RC>
 __global__ void __launch_bounds__(XCfg<T, U, NC, RC>::NT, XCfg<T, U, NC, RC>::MINB)
     xpass_kernel(const XArgs<T> a, int ntiles) {
@@ -1075,10 +1076,10 @@ template <typename T> struct Spec;
 // small CTAs: more of them per grid, and barriers that fewer warps wait at.
 // 512 threads everywhere left 512^2 17 y-pass CTAs and 1024^2 65 for 148 SMs. us per
 // step with (rows, columns) of 512-thread CTAs and with these: 256^2 U=1 16.4
-// (8, 32) and 11.6; 512^2 19.2 (8, 16) and 13.6, U=2 28.3 (4, 8) and 15.4;
-// 768^2 22.0 (8, 8) and 18.0, U=2 33.4 (4, 4) and 23.5; 1024^2 34.4 (8, 8) and 18.4,
-// U=2 36.7 (4, 4) and 24.4; 2048^2 52.1 (8, 4) and 41.3, U=2 92.6 (4, 2) and 77.2;
-// 4096^2 157.9 (4, 2) and 140. Fewer still lose: 1024^2 U=2 one row, one column
+// (8, 32) and 11.2; 512^2 19.2 (8, 16) and 13.2, U=2 28.3 (4, 8) and 15.0;
+// 768^2 22.0 (8, 8) and 17.1, U=2 33.4 (4, 4) and 22.9; 1024^2 34.4 (8, 8) and 18.0,
+// U=2 36.7 (4, 4) and 24.1; 2048^2 52.1 (8, 4) and 40.4, U=2 92.6 (4, 2) and 76.6;
+// 4096^2 157.9 (4, 2) and 138.5. Fewer still lose: 1024^2 U=2 one row, one column
 // 39.6; 4096^2 U=2 one row (8 bytes per column and tile) 409, two rows 282.
 template <> struct Spec<float> {
 	static constexpr bool has(int U, int N) {
